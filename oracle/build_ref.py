@@ -184,7 +184,7 @@ def build_auswertung(name, frames, force=False):
 
 
 def build(names=None, jobs=4):
-    if not os.path.isdir(REF):
+    if not os.path.isfile(os.path.join(REF, REF_TUS[0])):
         return []
     names = names or REF_BUILDS
     with ThreadPoolExecutor(jobs) as ex:
