@@ -35,7 +35,7 @@ enum RunFlags : int {
 enum ErrBits : int {
   E_DEPOSIT_OVERFLOW = 1,  // staged particle set of a mesh tile exceeded capacity
   E_NONFINITE = 2,         // a particle position became NaN/Inf
-  E_BARRIER_TIMEOUT = 4,   // a grid-wide barrier of the fused step gave up waiting
+  E_BARRIER_TIMEOUT = 4,   // a grid-wide barrier of the resident step gave up waiting
 };
 
 // Immutable per-run description (device copy in an array indexed by run).
@@ -85,10 +85,10 @@ struct RunDesc {
   float2* Fw;       // per pid: WCA force (drop-in routines)
   float2* Fk;       // per pid: capillary force
   float2* Fn;       // per pid: noise
-  // Z*Z 64-bit fixed-point density sums of the fused and pipelined steps
-  // (nullptr in the descriptions other kernels receive): the move deposits
-  // the new positions, the next forward row pass consumes them and clears
-  // the words
+  // Z*Z 64-bit fixed-point density sums of the resident and pipelined steps:
+  // the move deposits the new positions, the next forward row pass consumes
+  // them. Fixed dt on a power-of-two mesh: an array of its own; other runs
+  // (resident step): spec2's memory in the device table
   unsigned long long* dacc;
 };
 

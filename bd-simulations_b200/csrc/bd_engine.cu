@@ -1,5 +1,5 @@
-// Engine implementation: per-run device memory, the batched launch plan and
-// graph capture of the fused step.
+// Engine implementation: per-run device memory, the batched launch plan, the
+// resident step's launches and graph capture of the launch-per-step forms.
 #include "bd_engine.h"
 
 #include <algorithm>
@@ -106,7 +106,7 @@ static int ilog2(int z) {
   return l;
 }
 
-// A run can step with the density deposited in the move (fused step or
+// A run can step with the density deposited in the move (resident step or
 // pipelined stage step): a power-of-two mesh, a fixed dt, a mesh at all.
 static bool deposit_in_move(const bd_params& p) {
   bd_derived dv;
@@ -187,6 +187,8 @@ Engine::~Engine() {
     if (ev_fork[k]) cudaEventDestroy(ev_fork[k]);
     if (ev_join[k]) cudaEventDestroy(ev_join[k]);
   }
+  for (auto q : res_streams) cudaStreamDestroy(q);
+  if (ev_res) cudaEventDestroy(ev_res);
   if (stream2) cudaStreamDestroy(stream2);
   if (stream) cudaStreamDestroy(stream);
 }
@@ -200,6 +202,7 @@ int Engine::init(int dev) {
   CK(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
   CK(cudaStreamCreateWithFlags(&stream2, cudaStreamNonBlocking));
   CK(cudaEventCreateWithFlags(&ev_stage, cudaEventDisableTiming));
+  CK(cudaEventCreateWithFlags(&ev_res, cudaEventDisableTiming));
   for (auto& e : ev_piece) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
   for (int k = 0; k < 2; k++) {
     CK(cudaEventCreateWithFlags(&ev_fork[k], cudaEventDisableTiming));
@@ -409,58 +412,312 @@ void Engine::drop_graphs() {
   if (g1) cudaGraphExecDestroy(g1);
   if (gK) cudaGraphExecDestroy(gK);
   g1 = gK = nullptr;
+  graphs_ok = false;
 }
 
-// The fused step applies to one run with a mesh, a power-of-two mesh side
-// from 8 to 1024 and a fixed dt; its transform items are sized so that one
-// CTA handles at most one (at least two CTAs per SM are resident at ~100
-// registers per thread).
-int Engine::plan_fused() {
-  fused = false;
-  if (runs.size() != 1) return BD_OK;
-  const RunHost& r = *runs[0];
-  const int Z = r.Z;
-  if (!r.d.dacc || Z < 8 || Z > 1024) return BD_OK;
-  FusedPlan P{};
-  P.lz = ilog2(Z);
-  int nsm = 0;
-  CK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, device));
-  // CTAs: two per SM once the particles fill a CTA per SM; a small run takes
-  // fewer (at least 32), so that its grid barriers wait on fewer arrivals
-  const int blocks = (r.N + 255) / 256;
-  const int gmin = blocks >= nsm ? 2 * nsm : std::max(32, blocks);
-  auto size_items = [&](int count, int tps, int& l, int& n) {
-    l = 0;
-    while ((count >> l) > gmin && ((2 << l) * tps) <= FFT2_THREADS && (count >> (l + 1)) >= 1) l++;
-    n = count >> l;
+// The resident step takes runs on power-of-two meshes from 8 to 1024 and on
+// meshes with a factor 3 up to 768, ideal-gas runs too, with a fixed or an
+// adaptive dt. Meshes whose transforms are not compiled for their length (a
+// factor 9 or more) up to 648: measured, us per step (resident | stage
+// kernels), 64 000 particles: side 576 48 | 72, 864 107 | 96, 1152 167 | 139.
+static bool resident_run(const RunHost& r) {
+  if (r.idgas) return true;
+  return pow2(r.Z) ? r.Z >= 8 && r.Z <= 1024 : r.Z <= 648 || r.Z == 768;
+}
+
+static int resident_lz(const RunHost& r) {
+  if (r.idgas) return 0;
+  if (pow2(r.Z)) return ilog2(r.Z);
+  for (int lz = 20; lz <= 24; lz++)
+    if (res_side(lz) == r.Z) return lz;
+  return 0;
+}
+
+// Item sizes of a run stepped by G CTAs whose transforms are done by nt
+// threads each (Item.a/b/c: log2 of the rows forward, columns and rows
+// inverse per item) and the shared memory they need.
+static Item resident_item(const RunHost& r, int run, int G, int nt, size_t* smem) {
+  Item I{run, 0, 0, 0};
+  *smem = RES_DESC_BYTES + RES_TW_BYTES(r.idgas ? 0 : r.Z);
+  if (r.idgas) return I;
+  const int Z = r.Z, n = Z / 2;
+  // the size whose rounds cost the busiest CTA least: each round has a fixed
+  // part (round trips, barriers between the passes) and its share of elements
+  auto size = [&](int count, int len, int thr) {
+    int best = 0;
+    double cost = 1e30;
+    for (int l = 0; l < 6 && count % (1 << l) == 0 && (thr << l) <= nt; l++) {
+      const int rounds = ((count >> l) + G - 1) / G;
+      const double c = rounds * (4.0 + (double)(len << l) / nt);
+      if (c < cost - 1e-9) cost = c, best = l;
+    }
+    return best;
   };
-  size_items(Z, fft2_tps(P.lz - 1), P.lrf, P.nrf);
-  size_items(Z / 2, fft2_tps(P.lz), P.lw, P.ncl);
-  size_items(Z, fft2_tps(P.lz), P.lri, P.nri);
-  P.nch = (int)(((long long)r.C * r.C + SCAN_CHUNK - 1) / SCAN_CHUNK);
-  // the forward row items run beside the scan chunks, on the other CTAs
-  // where the threads allow
-  while (P.nrf + P.nch > gmin && P.nrf > 1 && ((2 << P.lrf) * fft2_tps(P.lz - 1)) <= FFT2_THREADS) {
-    P.lrf++;
-    P.nrf >>= 1;
+  if (pow2(Z)) {
+    // as many sequences per item as nt threads take at four elements each
+    const int lz = ilog2(Z);
+    I.a = size(Z, n, fft4_tps(lz - 1));
+    I.b = size(n, 2 * Z, 2 * fft4_tps(lz));  // both inverse transforms at once
+    I.c = size(Z, Z, fft4_tps(lz));
+    *smem += std::max((size_t)(1 << I.a) * fft2_stride(n),
+                      std::max((size_t)2 * (1 << I.b) * fft2_stride(Z), (size_t)(1 << I.c) * fft2_stride(Z))) *
+             8;
+  } else {
+    // up to two butterflies per thread and stage
+    I.a = size(Z, n, n / 8);
+    I.b = size(n, 2 * Z, Z / 4);
+    I.c = size(Z, Z, Z / 8);
+    *smem += std::max((size_t)n << I.a, std::max((size_t)(2 * Z) << I.b, (size_t)Z << I.c)) * 8;
   }
-  const int e = fused_configure(P, device);
-  if (e) {
-    cudaGetLastError();
-    return BD_OK;  // not available: the stage kernels run instead
+  *smem = (*smem + 255) & ~(size_t)255;
+  return I;
+}
+
+// Clusters of cs (1, 2, 4, 8, 16) CTAs of the many-run kernels that the device
+// holds at once: every mesh's kernel has the same threads, register bound and
+// largest shared memory, so one of them is asked, once per process, device and
+// size (an occupancy query takes a few hundred microseconds).
+static int clusters_fit(int cs, int device) {
+  static std::mutex mu;
+  static int fit[64][5] = {};
+  if (device < 0 || device >= 64) return 0;
+  const int k = ilog2(cs);
+  std::lock_guard<std::mutex> g(mu);
+  if (!fit[device][k]) {
+    int n = 0;
+    if (resident_configure(7, false, res_max_smem(false), cs, device, &n) || n <= 0) {
+      cudaGetLastError();
+      n = -1;
+    }
+    fit[device][k] = n;
   }
-  P.grid = std::min(P.grid, std::max(gmin, std::max(P.nrf, std::max(P.ncl, P.nri))));
-  if (P.nrf > P.grid || P.ncl > P.grid || P.nri > P.grid) return BD_OK;
+  return std::max(0, fit[device][k]);
+}
+
+// The resident step's work items, appended to the plan's lists (several
+// runs: one item per run, grouped by mesh size and cluster size).
+void Engine::resident_items(std::vector<Item>& all) {
+  resident = false;
+  fused = false;
+  res_groups.clear();
+  if (runs.empty()) return;
+  for (auto* r : runs)
+    if (!resident_run(*r)) return;
+  long long total = 0;
+  for (auto* r : runs) total += r->N;
+  // steps per launch: about 50 ms of device time at most
+  res_chunk = (int)std::max<long long>(8, std::min<long long>(1024, 400000000ll / std::max<long long>(total, 1)));
+  if (runs.size() == 1) {
+    resident = true;
+    return;
+  }
+  struct Ent {
+    Item I;
+    int lz, cs;
+    size_t smem;
+    double load, share;
+  };
+  std::vector<Ent> v;
+  // load: particles and a quarter of the mesh points per CTA
+  auto weight = [&](const RunHost& r) { return r.N + (r.idgas ? 0.0 : 0.25 * r.Z * r.Z); };
+  const double limit = piped ? 800.0 : 20000.0;
+  for (auto* r : runs)
+    if (weight(*r) > 16 * limit) return;
+  // every run on clusters of one size, the largest at which the whole batch
+  // is resident at once; then larger clusters for runs that would hold the
+  // others up, while there is room to spare. share: the part of the GPU one
+  // cluster takes (the device is asked: clusters of 16 pack badly into GPCs)
+  auto entry = [&](size_t k, int cs) {
+    const RunHost& r = *runs[k];
+    Ent e{};
+    e.lz = resident_lz(r);
+    e.cs = cs;
+    e.I = resident_item(r, (int)k, cs, res_threads(false) / 2, &e.smem);
+    e.load = weight(r) / cs;
+    const int n = e.smem + (size_t)res_pcap(false) * 32 <= res_max_smem(false) ? clusters_fit(cs, device) : 0;
+    e.share = n > 0 ? 1.0 / n : 1e9;
+    return e;
+  };
+  // a batch that takes a mix of cluster sizes fills the GPU less well (0.8)
+  double most = 1e30;
+  for (int base = 16; base >= 1; base /= 2) {
+    std::vector<Ent> w;
+    double used = 0.0;
+    for (size_t k = 0; k < runs.size() && used <= 1.0; k++) {
+      w.push_back(entry(k, base));
+      used += w.back().share;
+    }
+    if (used > 1.0) continue;
+    size_t top = 0;
+    for (;;) {
+      for (size_t k = 0; k < w.size(); k++)
+        if (w[k].load > w[top].load) top = k;
+      if (w[top].cs >= 16) break;
+      const Ent e = entry(top, w[top].cs * 2);
+      if (used + e.share - w[top].share > 0.8) break;
+      used += e.share - w[top].share;
+      w[top] = e;
+    }
+    if (w[top].load < 0.95 * most) {
+      most = w[top].load;
+      v.swap(w);
+    }
+  }
+  // loads where the launch-per-step forms are the better ones. Measured, us per step
+  // (resident | other), runs x particles: pipelined step 8 x 4000 16 | 23,
+  // 32 x 4000 24 | 28, 64 x 2000 25 | 29 (loads to 760), 64 x 4000 41 | 40,
+  // 32 x 8000 40 | 38 (from 1260 on). Stage kernels (adaptive dt or meshes
+  // with a factor 3): 16 x 8000 84 | 208, 64 x 32 000 522 | 912 (load 17 000,
+  // the largest measured)
+  if (v.empty() || most > limit) return;
+  std::stable_sort(v.begin(), v.end(), [](const Ent& a, const Ent& b) {
+    return a.lz != b.lz ? a.lz < b.lz : a.cs != b.cs ? a.cs > b.cs : a.load > b.load;
+  });
+  for (size_t k = 0; k < v.size(); k++) {
+    if (res_groups.empty() || res_groups.back().lz != v[k].lz || res_groups.back().cs != v[k].cs)
+      res_groups.push_back({v[k].lz, v[k].cs, (int)all.size(), 0, 0, 0.0});
+    ResGroup& g = res_groups.back();
+    g.n++;
+    g.smem = std::max(g.smem, v[k].smem);
+    g.load = std::max(g.load, v[k].load);
+    all.push_back(v[k].I);
+  }
+  std::stable_sort(res_groups.begin(), res_groups.end(),
+                   [](const ResGroup& a, const ResGroup& b) { return a.load > b.load; });
+  resident = true;
+}
+
+// Launch shapes of the resident step (after resident_items); resident stays
+// false when a launch does not fit, and the stage kernels run instead.
+int Engine::plan_resident() {
+  if (!resident) return BD_OK;
+  resident = false;
   if (!d_bar) {
     CK(cudaMalloc(&d_bar, 2 * sizeof(unsigned)));
     CK(cudaMemsetAsync(d_bar, 0, 2 * sizeof(unsigned), stream));
   }
-  // the run's density accumulator (cleared again by the prologue that
-  // precedes the first fused step)
-  P.dacc = r.d.dacc;
-  fplan = P;
-  dep_valid = false;
-  fused = true;
+  if (runs.size() > 1) {
+    for (const ResGroup& g : res_groups) {
+      if (res_configured.count(g.lz)) continue;
+      int n = 0;
+      if (resident_configure(g.lz, false, g.smem + (size_t)res_pcap(false) * 32, g.cs, device, &n) || n <= 0) {
+        cudaGetLastError();
+        return BD_OK;
+      }
+      res_configured.insert(g.lz);
+    }
+    while (res_streams.size() + 1 < res_groups.size()) {
+      cudaStream_t s = nullptr;
+      CK(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
+      res_streams.push_back(s);
+    }
+    resident = true;
+    return BD_OK;
+  }
+  const RunHost& r = *runs[0];
+  int nsm = 0;
+  CK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, device));
+  rone_lz = resident_lz(r);
+  // one cluster of 16 CTAs, whose barrier is cheap, or the grid. Measured, us
+  // per step (cluster | grid), particles and mesh side: 500, 64 12.6 | 15.2;
+  // 2000, 128 14.3 | 15.5; 4000, 64 15.4 | 14.9; 4000, 128 17.1 | 15.4;
+  // 1000, 192 20.7 | 16.0
+  res_cs = r.N <= 3000 && r.Z <= 128 ? 16 : 0;
+  // grid mode: one CTA per SM; a small run takes fewer (at least 32, one per
+  // 64 particles and per three mesh rows), so that its barriers wait on fewer
+  // arrivals
+  const int want = std::max(32, std::min(nsm, std::max((r.N + 63) / 64, r.idgas ? 0 : r.Z / 3)));
+  size_t sm_c = 0, sm_g = 0;
+  rone_cluster = resident_item(r, 0, 16, res_threads(true) / 2, &sm_c);
+  rone_grid = resident_item(r, 0, want, res_threads(true) / 2, &sm_g);
+  const size_t work = std::max(sm_c, sm_g);
+  rone_smem = work + (size_t)res_pcap(true) * 32;
+  int n = 0;
+  if (res_cs && (resident_configure(rone_lz, true, rone_smem, res_cs, device, &n) || n <= 0)) {
+    cudaGetLastError();
+    res_cs = 0;
+  }
+  if (resident_configure(rone_lz, true, rone_smem, 0, device, &n) || n <= 0) {
+    cudaGetLastError();
+    return BD_OK;
+  }
+  res_grid = std::min(n, want);
+  rone = ResArgs{};
+  rone.one = table_desc(0);
+  rone.dyn = d_dyn;
+  rone.bar = d_bar;
+  rone.part_off = (int)work;
+  rone.pcap = res_pcap(true);
+  resident = true;
+  fused = r.d.dacc != nullptr;
+  return BD_OK;
+}
+
+// A run's description as the device table holds it: runs without a density
+// accumulator of their own use spec2's memory (bd_resident.cuh).
+RunDesc Engine::table_desc(size_t k) const {
+  RunDesc d = runs[k]->d;
+  if (!d.dacc) d.dacc = reinterpret_cast<unsigned long long*>(d.spec2);
+  return d;
+}
+
+// nsteps steps of the only run in one launch; fault: with the pending
+// recovery-path test (grid mode); ts: phase timestamps of one step.
+int Engine::launch_one(int nsteps, bool fault, unsigned long long* ts) {
+  ResArgs A = rone;
+  A.nsteps = nsteps;
+  A.ts = ts;
+  const int cs = fault ? 0 : res_cs;
+  A.grid_mode = cs == 0;
+  A.one_item = cs ? rone_cluster : rone_grid;
+  if (fault) {
+    A.skip_barrier = fault_barrier;
+    A.skip_cta = res_grid - 1;
+    A.max_polls = fault_polls;
+    fault_barrier = 0;
+  }
+  return launch_resident(rone_lz, true, A, 1, cs, res_grid, rone_smem, stream) ? BD_ERR_CUDA : BD_OK;
+}
+
+// nsteps resident steps of every run, at most res_chunk per launch. Several
+// groups advance independently on streams of their own, forked from and
+// joined to the engine's stream once.
+int Engine::step_resident(long long nsteps) {
+  if (runs.size() == 1) {
+    if (fault_barrier > 0 && nsteps > 0) {
+      RK(launch_one(1, true, nullptr));
+      nsteps--;
+    }
+    while (nsteps > 0) {
+      const int k = (int)std::min<long long>(nsteps, res_chunk);
+      RK(launch_one(k, false, nullptr));
+      nsteps -= k;
+    }
+    return BD_OK;
+  }
+  const size_t ng = res_groups.size();
+  if (ng > 1) {
+    CK(cudaEventRecord(ev_res, stream));
+    for (size_t g = 1; g < ng; g++) CK(cudaStreamWaitEvent(res_streams[g - 1], ev_res, 0));
+  }
+  ResArgs A{};
+  A.runs = d_runs;
+  A.dyn = d_dyn;
+  while (nsteps > 0) {
+    A.nsteps = (int)std::min<long long>(nsteps, res_chunk);
+    for (size_t g = 0; g < ng; g++) {
+      const ResGroup& q = res_groups[g];
+      A.items = it(q.off);
+      A.part_off = (int)q.smem;
+      A.pcap = res_pcap(false);
+      RK(launch_resident(q.lz, false, A, q.n, q.cs, 0, q.smem + (size_t)A.pcap * 32, g ? res_streams[g - 1] : stream));
+    }
+    nsteps -= A.nsteps;
+  }
+  for (size_t g = 1; g < ng; g++) {
+    CK(cudaEventRecord(ev_res, res_streams[g - 1]));
+    CK(cudaStreamWaitEvent(stream, ev_res, 0));
+  }
   return BD_OK;
 }
 
@@ -484,8 +741,7 @@ int Engine::upload_tables() {
   }
   std::vector<RunDesc> hd(runs.size());
   for (size_t k = 0; k < runs.size(); k++) {
-    hd[k] = runs[k]->d;
-    if (!piped) hd[k].dacc = nullptr;  // only the pipelined stage step deposits through the table
+    hd[k] = table_desc(k);
   }
   std::vector<RunDyn> hy;
   if (!runs.empty()) CK(h2d_nosync(stream, d_runs, hd.data(), hd.size() * sizeof(RunDesc)));
@@ -530,7 +786,7 @@ int Engine::build_plan() {
   CK(cudaSetDevice(device));
   CK(cudaStreamSynchronize(stream));  // earlier work may still read the old tables
   drop_graphs();
-  dep_valid = false;  // the next fused or pipelined step starts with the prologue
+  dep_valid = grids_valid = false;  // the next resident or pipelined step starts with the prologue
   descs_ok = false;   // the descriptions depend on the plan (the accumulator of piped runs)
   std::vector<Item> all, dep, part, chunk;
   // FFT items: [0] meshes with a factor 3, [1 + lz] power-of-two meshes 2^lz
@@ -662,7 +918,7 @@ int Engine::build_plan() {
   off_part_all = off_part;
   n_part_all = n_part;
   // pipelined stage step: several runs, every one depositing in the move. A
-  // single run takes the fused step (mesh up to 1024^2) or the classic stage
+  // single run takes the resident step (mesh up to 1024^2) or the classic stage
   // kernels: alone on a large mesh, the tile deposit is cheaper than the
   // move's atomics and its transforms leave the sort nothing to overlap with
   piped = pipe_runs;
@@ -716,6 +972,7 @@ int Engine::build_plan() {
     put(grp, off_pscan, n_pscan);
     put(su, off_psu, n_psu);
   }
+  resident_items(all);
   if (all.size() > d_items_cap) {
     if (d_items) cudaFree(d_items);
     d_items = nullptr;
@@ -725,40 +982,21 @@ int Engine::build_plan() {
   if (!all.empty())
     CK(h2d(stream, d_items, all.data(), all.size() * sizeof(Item)));
   RK(upload_tables());
-  RK(plan_fused());
+  RK(plan_resident());
   RK(plan_tail());
   planned = true;
-  int st = make_graphs();
-  if (st != BD_OK && fused) {
-    // the cooperative launch could not be captured: stage kernels instead
-    cudaGetLastError();
-    drop_graphs();
-    fused = false;
-    st = make_graphs();
-  }
-  return st;
+  return BD_OK;
 }
 
-// One fused step of every run. ev (optional, 10 events) brackets the stages:
+// One step of every run in a launch-per-step form. ev (optional, 10 events) brackets the stages:
 // ev[0] | deposit | ev[1] | row FFT | ev[2] | column FFT | ev[3] | inverse
 // row FFT | ev[4] | particles (+ move) | ev[5] | count scan (+ step end) |
 // ev[6] | scatter | ev[7] .. ev[9] (no further launches)
 int Engine::enqueue_step(cudaStream_t s, cudaEvent_t* ev) {
-  if (fused && !ev) {
-    FusedPlan P = fplan;
-    if (fault_barrier > 0) {
-      P.skip_barrier = fault_barrier;
-      P.skip_cta = P.grid - 1;
-      P.max_polls = fault_polls;
-      fault_barrier = 0;
-    }
-    const int e = launch_fused(runs[0]->d, d_dyn, P, d_bar, s);
-    return e ? BD_ERR_CUDA : BD_OK;
-  }
   if (piped && !ev) return pipe_form == PIPE_TWO && tail_ok ? enqueue_pipe2(s) : enqueue_pipe(s, nullptr);
   // the classic stage kernels leave no pipeline state (they run here for the
   // stage timings of a fused or pipelined plan too)
-  if (fused || piped) RK(dep_invalidate());
+  RK(dep_invalidate());
   if (ev) cudaEventRecord(ev[0], s);
   if (n_dep > 0) RK(launch_deposit(d_runs, d_dyn, it(off_dep), n_dep, mt_max, rows_max, -1, 1, s));
   if (ev) cudaEventRecord(ev[1], s);
@@ -767,10 +1005,10 @@ int Engine::enqueue_step(cudaStream_t s, cudaEvent_t* ev) {
   else if (ev)
     for (int k = 2; k <= 4; k++) cudaEventRecord(ev[k], s);
   if (split) {
-    RK(launch_particles(d_runs, d_dyn, it(off_part), n_part, MODE_FORCES, 7, 1, s, 0, part_shape));
+    RK(launch_particles(d_runs, d_dyn, it(off_part), n_part, MODE_FORCES, 7, 1, s, part_shape));
     RK(launch_move(d_runs, d_dyn, it(off_part), n_part, 1, 0, s));
   } else {
-    RK(launch_particles(d_runs, d_dyn, it(off_part), n_part, MODE_STEP, 7, 1, s, 0, part_shape));
+    RK(launch_step(d_runs, d_dyn, it(off_part), n_part, 0, s, part_shape));
   }
   if (ev) cudaEventRecord(ev[5], s);
   RK(launch_sort(d_runs, d_dyn, 0, (int)runs.size(), it(off_chunk), n_chunk, it(off_part), n_part, 1,
@@ -794,7 +1032,7 @@ int Engine::enqueue_step(cudaStream_t s, cudaEvent_t* ev) {
 int Engine::enqueue_pipe(cudaStream_t s, cudaEvent_t* ev) {
   if (ev) CK(cudaEventRecord(ev[0], s));
   if (ev) CK(cudaEventRecord(ev[1], s));
-  RK(launch_particles(d_runs, d_dyn, it(off_part), n_part, MODE_STEP, 7, 1, s, 1, part_shape));
+  RK(launch_step(d_runs, d_dyn, it(off_part), n_part, 1, s, part_shape));
   if (ev) CK(cudaEventRecord(ev[2], s));
   CK(cudaEventRecord(ev_fork[0], s));
   CK(cudaStreamWaitEvent(stream2, ev_fork[0], 0));
@@ -814,7 +1052,7 @@ int Engine::enqueue_pipe(cudaStream_t s, cudaEvent_t* ev) {
 // cooperative tail (scan | next forward rows, scatter | next columns, step
 // end, the next step's inverse rows). ts (optional): the tail's timestamps.
 int Engine::enqueue_pipe2(cudaStream_t s, unsigned long long* ts) {
-  RK(launch_particles(d_runs, d_dyn, it(off_part), n_part, MODE_STEP, 7, 1, s, 1, part_shape));
+  RK(launch_step(d_runs, d_dyn, it(off_part), n_part, 1, s, part_shape));
   return launch_pipe_tail(d_runs, d_dyn, tplan, d_bar, s, ts) ? BD_ERR_CUDA : BD_OK;
 }
 
@@ -858,7 +1096,7 @@ int Engine::plan_tail() {
   return BD_OK;
 }
 
-int Engine::enqueue_fft(int require_active, cudaStream_t s, cudaEvent_t* ev) {
+int Engine::enqueue_fft(int require_active, cudaStream_t s, cudaEvent_t* ev, int first, int last) {
   FftPass gen[3];
   for (int q = 0; q < 3; q++) gen[q] = {it(fft_gen.off[q]), fft_gen.n[q], fft_gen.sm[q], fft_gen.thr[q]};
   Fft2Group g2[16];
@@ -868,11 +1106,11 @@ int Engine::enqueue_fft(int require_active, cudaStream_t s, cudaEvent_t* ev) {
     g2[k].lz = f.lz;
     for (int q = 0; q < 3; q++) g2[k].pass[q] = {it(f.off[q]), f.n[q], f.sm[q], f.thr[q]};
   }
-  return launch_fft(d_runs, d_dyn, gen, g2, ng, require_active, s, ev);
+  return launch_fft(d_runs, d_dyn, gen, g2, ng, require_active, s, ev, first, last);
 }
 
 int Engine::launches_per_step() const {
-  if (fused) return 1;
+  if (resident && runs.size() == 1) return 1;
   if (piped && pipe_form == PIPE_TWO && tail_ok) return 2;  // particles, cooperative tail
   if (piped) return 6;  // particles, then scan and scatter beside three transform passes
   int n = 0;
@@ -981,7 +1219,7 @@ int Engine::zeitschritt_debug(double mrd, bd_timestep_info* info, double* dt) {
   CK(cudaSetDevice(device));
   if (!planned) RK(build_plan());
   CK(cudaStreamSynchronize(stream));
-  RunDesc d = r.d;
+  RunDesc d = table_desc(0);
   d.mrd = (float)std::min(mrd, 1e30);
   d.flags |= F_ADAPTIVE;
   CK(h2d(stream, d_runs, &d, sizeof(d)));
@@ -995,7 +1233,8 @@ int Engine::zeitschritt_debug(double mrd, bd_timestep_info* info, double* dt) {
   if (st == BD_OK) st = dep_invalidate();
   if (st == BD_OK && cudaStreamSynchronize(stream) != cudaSuccess) st = BD_ERR_CUDA;
   r.adaptive = was_adaptive;
-  const cudaError_t e = h2d(stream, d_runs, &r.d, sizeof(r.d));
+  d = table_desc(0);
+  const cudaError_t e = h2d(stream, d_runs, &d, sizeof(d));
   if (st != BD_OK) return st;
   if (e != cudaSuccess) return BD_ERR_CUDA;
   RK(sync_check());
@@ -1115,13 +1354,14 @@ int Engine::fused_phase_times(int nsteps, double* ms, int nphases) {
   if (!planned) RK(build_plan());
   if (piped) return pipe_phase_times(nsteps, ms, nphases);
   if (!fused) return BD_ERR_STATE;
-  RK(fused_prologue());
+  RK(fused_prologue(false));
   unsigned long long* d_ts = nullptr;
   CK(cudaMalloc(&d_ts, (FUSED_PHASES + 1) * sizeof(unsigned long long)));
   double acc[FUSED_PHASES] = {0};
   int st = BD_OK;
   for (int k = 0; k < nsteps && st == BD_OK; k++) {
-    if (launch_fused(runs[0]->d, d_dyn, fplan, d_bar, stream, d_ts)) st = BD_ERR_CUDA;
+    st = launch_one(1, false, d_ts);
+    grids_valid = false;
     unsigned long long h[FUSED_PHASES + 1];
     if (st == BD_OK && cudaMemcpyAsync(h, d_ts, sizeof(h), cudaMemcpyDeviceToHost, stream) != cudaSuccess)
       st = BD_ERR_CUDA;
@@ -1142,7 +1382,7 @@ int Engine::fused_phase_times(int nsteps, double* ms, int nphases) {
 // beside the transform chain, whose inverse rows fill slot 0's place: slot 0
 // stays 0), summed over nsteps steps.
 int Engine::pipe_phase_times(int nsteps, double* ms, int nphases) {
-  RK(fused_prologue());
+  RK(fused_prologue(true));
   if (pipe_form == PIPE_TWO && tail_ok) return pipe2_phase_times(nsteps, ms, nphases);
   cudaEvent_t ev[FUSED_PHASES + 1];
   for (auto& e : ev) CK(cudaEventCreate(&e));
@@ -1178,7 +1418,7 @@ int Engine::pipe2_phase_times(int nsteps, double* ms, int nphases) {
   for (int k = 0; k < nsteps && st == BD_OK; k++) {
     if (cudaEventRecord(ev[0], stream) != cudaSuccess) st = BD_ERR_CUDA;
     if (st == BD_OK)
-      st = launch_particles(d_runs, d_dyn, it(off_part), n_part, MODE_STEP, 7, 1, stream, 1, part_shape)
+      st = launch_step(d_runs, d_dyn, it(off_part), n_part, 1, stream, part_shape)
                ? BD_ERR_CUDA
                : BD_OK;
     if (st == BD_OK && cudaEventRecord(ev[1], stream) != cudaSuccess) st = BD_ERR_CUDA;
@@ -1271,8 +1511,8 @@ int Engine::time_mesh_passes(int reps, cudaEvent_t e0, cudaEvent_t e1, double* m
 int Engine::time_particles(int shape, int reps, cudaEvent_t e0, cudaEvent_t e1, double* ms) {
   for (int k = 0; k <= reps; k++) {
     if (k == 1) CK(cudaEventRecord(e0, stream));
-    RK(launch_particles(d_runs, d_dyn, it(off_part), n_part, split ? MODE_FORCES : MODE_STEP, 7, 1, stream,
-                        piped ? 1 : 0, shape));
+    if (split) RK(launch_particles(d_runs, d_dyn, it(off_part), n_part, MODE_FORCES, 7, 1, stream, shape));
+    else RK(launch_step(d_runs, d_dyn, it(off_part), n_part, piped ? 1 : 0, stream, shape));
   }
   CK(cudaEventRecord(e1, stream));
   CK(cudaEventSynchronize(e1));
@@ -1406,6 +1646,7 @@ int Engine::make_graphs() {
     CK(e);
     (which == 0 ? g1 : gK) = ex;
   }
+  graphs_ok = true;
   return BD_OK;
 }
 
@@ -1417,19 +1658,20 @@ int Engine::step(long long nsteps) {
   CK(cudaSetDevice(device));
   if (!planned) RK(build_plan());
   if (runs.empty()) return BD_OK;
-  if ((fused || piped) && nsteps > 0) RK(fused_prologue());
-  if (fused && fault_barrier > 0 && nsteps > 0) {  // the faulted step is a direct launch
-    RK(enqueue_step(stream));
-    nsteps--;
+  if (nsteps == 0) return BD_OK;
+  // several runs: a call of one step takes the launch-per-step form
+  if (resident && (runs.size() == 1 || (nsteps > 1 && !(piped && pipe_form == PIPE_TWO)))) {
+    RK(fused_prologue(false));
+    grids_valid = false;
+    return step_resident(nsteps);
   }
+  if (piped) RK(fused_prologue(true));
+  else RK(dep_invalidate());
+  if (!graphs_ok) RK(make_graphs());
   while (nsteps >= K) {
     CK(cudaGraphLaunch(gK, stream));
     nsteps -= K;
   }
-  // the fused step alone is one kernel: launched directly rather than as a
-  // one-node graph
-  if (fused)
-    while (nsteps-- > 0) RK(enqueue_step(stream));
   while (nsteps-- > 0) CK(cudaGraphLaunch(g1, stream));
   return BD_OK;
 }
@@ -1450,15 +1692,16 @@ int Engine::sync_check() {
   return BD_OK;
 }
 
-// A fused step whose grid barrier failed ran no phase past that barrier (the
-// barrier fails for every CTA or for none), so its positions (recA) are those
-// before the step, and the step counter, time and budget did not advance.
-// What the phases before the barrier left behind is cleared: the barrier
-// words, the cell counts, chunk totals and density accumulator the move adds
-// to, the moved-cell counters and the error bit; the cell starts (which the
-// scan may have rebuilt for the new keys) come back from a counting sort of
-// the unchanged records; the next fused step recomputes the spectrum
-// (prologue). The step can then be taken again with the same bits.
+// A resident step whose grid barrier failed ran no phase past that barrier (the
+// barrier fails for every CTA or for none). Within a step its positions (recA)
+// are those before it, and the step counter, time and budget did not advance;
+// at the barrier between two steps the earlier one is complete. What the
+// phases before the barrier left behind is cleared: the barrier words, the
+// cell counts, chunk totals and density accumulator the move adds to, the
+// moved-cell counters, the dt bound and the error bit; the cell starts (which
+// the scan may have rebuilt for the new keys) come back from a counting sort
+// of the unchanged records; the next step recomputes the spectrum (prologue).
+// The step can then be taken again with the same bits.
 int Engine::recover_fused() {
   if (d_bar) CK(cudaMemsetAsync(d_bar, 0, 2 * sizeof(unsigned), stream));
   for (size_t k = 0; k < runs.size(); k++) {
@@ -1470,6 +1713,8 @@ int Engine::recover_fused() {
     CK(d2h(stream, &y, d_dyn + k, sizeof(RunDyn)));
     y.err &= ~E_BARRIER_TIMEOUT;
     y.moved[0] = y.moved[1] = 0;
+    const float big = 3.0e38f;
+    std::memcpy(&y.dt_bits, &big, 4);
     CK(h2d(stream, d_dyn + k, &y, sizeof(RunDyn)));
     if (runs[k]->has_pos) {
       CK(cudaMemcpyAsync(d.recB, d.recA, (size_t)runs[k]->N * sizeof(Rec), cudaMemcpyDeviceToDevice, stream));
@@ -1478,7 +1723,7 @@ int Engine::recover_fused() {
   }
   for (auto* r : runs)
     if (r->d.dacc) CK(cudaMemsetAsync(r->d.dacc, 0, (size_t)r->Z * r->Z * sizeof(unsigned long long), stream));
-  dep_valid = false;
+  RK(dep_invalidate());
   CK(cudaStreamSynchronize(stream));
   return BD_OK;
 }
@@ -1943,33 +2188,27 @@ int Engine::refresh() {
   return dep_invalidate();
 }
 
-// The fused step's pipeline state (spec2 of the current positions, dacc
-// clear) no longer holds: the next fused step is preceded by the prologue.
+// The pipeline state (spec2 of the current positions, dacc clear) no longer
+// holds: the next resident or pipelined step is preceded by the prologue.
 int Engine::dep_invalidate() {
-  dep_valid = false;
+  dep_valid = grids_valid = false;
   return BD_OK;
 }
 
-// deposit + forward row and column passes with the stage kernels: what a
-// fused or pipelined step expects to find
-int Engine::fused_prologue() {
-  if (dep_valid) return BD_OK;
-  for (auto* r : runs)
-    if (r->d.dacc) CK(cudaMemsetAsync(r->d.dacc, 0, (size_t)r->Z * r->Z * sizeof(unsigned long long), stream));
-  RK(launch_deposit(d_runs, d_dyn, it(off_dep), n_dep, mt_max, rows_max, -1, 0, stream));
-  FftPass gen[3];
-  for (int q = 0; q < 3; q++) gen[q] = {it(fft_gen.off[q]), fft_gen.n[q], fft_gen.sm[q], fft_gen.thr[q]};
-  Fft2Group g2[16];
-  const int ng = (int)std::min<size_t>(fft_p2.size(), 16);
-  for (int k = 0; k < ng; k++) {
-    const FftSet& f = fft_p2[k];
-    g2[k].lz = f.lz;
-    for (int q = 0; q < 3; q++) g2[k].pass[q] = {it(f.off[q]), f.n[q], f.sm[q], f.thr[q]};
+// What a resident or pipelined step expects to find, with the stage kernels:
+// deposit, forward row and column passes; grids (the pipelined step): the
+// force grids too, which a resident step does not leave behind
+int Engine::fused_prologue(bool grids) {
+  if (dep_valid && (grids_valid || !grids)) return BD_OK;
+  if (!dep_valid) {
+    for (auto* r : runs)
+      if (r->d.dacc)
+        CK(cudaMemsetAsync(r->d.dacc, 0, (size_t)r->Z * r->Z * sizeof(unsigned long long), stream));
+    if (n_dep > 0) RK(launch_deposit(d_runs, d_dyn, it(off_dep), n_dep, mt_max, rows_max, -1, 0, stream));
   }
-  // the fused step starts with the inverse row pass; the pipelined step's
-  // transform chain ends with it, so its first step finds the force grids
-  RK(launch_fft(d_runs, d_dyn, gen, g2, ng, 0, stream, nullptr, piped ? 3 : 2));
+  if (n_dep > 0) RK(enqueue_fft(0, stream, nullptr, dep_valid ? 2 : 0, grids ? 2 : 1));
   dep_valid = true;
+  grids_valid = grids;
   return BD_OK;
 }
 

@@ -8,6 +8,7 @@
 #include <memory>
 #include <mutex>
 #include <random>
+#include <set>
 #include <string>
 #include <thread>
 #include <vector>
@@ -192,10 +193,33 @@ class Engine {
   std::unique_ptr<HostPool> hpool;
   HostPool& host_pool();
   int download_dyn();
-  // fused step (one run, power-of-two mesh up to 1024^2, fixed dt): one
-  // cooperative launch per step instead of the stage kernels
+  // resident step (bd_resident.cuh): the step loop of a run in one launch.
+  // resident: every run qualifies; one run: rone (cluster of res_cs CTAs, or
+  // the cooperative grid of res_grid CTAs when res_cs is 0); several runs:
+  // one launch per group (mesh size, cluster size), on streams of their own
+  bool resident = false;
+  struct ResGroup {
+    int lz, cs, off, n;
+    size_t smem;
+    double load;  // particles per CTA of its largest run
+  };
+  std::vector<ResGroup> res_groups;
+  std::set<int> res_configured;           // mesh classes whose kernel attributes are set
+  std::vector<cudaStream_t> res_streams;  // for the second and later groups
+  cudaEvent_t ev_res = nullptr;
+  ResArgs rone{};
+  Item rone_cluster{}, rone_grid{};  // item sizes of the two modes
+  int rone_lz = 0, res_cs = 0, res_grid = 0;
+  size_t rone_smem = 0;
+  int res_chunk = 1;  // steps per launch
+  void resident_items(std::vector<Item>& all);
+  int plan_resident();
+  int launch_one(int nsteps, bool fault, unsigned long long* ts);
+  int step_resident(long long nsteps);
+  RunDesc table_desc(size_t k) const;
+  // one run on a power-of-two mesh with a fixed dt, resident (the fused step
+  // of the API: bd_fused_phase_times, bd_inject_barrier_timeout)
   bool fused = false;
-  FusedPlan fplan{};
   unsigned* d_bar = nullptr;
   // pipelined stage step (power-of-two meshes, fixed dt, two or more runs):
   // six launches per step, the density deposited in the move, its transform
@@ -219,12 +243,13 @@ class Engine {
   PipeTail tplan{};
   bool tail_ok = false;  // the cooperative tail kernel fits (else six launches)
   int enqueue_pipe2(cudaStream_t s, unsigned long long* ts = nullptr);
-  // fused and pipelined steps: whether the spectrum (spec2) belongs to the
+  // resident and pipelined steps: whether the spectrum (spec2) belongs to the
   // current positions, with every run's density accumulator (RunDesc::dacc)
-  // zero; cleared when positions change outside those steps (stream-ordered)
-  bool dep_valid = false;
+  // zero, and whether the force grids do (the pipelined step starts from
+  // them); cleared when positions change outside those steps (stream-ordered)
+  bool dep_valid = false, grids_valid = false;
   int dep_invalidate();
-  int fused_prologue();
+  int fused_prologue(bool grids);
   // one-shot fault of the next fused launch (inject_barrier_timeout)
   int fault_barrier = 0;
   unsigned fault_polls = 0;
@@ -234,13 +259,13 @@ class Engine {
   int K = 16;
 
   int enqueue_step(cudaStream_t s, cudaEvent_t* ev = nullptr);
-  int enqueue_fft(int require_active, cudaStream_t s, cudaEvent_t* ev);
+  int enqueue_fft(int require_active, cudaStream_t s, cudaEvent_t* ev, int first = 0, int last = 2);
   int time_mesh_passes(int reps, cudaEvent_t e0, cudaEvent_t e1, double* ms);
   int time_particles(int shape, int reps, cudaEvent_t e0, cudaEvent_t e1, double* ms);
   int tune_particles(int reps, cudaEvent_t e0, cudaEvent_t e1, bd_tune_result* out);
-  int plan_fused();
   int plan_tail();
   int make_graphs();
+  bool graphs_ok = false;
   void drop_graphs();
   Item* it(int off) { return d_items + off; }
 };

@@ -26,6 +26,30 @@ struct FftPlan {
   int lh[16];  // log2 of the butterfly span h = m/r of stage q (pow2 plans)
 };
 
+// The threads that work on one item together: a whole CTA, or half of one
+// with a named barrier of its own, so that the two halves of a resident CTA
+// work on different things between group barriers. tid: index in the team.
+struct CtaTeam {
+  int tid;
+  __device__ __forceinline__ CtaTeam() : tid((int)threadIdx.x) {}
+  __device__ __forceinline__ int nt() const { return (int)blockDim.x; }
+  __device__ __forceinline__ void sync() const { __syncthreads(); }
+};
+// half ID (0: the lower threads) of a CTA of 2*NT threads, NT a power of two
+template <int ID, int NT>
+struct HalfTeam {
+  int tid;
+  __device__ __forceinline__ HalfTeam() {
+    // the index is opaque to the compiler: an item loop around a transform
+    // would otherwise keep every pass's per-thread addresses live and spill
+    unsigned t = threadIdx.x;
+    asm volatile("" : "+r"(t));
+    tid = (int)(t & (unsigned)(NT - 1));
+  }
+  __device__ __forceinline__ int nt() const { return NT; }
+  __device__ __forceinline__ void sync() const { asm volatile("bar.sync %0, %1;" ::"n"(ID + 1), "n"(NT) : "memory"); }
+};
+
 __device__ __forceinline__ float2 cmul(float2 a, float2 b) {
   return make_float2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
 }
@@ -82,9 +106,11 @@ __device__ __forceinline__ void dft_small(float2* v, int r, float sg) {
 }
 
 // Decimation-in-frequency stages. inv selects the sign (+1 when true).
-// Caller syncs before; every stage ends with a sync.
-__device__ inline void fft_dif(float2* s, const FftPlan& P, int lognseq, const float2* tw,
-                               int twstride, bool inv) {
+// Caller syncs before; every stage ends with a sync of the team. TWS: tw is
+// a copy in shared memory.
+template <bool TWS, class Team>
+__device__ __forceinline__ void fft_dif(const Team& T, float2* s, const FftPlan& P, int lognseq,
+                                        const float2* tw, int twstride, bool inv) {
   const int n = P.n, nseq = 1 << lognseq;
   const float sg = inv ? 1.f : -1.f;
   int m = n;
@@ -93,7 +119,7 @@ __device__ inline void fft_dif(float2* s, const FftPlan& P, int lognseq, const f
     const int h = m / r;
     const int tws = (n / m) * twstride;
     const int total = (n / r) << lognseq;
-    for (int idx = threadIdx.x; idx < total; idx += blockDim.x) {
+    for (int idx = T.tid; idx < total; idx += T.nt()) {
       const int b = idx & (nseq - 1);
       const int qq = idx >> lognseq;
       const int g = P.pow2 ? (qq >> P.lh[q]) : qq / h;
@@ -107,7 +133,7 @@ __device__ inline void fft_dif(float2* s, const FftPlan& P, int lognseq, const f
 #pragma unroll
       for (int u = 1; u < 4; u++)
         if (u < r) {
-          float2 w = __ldg(&tw[e * u * tws]);
+          float2 w = TWS ? tw[e * u * tws] : __ldg(&tw[e * u * tws]);
           if (inv) w.y = -w.y;
           v[u] = cmul(v[u], w);
         }
@@ -115,14 +141,15 @@ __device__ inline void fft_dif(float2* s, const FftPlan& P, int lognseq, const f
       for (int u = 0; u < 4; u++)
         if (u < r) s[((base + u * h) << lognseq) | b] = v[u];
     }
-    __syncthreads();
+    T.sync();
     m = h;
   }
 }
 
 // Decimation-in-time stages: the forward stages undone in reverse order.
-__device__ inline void fft_dit(float2* s, const FftPlan& P, int lognseq, const float2* tw,
-                               int twstride, bool inv) {
+template <bool TWS, class Team>
+__device__ __forceinline__ void fft_dit(const Team& T, float2* s, const FftPlan& P, int lognseq,
+                                        const float2* tw, int twstride, bool inv) {
   const int n = P.n, nseq = 1 << lognseq;
   const float sg = inv ? 1.f : -1.f;
   int m = 1;
@@ -132,7 +159,7 @@ __device__ inline void fft_dit(float2* s, const FftPlan& P, int lognseq, const f
     const int h = m / r;
     const int tws = (n / m) * twstride;
     const int total = (n / r) << lognseq;
-    for (int idx = threadIdx.x; idx < total; idx += blockDim.x) {
+    for (int idx = T.tid; idx < total; idx += T.nt()) {
       const int b = idx & (nseq - 1);
       const int qq = idx >> lognseq;
       const int g = P.pow2 ? (qq >> P.lh[q]) : qq / h;
@@ -145,7 +172,7 @@ __device__ inline void fft_dit(float2* s, const FftPlan& P, int lognseq, const f
 #pragma unroll
       for (int u = 1; u < 4; u++)
         if (u < r) {
-          float2 w = __ldg(&tw[e * u * tws]);
+          float2 w = TWS ? tw[e * u * tws] : __ldg(&tw[e * u * tws]);
           if (inv) w.y = -w.y;
           v[u] = cmul(v[u], w);
         }
@@ -154,8 +181,81 @@ __device__ inline void fft_dit(float2* s, const FftPlan& P, int lognseq, const f
       for (int t = 0; t < 4; t++)
         if (t < r) s[((base + t * h) << lognseq) | b] = v[t];
     }
-    __syncthreads();
+    T.sync();
   }
 }
+
+// The same transforms for a length known at compile time (the resident step's
+// meshes of 3 * 2^k points a side): index arithmetic by constants, one
+// butterfly per thread and stage where the team has enough threads. Sequence b
+// starts at s + b*N, elements in order; the arithmetic of every butterfly is
+// fft_dif's and fft_dit's, so are the results. tw: in shared memory, read with
+// stride TWS (tw[t] = exp(-2 pi i t/(N*TWS))).
+__host__ __device__ constexpr int fftc_radix(int m) { return m % 4 == 0 ? 4 : m % 2 == 0 ? 2 : 3; }
+
+template <int N, int M, int TWS, bool DIT, class Team>
+__device__ __forceinline__ void fftc_stage(const Team& T, float2* s, int nseq, const float2* tw) {
+  constexpr int r = fftc_radix(M), h = M / r, per = N / r, st = (N / M) * TWS;
+  constexpr float sg = DIT ? 1.f : -1.f;
+  const int total = nseq * per;
+  for (int idx = T.tid; idx < total; idx += T.nt()) {
+    const int b = idx / per, qq = idx - b * per;
+    const int g = qq / h, e = qq - g * h;
+    float2* q = s + b * N + g * M + e;
+    float2 v[4];
+#pragma unroll
+    for (int t = 0; t < r; t++) v[t] = q[t * h];
+    if (!DIT) dft_small(v, r, sg);
+#pragma unroll
+    for (int u = 1; u < r; u++) {
+      float2 w = tw[e * u * st];
+      if (DIT) w.y = -w.y;
+      v[u] = cmul(v[u], w);
+    }
+    if (DIT) dft_small(v, r, sg);
+#pragma unroll
+    for (int t = 0; t < r; t++) q[t * h] = v[t];
+  }
+  T.sync();
+}
+// forward, natural order in, digit-reversed out
+template <int N, int TWS, int M = N>
+struct FftcDif {
+  template <class Team>
+  static __device__ __forceinline__ void run(const Team& T, float2* s, int nseq, const float2* tw) {
+    if constexpr (M > 1) {
+      fftc_stage<N, M, TWS, false>(T, s, nseq, tw);
+      FftcDif<N, TWS, M / fftc_radix(M)>::run(T, s, nseq, tw);
+    }
+  }
+  // frequency -> storage position, and back (fft_pos, fft_freq)
+  static __device__ __forceinline__ int pos(int k) {
+    if constexpr (M > 1) {
+      constexpr int r = fftc_radix(M), h = M / r;
+      return (k % r) * h + FftcDif<N, TWS, h>::pos(k / r);
+    } else {
+      return 0;
+    }
+  }
+  static __device__ __forceinline__ int freq(int p) {
+    if constexpr (M > 1) {
+      constexpr int r = fftc_radix(M), h = M / r;
+      return p / h + r * FftcDif<N, TWS, h>::freq(p % h);
+    } else {
+      return 0;
+    }
+  }
+};
+// inverse, digit-reversed in, natural order out
+template <int N, int TWS, int M = N>
+struct FftcDit {
+  template <class Team>
+  static __device__ __forceinline__ void run(const Team& T, float2* s, int nseq, const float2* tw) {
+    if constexpr (M > 1) {
+      FftcDit<N, TWS, M / fftc_radix(M)>::run(T, s, nseq, tw);
+      fftc_stage<N, M, TWS, true>(T, s, nseq, tw);
+    }
+  }
+};
 
 }  // namespace bd

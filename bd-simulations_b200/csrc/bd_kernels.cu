@@ -11,67 +11,16 @@
 // run in a fixed order, so results do not depend on scheduling.
 #include <algorithm>
 #include <cstdio>
-#include <cuda/atomic>
 #include <cstdint>
 #include <cuda_runtime.h>
 
 #include "bd_common.cuh"
 #include "bd_fft.cuh"
 #include "bd_fft2.cuh"
+#include "bd_items.cuh"
 #include "bd_kernels.h"
 
 namespace bd {
-
-__device__ __forceinline__ int wrapi(int a, int m) {
-  a %= m;
-  return a < 0 ? a + m : a;
-}
-
-// a in (-m, 2m) into [0, m)
-__device__ __forceinline__ int wrap1(int a, int m) {
-  return a < 0 ? a + m : (a >= m ? a - m : a);
-}
-
-__device__ __forceinline__ bool run_active(const RunDyn* dyn, int run) {
-  return dyn[run].steps_left > 0;
-}
-
-// Load of data that earlier kernels wrote: through the read-only cache when
-// NC, or a plain (coherent) load where the same kernel also writes it (the
-// fused step).
-template <bool NC, class T>
-__device__ __forceinline__ T ldm(const T* p) {
-  if constexpr (NC) return __ldg(p);
-  else return *p;
-}
-
-// Exclusive scan over the CTA (any multiple of 32 threads up to 1024);
-// sh: 32 ints of shared scratch. All threads must call it.
-__device__ inline int block_excl_scan(int v, int* sh) {
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  int x = v;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const int y = __shfl_up_sync(0xffffffffu, x, o);
-    if (lane >= o) x += y;
-  }
-  if (lane == 31) sh[w] = x;
-  __syncthreads();
-  if (w == 0) {
-    int s = lane < (int)(blockDim.x >> 5) ? sh[lane] : 0;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const int y = __shfl_up_sync(0xffffffffu, s, o);
-      if (lane >= o) s += y;
-    }
-    sh[lane] = s;
-  }
-  __syncthreads();
-  const int base = w > 0 ? sh[w - 1] : 0;
-  const int r = base + x - v;
-  __syncthreads();
-  return r;
-}
 
 // In-place exclusive scan of n counts stored with a stride: a[k*stride] ->
 // out[k*stride + 1]; writes the total to out[n*stride]. All threads call it.
@@ -207,40 +156,6 @@ __device__ inline void deposit_tile(const RunDesc& R, int scheme, int x0, int y0
   __syncthreads();
 }
 
-// The same contributions as deposit_tile, of one particle, added straight to
-// the fused step's accumulator R.dacc with 64-bit integer atomics (mesh point
-// k*Z + l); the integer sums, and so the density, are those of the tiles.
-__device__ __forceinline__ void deposit_acc(const RunDesc& R, const Rec& p) {
-  int ic, jc;
-  cell_ij(R, p.cell, ic, jc);
-  int k, l;
-  float tx, ty;
-  mesh_axis(R, ic, p.ox, k, tx);
-  mesh_axis(R, jc, p.oy, l, ty);
-  const float scale = __int_as_float((127 + R.fx_shift) << 23);
-  const float q = p.pid < R.N1 ? 1.0f : R.q2;
-  unsigned long long* acc = R.dacc;
-  if (R.scheme == NGP) {
-    float c = R.drho;
-    if (p.pid >= R.N1) c *= q;
-    atomicAdd(&acc[(size_t)k * R.Z + l], (unsigned long long)(long long)__float2int_rn(c * scale));
-    return;
-  }
-  float wx[3], wy[3];
-  axis_weights(R.scheme, tx, wx);
-  axis_weights(R.scheme, ty, wy);
-#pragma unroll
-  for (int a = 0; a < 3; a++) {
-    const size_t row = (size_t)wrap1(k + a - 1, R.Z) * R.Z;
-#pragma unroll
-    for (int b = 0; b < 3; b++) {
-      float c = wx[a] * wy[b] * R.drho;
-      if (p.pid >= R.N1) c *= q;
-      atomicAdd(&acc[row + wrap1(l + b - 1, R.Z)], (unsigned long long)(long long)__float2int_rn(c * scale));
-    }
-  }
-}
-
 __global__ void __launch_bounds__(256) k_deposit(const RunDesc* __restrict__ runs,
                                                  const RunDyn* __restrict__ dyn,
                                                  const Item* __restrict__ items, int nitems,
@@ -281,7 +196,7 @@ __global__ void __launch_bounds__(FFT_THREADS) k_fft_rows_fwd(const RunDesc* __r
       s[(m << lr) | b] = v;
     }
     __syncthreads();
-    fft_dif(s, R.plan_half, lr, R.tw, 2, false);
+    fft_dif<false>(CtaTeam(), s, R.plan_half, lr, R.tw, 2, false);
     for (int i = threadIdx.x; i < (n << lr); i += blockDim.x) {
       const int b = i / n, j = i - b * n;
       const float2 zj = s[(__ldg(&R.pos_half[j]) << lr) | b];
@@ -327,7 +242,7 @@ __global__ void __launch_bounds__(FFT_THREADS) k_fft_cols(const RunDesc* __restr
       sA[i] = R.spec[(size_t)k * n + col0 + c];
     }
     __syncthreads();
-    fft_dif(sA, R.plan_full, lw, R.tw, 1, false);
+    fft_dif<false>(CtaTeam(), sA, R.plan_full, lw, R.tw, 1, false);
     // columns other than the packed one: independent per element
     for (int i = threadIdx.x; i < (Z << lw); i += blockDim.x) {
       const int pos = i >> lw, c = i & (W - 1);
@@ -374,8 +289,8 @@ __global__ void __launch_bounds__(FFT_THREADS) k_fft_cols(const RunDesc* __restr
       }
     }
     __syncthreads();
-    fft_dit(sA, R.plan_full, lw, R.tw, 1, true);
-    fft_dit(sB, R.plan_full, lw, R.tw, 1, true);
+    fft_dit<false>(CtaTeam(), sA, R.plan_full, lw, R.tw, 1, true);
+    fft_dit<false>(CtaTeam(), sB, R.plan_full, lw, R.tw, 1, true);
     for (int i = threadIdx.x; i < (Z << lw); i += blockDim.x) {
       const int k = i >> lw, c = i & (W - 1);
       const float2 a = sA[i], b = sB[i];
@@ -422,190 +337,13 @@ __global__ void __launch_bounds__(FFT_THREADS) k_fft_rows_inv(const RunDesc* __r
       s[(__ldg(&R.pos_full[j]) << lr) | b] = h;
     }
     __syncthreads();
-    fft_dit(s, R.plan_full, lr, R.tw, 1, true);
+    fft_dit<false>(CtaTeam(), s, R.plan_full, lr, R.tw, 1, true);
     for (int i = threadIdx.x; i < (Z << lr); i += blockDim.x) {
       const int b = i / Z, l = i - b * Z;
       R.H[(size_t)(row0 + b) * Z + l] = s[(l << lr) | b];
     }
     __syncthreads();
   }
-}
-
-// ---------------------------------------------------------------------------
-// Power-of-two meshes: the same three passes with the register-radix
-// Stockham transform (bd_fft2.cuh), natural order throughout. Items are
-// sized on the host so that one item's sequences need at most blockDim.x
-// threads.
-
-// Row pass, forward, of rows row0 .. row0 + 2^lr - 1 (layout as
-// k_fft_rows_fwd). tw: the run's twiddle table, in shared memory when TWS.
-// FROM_ACC (fused step): the rows come from the fixed-point accumulator
-// R.dacc, converted as deposit_tile converts its sums; the density is also
-// stored to R.rho and the accumulator words are cleared for the next step.
-template <int LZ, bool TWS, bool FROM_ACC = false>
-__device__ __forceinline__ void fft2_rows_fwd_item(const RunDesc& R, int row0, int lr, float2* s,
-                                                   const float2* tw) {
-  constexpr int Z = 1 << LZ, n = Z >> 1, lz = LZ, ln = LZ - 1;
-  constexpr int ss = fft2_stride(n);
-  float2* src = reinterpret_cast<float2*>(R.rho) + (size_t)row0 * n;
-  if (FROM_ACC) {
-    ulonglong2* acc = reinterpret_cast<ulonglong2*>(R.dacc) + (size_t)row0 * n;
-    const double inv = 1.0 / (double)__int_as_float((127 + R.fx_shift) << 23);
-    for (int i = threadIdx.x; i < (n << lr); i += blockDim.x) {
-      const int b = i >> ln, m = i & (n - 1);
-      const ulonglong2 a = acc[i];
-      const float2 v = make_float2((float)((double)(long long)a.x * inv), (float)((double)(long long)a.y * inv));
-      s[b * ss + pad16(m)] = v;
-      src[i] = v;
-      acc[i] = make_ulonglong2(0ull, 0ull);
-    }
-  } else {
-    for (int i = threadIdx.x; i < (n << lr); i += blockDim.x) {
-      const int b = i >> ln, m = i & (n - 1);
-      s[b * ss + pad16(m)] = src[i];
-    }
-  }
-  __syncthreads();
-  Fft2Sched<LZ - 1, 0, TWS>::run(s, ss, 1 << lr, tw, lz, -1.f);
-  // the half spectrum is stored by column (slot j of row k at spec[j*Z + k]),
-  // so the column pass reads whole columns. Consecutive threads take groups
-  // of rb = min(2^lr, 4) consecutive rows of one slot (a whole 32-byte sector
-  // of a column from 4 rows on), then the next slot: at most rb-way bank
-  // conflicts on the rows' shared-memory reads.
-  const int lrb = lr < 2 ? lr : 2;
-  const int rbm = (1 << lrb) - 1;
-  for (int i = threadIdx.x; i < (n << lr); i += blockDim.x) {
-    const int rest = i >> lrb;
-    const int j = rest & (n - 1), b = ((rest >> ln) << lrb) + (i & rbm);
-    const float2 zj = s[b * ss + pad16(j)];
-    const float2 zc = s[b * ss + pad16((n - j) & (n - 1))];
-    float2 out;
-    if (j == 0) {
-      out = make_float2(zj.x + zj.y, zj.x - zj.y);
-    } else {
-      // E = (zj + conj zc)/2, O = (zj - conj zc)/(2i), X = E + w^j O
-      const float2 E = make_float2(0.5f * (zj.x + zc.x), 0.5f * (zj.y - zc.y));
-      const float2 O = make_float2(0.5f * (zj.y + zc.y), -0.5f * (zj.x - zc.x));
-      out = cadd(E, cmul(TWS ? tw[j] : __ldg(&tw[j]), O));
-    }
-    R.spec[(size_t)j * Z + row0 + b] = out;
-  }
-  __syncthreads();
-}
-
-// Green's multiply of the packed column (ky = 0 and ky = Z/2 travel as
-// C = A + iB): split with the partner Cm = C[-kx], multiply A and B by
-// i*s*g with their own factors, pack the Fx and Fy results again.
-__device__ __forceinline__ void packed_green(const RunDesc& R, int kx, float2 Cv, float2 Cm, int n, int Z,
-                                             float sy0, float syn, float2& P, float2& Q) {
-  // A = (C + conj Cm)/2 ; B = (C - conj Cm)/(2i)
-  const float2 A = make_float2(0.5f * (Cv.x + Cm.x), 0.5f * (Cv.y - Cm.y));
-  const float2 Bv = make_float2(0.5f * (Cv.y + Cm.y), -0.5f * (Cv.x - Cm.x));
-  const float gA = __ldg(&R.green[kx]);
-  const float gB = __ldg(&R.green[(size_t)n * Z + kx]);
-  const float sx = __ldg(&R.sxt[kx]);
-  const float2 FxA = make_float2(-sx * gA * A.y, sx * gA * A.x);
-  const float2 FxB = make_float2(-sx * gB * Bv.y, sx * gB * Bv.x);
-  const float2 FyA = make_float2(-sy0 * gA * A.y, sy0 * gA * A.x);
-  const float2 FyB = make_float2(-syn * gB * Bv.y, syn * gB * Bv.x);
-  P = make_float2(FxA.x - FxB.y, FxA.y + FxB.x);
-  Q = make_float2(FyA.x - FyB.y, FyA.y + FyB.x);
-}
-
-// Column pass (as k_fft_cols) of the 2^lw adjacent half-spectrum columns
-// from col0; smem holds 2 * 2^lw sequences.
-template <int LZ, bool TWS>
-__device__ __forceinline__ void fft2_cols_item(const RunDesc& R, int col0, int lw, float2* sA, const float2* tw) {
-  constexpr int Z = 1 << LZ, n = Z >> 1, lz = LZ;
-  constexpr int ss = fft2_stride(Z);
-  const int W = 1 << lw;
-  float2* sB = sA + W * ss;
-  // the row pass stored the half spectrum by column: whole columns are read
-  const float2* src = R.spec + (size_t)col0 * Z;
-  for (int i = threadIdx.x; i < (Z << lw); i += blockDim.x) {
-    const int c = i >> lz, k = i & (Z - 1);
-    sA[c * ss + pad16(k)] = src[i];
-  }
-  __syncthreads();
-  Fft2Sched<LZ, 0, TWS>::run(sA, ss, W, tw, lz, -1.f);
-  for (int i = threadIdx.x; i < (Z << lw); i += blockDim.x) {
-    const int c = i >> lz, kx = i & (Z - 1);
-    const int j = col0 + c;
-    if (j == 0) continue;
-    const float g = __ldg(&R.green[(size_t)j * Z + kx]);
-    const float gx = __ldg(&R.sxt[kx]) * g;
-    const float gy = __ldg(&R.syt[j]) * g;
-    const int a = c * ss + pad16(kx);
-    const float2 v = sA[a];
-    sA[a] = make_float2(-gx * v.y, gx * v.x);
-    sB[a] = make_float2(-gy * v.y, gy * v.x);
-  }
-  if (col0 == 0) {
-    // packed column (ky = 0, ky = Z/2): C = A + iB. Element kx of A, B
-    // needs C[kx] and C[-kx], so one thread handles both of a pair and
-    // writes them in place.
-    const float sy0 = __ldg(&R.syt[0]), syn = __ldg(&R.syt[n]);
-    for (int kx = threadIdx.x; kx <= n; kx += blockDim.x) {
-      const int km = (Z - kx) & (Z - 1);
-      const float2 Ck = sA[pad16(kx)], Cm = sA[pad16(km)];
-      float2 P, Q;
-      packed_green(R, kx, Ck, Cm, n, Z, sy0, syn, P, Q);
-      sA[pad16(kx)] = P;
-      sB[pad16(kx)] = Q;
-      if (km != kx) {
-        packed_green(R, km, Cm, Ck, n, Z, sy0, syn, P, Q);
-        sA[pad16(km)] = P;
-        sB[pad16(km)] = Q;
-      }
-    }
-  }
-  __syncthreads();
-  if (2 * W * fft2_tps(lz) <= (int)blockDim.x) {
-    Fft2Sched<LZ, 0, TWS>::run(sA, ss, 2 * W, tw, lz, 1.f);  // sB follows sA: 2W sequences
-  } else {
-    Fft2Sched<LZ, 0, TWS>::run(sA, ss, W, tw, lz, 1.f);
-    Fft2Sched<LZ, 0, TWS>::run(sB, ss, W, tw, lz, 1.f);
-  }
-  for (int i = threadIdx.x; i < (Z << lw); i += blockDim.x) {
-    const int k = i >> lw, c = i & (W - 1);
-    const float2 a = sA[c * ss + pad16(k)], b = sB[c * ss + pad16(k)];
-    R.spec2[(size_t)k * n + col0 + c] = make_float4(a.x, a.y, b.x, b.y);
-  }
-  __syncthreads();
-}
-
-// Row pass, inverse (as k_fft_rows_inv), of rows row0 .. row0 + 2^lr - 1.
-template <int LZ, bool TWS>
-__device__ __forceinline__ void fft2_rows_inv_item(const RunDesc& R, int row0, int lr, float2* s, const float2* tw) {
-  constexpr int Z = 1 << LZ, n = Z >> 1, lz = LZ;
-  constexpr int ss = fft2_stride(Z);
-  for (int i = threadIdx.x; i < (Z << lr); i += blockDim.x) {
-    const int b = i >> lz, j = i & (Z - 1);
-    const float4* rb = R.spec2 + (size_t)(row0 + b) * n;
-    float2 h;
-    if (j == 0) {
-      const float4 v = rb[0];
-      h = make_float2(v.x, v.z);
-    } else if (j == n) {
-      const float4 v = rb[0];
-      h = make_float2(v.y, v.w);
-    } else if (j < n) {
-      const float4 v = rb[j];
-      h = make_float2(v.x - v.w, v.y + v.z);
-    } else {
-      const float4 v = rb[Z - j];
-      h = make_float2(v.x + v.w, -v.y + v.z);
-    }
-    s[b * ss + pad16(j)] = h;
-  }
-  __syncthreads();
-  Fft2Sched<LZ, 0, TWS>::run(s, ss, 1 << lr, tw, lz, 1.f);
-  float2* dst = R.H + (size_t)row0 * Z;
-  for (int i = threadIdx.x; i < (Z << lr); i += blockDim.x) {
-    const int b = i >> lz, l = i & (Z - 1);
-    dst[i] = s[b * ss + pad16(l)];
-  }
-  __syncthreads();
 }
 
 // The three passes as kernels, one item per CTA (an item loop around the
@@ -621,7 +359,7 @@ __global__ void __launch_bounds__(FFT2_THREADS) k_fft2_rows_fwd(const RunDesc* _
   const Item I = items[blockIdx.x];
   if (require_active && !run_active(dyn, I.run)) return;
   const RunDesc& R = runs[I.run];
-  fft2_rows_fwd_item<LZ, false>(R, I.a, I.c, (float2*)smem, R.tw);
+  fft2_rows_fwd_item<LZ, false, false>(CtaTeam(), R, I.a, I.c, (float2*)smem, R.tw);
 }
 
 template <int LZ>
@@ -634,7 +372,7 @@ __global__ void __launch_bounds__(FFT2_THREADS) k_fft2_cols(const RunDesc* __res
   const Item I = items[blockIdx.x];
   if (require_active && !run_active(dyn, I.run)) return;
   const RunDesc& R = runs[I.run];
-  fft2_cols_item<LZ, false>(R, I.a, I.c, (float2*)smem, R.tw);
+  fft2_cols_item<LZ, false>(CtaTeam(), R, I.a, I.c, (float2*)smem, R.tw);
 }
 
 // Meshes of 2048 and more: the column pass with 1024 threads, so that an
@@ -651,7 +389,7 @@ __global__ void __launch_bounds__(FFT2_WIDE_THREADS) k_fft2_cols_wide(const RunD
   const Item I = items[blockIdx.x];
   if (require_active && !run_active(dyn, I.run)) return;
   const RunDesc& R = runs[I.run];
-  fft2_cols_item<LZ, false>(R, I.a, I.c, (float2*)smem, R.tw);
+  fft2_cols_item<LZ, false>(CtaTeam(), R, I.a, I.c, (float2*)smem, R.tw);
 }
 
 template <int LZ>
@@ -664,379 +402,50 @@ __global__ void __launch_bounds__(FFT2_THREADS) k_fft2_rows_inv(const RunDesc* _
   const Item I = items[blockIdx.x];
   if (require_active && !run_active(dyn, I.run)) return;
   const RunDesc& R = runs[I.run];
-  fft2_rows_inv_item<LZ, false>(R, I.a, I.c, (float2*)smem, R.tw);
+  fft2_rows_inv_item<LZ, false>(CtaTeam(), R, I.a, I.c, (float2*)smem, R.tw);
 }
 
-// ---------------------------------------------------------------------------
-// Per-particle physics shared by the staged and the global neighbour paths.
-
-// Interpolated capillary force (gridRoutinen.cpp:81-126, 284-407, 551-668).
-template <bool NC>
-__device__ inline float2 mesh_force(const RunDesc& R, const Rec& p, int ic, int jc, int scheme) {
-  int k, l;
-  float tx, ty;
-  mesh_axis(R, ic, p.ox, k, tx);
-  mesh_axis(R, jc, p.oy, l, ty);
-  const bool sp2 = p.pid >= R.N1;
-  if (scheme == NGP) {
-    const float2 h = ldm<NC>(&R.H[(size_t)k * R.Z + l]);
-    if (!sp2) return h;
-    // species 2 reads the imaginary part of the x grid in the reference
-    // (gridRoutinen.cpp:123), which is zero up to rounding
-    if (R.flags & F_NGP_REFCOMPAT) return make_float2(R.q2 * h.x, 0.0f);
-    return make_float2(R.q2 * h.x, R.q2 * h.y);
-  }
-  float wx[3], wy[3];
-  axis_weights(scheme, tx, wx);
-  axis_weights(scheme, ty, wy);
-  const int km = k == 0 ? R.Z - 1 : k - 1, kp = k == R.Z - 1 ? 0 : k + 1;
-  const int lm = l == 0 ? R.Z - 1 : l - 1, lp = l == R.Z - 1 ? 0 : l + 1;
-  const int ks[3] = {km, k, kp};
-  float fx = 0.f, fy = 0.f;
-#pragma unroll
-  for (int a = 0; a < 3; a++) {
-    const float2* row = R.H + (size_t)ks[a] * R.Z;
-    const float2 h0 = ldm<NC>(&row[lm]), h1 = ldm<NC>(&row[l]), h2 = ldm<NC>(&row[lp]);
-    fx += wx[a] * (wy[0] * h0.x + wy[1] * h1.x + wy[2] * h2.x);
-    fy += wx[a] * (wy[0] * h0.y + wy[1] * h1.y + wy[2] * h2.y);
-  }
-  if (sp2) {
-    fx *= R.q2;
-    fy *= R.q2;
-  }
-  return make_float2(fx, fy);
-}
-
-// WCA parameters of one particle against neighbours of its own and of the
-// other species (dynamik_methoden.cpp:679-686, 851-865, 1021-1035), held in
-// registers for its pair loop. mask selects pair types (1: 11, 2: 22, 4: 12).
-struct WcaP {
-  float pre_s, sig_s, sig2_s;  // same species
-  float pre_x, sig_x, sig2_x;  // other species
-  float B, cut2, maxPair, L;
-  float scale;                 // 2^wfx_shift: pair terms are summed in 64-bit fixed point
-  int N1;
-  bool sp, on_s, on_x, smallbox;
-};
-
-__device__ __forceinline__ WcaP wca_params(const RunDesc& R, const Rec& p, int mask) {
-  WcaP W;
-  W.sp = p.pid >= R.N1;
-  const int ts = W.sp ? 1 : 0;
-  W.pre_s = R.wpre[ts];
-  W.sig_s = R.wsig[ts];
-  W.sig2_s = R.wsig2[ts];
-  W.pre_x = R.wpre[2];
-  W.sig_x = R.wsig[2];
-  W.sig2_x = R.wsig2[2];
-  W.on_s = (mask & (W.sp ? 2 : 1)) != 0;
-  W.on_x = (mask & 4) != 0;
-  W.B = R.B;
-  W.cut2 = R.cut2;
-  W.maxPair = R.maxPair;
-  W.L = R.L;
-  W.N1 = R.N1;
-  W.smallbox = (R.flags & F_SMALLBOX) != 0;
-  W.scale = __int_as_float((127 + R.wfx_shift) << 23);
-  return W;
-}
-
-// WCA contribution of neighbour q on particle p, added to the fixed-point
-// sum (fx, fy): rounded once per pair term, the sum does not depend on the
-// order in which neighbours are visited. da, db: cell step from p's cell to
-// q's cell.
-__device__ __forceinline__ void wca_pair(const WcaP& W, const Rec& p, const Rec& q, int da, int db, long long& fx,
-                                         long long& fy) {
-  const bool same = (q.pid >= W.N1) == W.sp;
-  if (!(same ? W.on_s : W.on_x)) return;
-  float dx = (p.ox - q.ox) - (float)da * W.B;
-  float dy = (p.oy - q.oy) - (float)db * W.B;
-  // minimum image, as abstand2_* (allgemeine_methoden.cpp:100-166). With
-  // offsets in (-B, 2B] and neighbouring cells |d| < 3B, which is below L/2
-  // from 7 cells per side on; only smaller boxes need the wrap.
-  if (W.smallbox) {
-    dx -= W.L * rintf(dx / W.L);
-    dy -= W.L * rintf(dy / W.L);
-  }
-  const float a2 = dx * dx + dy * dy;
-  const float a2s = a2 * (same ? W.sig2_s : W.sig2_x);
-  if (a2s > W.cut2) return;
-  const float coef = wca_coef(a2s, same ? W.pre_s : W.pre_x, W.maxPair);
-  const float sg = same ? W.sig_s : W.sig_x;
-  fx += __float2ll_rn(coef * (dx * sg) * W.scale);
-  fy += __float2ll_rn(coef * (dy * sg) * W.scale);
-}
-
-// Re-binning of one axis after a move (refresh_erwNachbar,
-// dynamik_methoden.cpp:216-325): the cell moves by floor(off/B) and the
-// offset becomes fmod(off + B, B). For off in [-B, 0) the new offset is
-// off + B, kept as is when FP32 rounds it to B (a legal offset) instead of
-// wrapping to 0, which would move the particle by a whole cell. For
-// off < -B the reference's fmod keeps a negative offset; reproduced.
-__device__ inline void rebin_axis(float off, float B, int& n, float& no) {
-  if (off >= 0.0f && off < B) {
-    n = 0;
-    no = off;
-  } else if (off == B) {
-    n = 1;
-    no = 0.0f;
-  } else if (off > B && off < 2.0f * B) {
-    n = 1;
-    no = off - B;
-  } else if (off < 0.0f && off >= -B) {
-    n = -1;
-    no = off + B;
-  } else if (off >= 2.0f * B) {
-    const float fl = floorf(off / B);
-    n = (int)fl;
-    no = fmaf(-fl, B, off);
-    if (no >= B) {
-      no -= B;
-      n++;
-    } else if (no < 0.0f) {
-      no += B;
-      n--;
-    }
-  } else if (off < -B) {
-    n = (int)floorf(off / B);
-    no = fmodf(off + B, B);
-  } else {  // NaN
-    n = 0;
-    no = off;
-  }
-}
-
-struct StepOut {
-  Rec r;
-  int key;
-};
-
-// Euler-Maruyama update (zeitschritt, dynamik_methoden.cpp:117-157) and
-// re-binning of one particle.
-__device__ inline Rec move_particle(const RunDesc& R, Rec p, float2 F, float2 xi, float dt,
-                                    int* err, bool apply = true) {
-  if (apply) {
-    const float sq = sqrtf(2.0f * R.T * dt);
-    p.ox += dt * F.x + sq * xi.x;
-    p.oy += dt * F.y + sq * xi.y;
-  }
-  if (apply && (R.flags & F_RADIAL) && p.pid >= R.N1) {
-    int ic, jc;
-    cell_ij(R, p.cell, ic, jc);
-    const double mitte = 0.5 * R.L_d;
-    const double x = ic * R.B_d + (double)p.ox;
-    const double y = jc * R.B_d + (double)p.oy;
-    const double dxm = mitte - x, dym = mitte - y;
-    const double abst = sqrt(dxm * dxm + dym * dym);
-    const int t = p.pid - R.N1;
-    // cos / sin of 2 pi t / N2 as sincospi (no large-argument reduction path)
-    double sn, cs;
-    sincospi(2.0 * t / R.N2, &sn, &cs);
-    p.ox = (float)((double)p.ox + (mitte + abst * cs - x));
-    p.oy = (float)((double)p.oy + (mitte + abst * sn - y));
-  }
-  if (!isfinite(p.ox) || !isfinite(p.oy)) {
-    atomicOr(err, E_NONFINITE);
-    return p;
-  }
-  if (p.ox < 0.0f || p.ox > R.B || p.oy < 0.0f || p.oy > R.B) {
-    int nx, ny;
-    float ox, oy;
-    rebin_axis(p.ox, R.B, nx, ox);
-    rebin_axis(p.oy, R.B, ny, oy);
-    int ic, jc;
-    cell_ij(R, p.cell, ic, jc);
-    const int icn = wrapi(ic + nx, R.C), jcn = wrapi(jc + ny, R.C);
-    p.cell = icn * R.C + jcn;
-    p.ox = ox;
-    p.oy = oy;
-  }
-  return p;
-}
-
-// optimaler_zeitschritt bound of one component (dynamik_methoden.cpp:1420-1491):
-// dt < (w-|u|)^2 with u = xi sqrt(T/2)/F, w = sqrt(u^2 + m/|F|). In FP32
-// w - |u| cancels when u^2 >> m/|F|, so it is evaluated as the equal
-// (m/|F|) / (w + |u|).
-__device__ inline float dt_bound(float F, float nz, float mrd, float T) {
-  if (fabsf(F) < 1.0e-5f) return mrd * mrd / (2.0f * T * nz * nz);
-  const float u = nz * sqrtf(0.5f * T) / F;
-  const float a = mrd / fabsf(F);
-  const float w = sqrtf(u * u + a);
-  const float d = a / (w + fabsf(u));
-  return d * d;
-}
-
-
-template <bool NC, bool DEP>
-__device__ inline void finish_particle(const RunDesc& R, RunDyn& D, int mode, int mask,
-                                       const Rec& p, int ic, int jc, int gi, float2 Fw);
-
-template <bool NC>
-__device__ __forceinline__ Rec ldrec(const Rec* q) {
-  const int4 v = ldm<NC>(reinterpret_cast<const int4*>(q));
-  Rec r;
-  r.ox = __int_as_float(v.x);
-  r.oy = __int_as_float(v.y);
-  r.cell = v.z;
-  r.pid = v.w;
-  return r;
-}
-
-// WCA sum of particle p (at global index self, cell (ic, jc)) over the 3x3
-// neighbour cells, read straight from the cell-sorted array: per neighbour
-// row the cells jc-1, jc, jc+1 form one contiguous range unless the row
-// wraps. The fixed-point sum makes the result independent of the order of
-// the particles within a cell.
-template <bool NC>
-__device__ inline float2 wca_direct(const RunDesc& R, const Rec& p, int ic, int jc, int self, int m) {
-  long long fx = 0, fy = 0;
-  const WcaP W = wca_params(R, p, m);
-  const int C = R.C;
-  const Rec* rec = R.recA;
-  const int* start = R.start;
-  if (jc >= 1 && jc <= C - 2) {
-    // per neighbour row one contiguous range (cells jc-1 .. jc+1); the six
-    // bounds are loaded together
-    int beg[3], end[3];
-#pragma unroll
-    for (int a = 0; a < 3; a++) {
-      const int row = wrap1(ic + a - 1, C) * C;
-      beg[a] = ldm<NC>(&start[row + jc - 1]);
-      end[a] = ldm<NC>(&start[row + jc + 2]);
-    }
-#pragma unroll
-    for (int a = 0; a < 3; a++) {
-      const int cmid = wrap1(ic + a - 1, C) * C + jc;
-      if constexpr (!NC) {
-        // fused step (registers to spare): the next record is requested
-        // before the current pair is evaluated
-        Rec q;
-        if (beg[a] < end[a]) q = ldrec<NC>(&rec[beg[a]]);
-        for (int j = beg[a]; j < end[a]; j++) {
-          Rec qn = q;
-          if (j + 1 < end[a]) qn = ldrec<NC>(&rec[j + 1]);
-          if (j != self) wca_pair(W, p, q, a - 1, q.cell - cmid, fx, fy);
-          q = qn;
-        }
-      } else {
-        for (int j = beg[a]; j < end[a]; j++) {
-          if (j == self) continue;
-          const Rec q = ldrec<NC>(&rec[j]);
-          wca_pair(W, p, q, a - 1, q.cell - cmid, fx, fy);
-        }
-      }
-    }
-  } else {
-#pragma unroll 1
-    for (int da = -1; da <= 1; da++) {
-      const int row = wrap1(ic + da, C) * C;
-#pragma unroll 1
-      for (int db = -1; db <= 1; db++) {
-        const int g = row + wrap1(jc + db, C);
-        const int beg = ldm<NC>(&start[g]), end = ldm<NC>(&start[g + 1]);
-        for (int j = beg; j < end; j++) {
-          if (j == self) continue;
-          wca_pair(W, p, ldrec<NC>(&rec[j]), da, db, fx, fy);
-        }
-      }
-    }
-  }
-  const double inv = 1.0 / (double)W.scale;
-  return make_float2((float)((double)fx * inv), (float)((double)fy * inv));
-}
-
-// Forces and (MODE_STEP) the move of the particle at sorted index gi; DEP:
-// the move also deposits the new position into R.dacc.
-template <bool NC, bool DEP>
-__device__ __forceinline__ void particle_item(const RunDesc& R, RunDyn& D, int gi, int mode, int mask) {
-  const Rec p = ldrec<NC>(&R.recA[gi]);
-  int ic, jc;
-  cell_ij(R, p.cell, ic, jc);
-  int m = mask;
-  if (mode == MODE_SET) m &= p.pid >= R.N1 ? 2 : 1;
-  if (R.flags & F_IDGAS) m = 0;
-  const float2 Fw = m ? wca_direct<NC>(R, p, ic, jc, gi, m) : make_float2(0.f, 0.f);
-  finish_particle<NC, DEP>(R, D, mode, mask, p, ic, jc, gi, Fw);
-}
-
-// One thread per particle of the cell-sorted array.
-// deposit (MODE_STEP): the move adds the next step's density to each run's
-// accumulator R.dacc (the pipelined stage step, whose forward row pass reads it)
+// The step's particle kernel: forces, noise, move, re-binning and counts, one
+// thread per particle of the cell-sorted array. DEP: the move adds the next
+// step's density to each run's accumulator R.dacc (the pipelined stage step,
+// whose forward row pass reads it). A kernel of its own, not a mode of
+// k_particles: the pair loop tests no mask and less code is fetched.
 // MINB: CTAs per SM the compiler keeps registers for (4: at most 64
 // registers; 5: at most 51, more warps resident, a few values reloaded from
 // local memory); the batch autotuner picks one, the arithmetic is the same.
+template <int MINB, bool DEP>
+__global__ void __launch_bounds__(256, MINB) k_step(const RunDesc* __restrict__ runs, RunDyn* __restrict__ dyn,
+                                                    const Item* __restrict__ items, int nitems) {
+  for (int it = blockIdx.x; it < nitems; it += gridDim.x) {
+    const Item I = items[it];
+    const bool on = run_active(dyn, I.run);
+    // the pipelined step: the run's first block records whether the run takes
+    // part in this step, for the sort and transform kernels that follow (the
+    // step end changes the budget while they run)
+    if (DEP && I.a == 0 && threadIdx.x == 0) dyn[I.run].sorting = on ? 1 : 0;
+    if (!on) continue;
+    const RunDesc& R = runs[I.run];
+    const int gi = I.a * blockDim.x + threadIdx.x;
+    if (gi >= R.N) continue;
+    particle_item<true, DEP>(R, dyn[I.run], dyn[I.run].step, gi, MODE_STEP, 7);
+  }
+}
+
+// Forces only, stored by particle index: the drop-in WCA routines (MODE_SET,
+// MODE_ADD with their pair mask) and the adaptive step's (MODE_FORCES).
 template <int MINB>
 __global__ void __launch_bounds__(256, MINB) k_particles(const RunDesc* __restrict__ runs,
                                                    RunDyn* __restrict__ dyn,
                                                    const Item* __restrict__ items, int nitems,
-                                                   int mode, int mask, int require_active, int deposit) {
+                                                   int mode, int mask, int require_active) {
   for (int it = blockIdx.x; it < nitems; it += gridDim.x) {
     const Item I = items[it];
-    // the pipelined step (deposit): the run's first block records whether
-    // the run takes part in this step, for the sort and transform kernels
-    // that follow (the step end changes the budget while they run)
-    if (deposit && I.a == 0 && threadIdx.x == 0) dyn[I.run].sorting = run_active(dyn, I.run) ? 1 : 0;
     if (require_active && !run_active(dyn, I.run)) continue;
     const RunDesc& R = runs[I.run];
     const int gi = I.a * blockDim.x + threadIdx.x;
     if (gi >= R.N) continue;
-    if (deposit) particle_item<true, true>(R, dyn[I.run], gi, mode, mask);
-    else particle_item<true, false>(R, dyn[I.run], gi, mode, mask);
+    particle_item<true, false>(R, dyn[I.run], dyn[I.run].step, gi, mode, mask);
   }
-}
-
-
-// Count particle gi into its new cell (an add whose result nobody waits for;
-// the scatter takes the slots) and into the per-chunk total for the scan,
-// added once per group of lanes in the same chunk (neighbouring particles of
-// the cell-sorted order mostly share one). The cell is the key: the scatter
-// reads it from the record recB[gi].
-__device__ __forceinline__ void count_into_cell(const RunDesc& R, int gi, int key) {
-  atomicAdd(&R.count[key], 1);
-  const int ch = key / SCAN_CHUNK;
-  const unsigned grp = __match_any_sync(__activemask(), ch);
-  if ((threadIdx.x & 31) == __ffs(grp) - 1) atomicAdd(&R.chunk_sum[ch], __popc(grp));
-}
-
-// Everything after the WCA sum: store it (MODE_SET/ADD), or add the mesh
-// force and the noise and store the forces (MODE_FORCES) or move and re-bin
-// (MODE_STEP).
-template <bool NC, bool DEP>
-__device__ inline void finish_particle(const RunDesc& R, RunDyn& D, int mode, int mask,
-                                       const Rec& p, int ic, int jc, int gi, float2 Fw) {
-  const bool sp2 = p.pid >= R.N1;
-  if (mode == MODE_SET) {
-    if ((mask & (sp2 ? 2 : 1))) R.Fw[p.pid] = Fw;
-    return;
-  }
-  if (mode == MODE_ADD) {
-    float2 f = R.Fw[p.pid];
-    f.x += Fw.x;
-    f.y += Fw.y;
-    R.Fw[p.pid] = f;
-    return;
-  }
-  const float2 Fk = (R.flags & F_IDGAS) ? make_float2(0.f, 0.f) : mesh_force<NC>(R, p, ic, jc, R.scheme);
-  float2 xi = make_float2(0.f, 0.f);
-  if (!(R.flags & F_NOWCA)) xi = particle_noise(R.noise, R.seed, D.step, (uint32_t)p.pid);
-  if (mode == MODE_FORCES) {
-    R.Fw[p.pid] = Fw;
-    R.Fk[p.pid] = Fk;
-    R.Fn[p.pid] = xi;
-    float bnd = fminf(dt_bound(Fw.x + Fk.x, xi.x, R.mrd, R.T), dt_bound(Fw.y + Fk.y, xi.y, R.mrd, R.T));
-    if (!(bnd >= 0.f)) bnd = 3.0e38f;  // NaN never wins the minimum (std::min semantics)
-    if (bnd < R.dt_max) atomicMin(&D.dt_bits, __float_as_uint(bnd));
-    return;
-  }
-  // MODE_STEP
-  const float2 F = make_float2(Fw.x + Fk.x, Fw.y + Fk.y);
-  const Rec np = move_particle(R, p, F, xi, R.dt_max, &D.err);
-  R.recB[gi] = np;
-  count_into_cell(R, gi, np.cell);
-  // the fused step and the pipelined stage step: the next step's density
-  if constexpr (DEP) deposit_acc(R, np);
-  if (np.cell != p.cell) atomicAdd(&D.moved[sp2 ? 1 : 0], 1);  // num_Zellwechsel of TimestepInfo
 }
 
 // Move from stored forces (adaptive dt: the reduced bound; fixed dt: dt_max),
@@ -1089,26 +498,8 @@ __global__ void __launch_bounds__(256) k_count(const RunDesc* __restrict__ runs,
 // cell of the particle-index order gives, which is the reference's
 // neighbour-list order after WCA_init (ascending index).
 
-// End of a step (one thread per run): advance the Philox step counter, the
-// simulated time and the steps budget; re-arm the adaptive dt reduction.
-__device__ inline void end_step(const RunDesc& R, RunDyn& D, int adaptive) {
-  double dt = R.dt_max_d;
-  if (adaptive && (R.flags & F_ADAPTIVE)) {
-    const float b = __uint_as_float(D.dt_bits);
-    dt = b < R.dt_max ? (double)b : R.dt_max_d;
-  }
-  D.dt = (float)dt;
-  D.t += dt;
-  D.step++;
-  D.steps_left--;
-  D.dt_bits = __float_as_uint(3.0e38f);
-  D.moved_last[0] = D.moved[0];
-  D.moved_last[1] = D.moved[1];
-  D.moved[0] = D.moved[1] = 0;
-}
-
 // Exclusive scan of one run's chunk totals into chunk_off; clears the
-// totals. With end_step (the fused step's sort) its thread 0 also ends the
+// totals. With end_step (a step's sort) its thread 0 also ends the
 // run's step: the particle kernels that read the step counter and the dt
 // bound are done, the scan and the scatter do not read them.
 __global__ void __launch_bounds__(1024) k_chunk_scan(const RunDesc* __restrict__ runs, RunDyn* __restrict__ dyn,
@@ -1178,36 +569,6 @@ __device__ __forceinline__ void scan_load(const RunDesc* __restrict__ runs, cons
   }
 }
 
-// start[] of one chunk from its counts v (eight per thread) and its offset.
-// The counts stay: the scatter counts them down to zero as it takes slots.
-// All threads call; sh: 32 ints.
-__device__ __forceinline__ void scan_chunk_store(const RunDesc& R, int chunk, int ncells, const int* v, int off,
-                                                 int* sh) {
-  constexpr int PER = SCAN_CHUNK / 256;
-  const int base = chunk * SCAN_CHUNK;
-  const int c0 = base + threadIdx.x * PER;
-  int loc = 0;
-#pragma unroll
-  for (int k = 0; k < PER; k++) loc += v[k];
-  int acc = block_excl_scan(loc, sh) + off;
-  int w[PER];
-#pragma unroll
-  for (int k = 0; k < PER; k++) {
-    w[k] = acc;
-    acc += v[k];
-  }
-  if (base + SCAN_CHUNK <= ncells) {
-    *reinterpret_cast<int4*>(&R.start[c0]) = make_int4(w[0], w[1], w[2], w[3]);
-    *reinterpret_cast<int4*>(&R.start[c0 + 4]) = make_int4(w[4], w[5], w[6], w[7]);
-  } else {
-#pragma unroll
-    for (int k = 0; k < PER; k++)
-      if (c0 + k < ncells) R.start[c0 + k] = w[k];
-  }
-  if (base + SCAN_CHUNK >= ncells && threadIdx.x == 0) R.start[ncells] = R.N;
-  __syncthreads();  // sh is reused by the next scan
-}
-
 __global__ void __launch_bounds__(256) k_scan(const RunDesc* __restrict__ runs, const RunDyn* __restrict__ dyn,
                                               const Item* __restrict__ items, int nitems, int require_active) {
   static_assert(SCAN_CHUNK == 2048, "eight counts per thread");
@@ -1219,19 +580,11 @@ __global__ void __launch_bounds__(256) k_scan(const RunDesc* __restrict__ runs, 
   for (;;) {
     const int itn = it + gridDim.x;
     if (itn < nitems) scan_load(runs, dyn, items[itn], require_active, nxt);
-    if (cur.on) scan_chunk_store(*cur.R, cur.chunk, cur.ncells, cur.v, cur.R->chunk_off[cur.chunk], sh);
+    if (cur.on) scan_chunk_store<SCAN_CHUNK / 256>(CtaTeam(), *cur.R, cur.chunk, cur.ncells, cur.v, cur.R->chunk_off[cur.chunk], sh);
     if (itn >= nitems) break;
     it = itn;
     cur = nxt;
   }
-}
-
-// Particle gi of the old order to start[cell] + slot, the slot taken by
-// counting the cell's count down (which leaves it zero for the next sort).
-__device__ __forceinline__ void scatter_particle(const RunDesc& R, int gi) {
-  const Rec q = R.recB[gi];
-  const int slot = atomicSub(&R.count[q.cell], 1) - 1;
-  R.recA[R.start[q.cell] + slot] = q;
 }
 
 // Places every particle at start[cell] + slot (slots in atomic order: the
@@ -1250,14 +603,13 @@ __global__ void __launch_bounds__(256) k_scatter(const RunDesc* __restrict__ run
   }
 }
 
-
 // ---------------------------------------------------------------------------
 // Pipelined stage step: any number of runs on power-of-two meshes with a
-// fixed dt, six launches per step. As in the fused step, the move deposits
+// fixed dt, six launches per step. As in the resident step, the move deposits
 // the next step's density (the same fixed-point integers as the tiles, into
 // each run's R.dacc), and the transform of the new density runs beside the
 // cell sort:
-//   k_particles     forces, noise, move, re-binning, counts, next density;
+//   k_step          forces, noise, move, re-binning, counts, next density;
 //                   marks the runs that take part (`sorting`)
 //   then, on two streams joined at the step's end:
 //   k_pipe_scan -> k_pipe_scatter (step end)
@@ -1275,9 +627,9 @@ __device__ __forceinline__ void pipe_fft_item(const RunDesc& R, const Item& I, f
   switch (I.b) {
 #define BD_CASE(L)                                                      \
   case L:                                                               \
-    if (PASS == 0) fft2_rows_inv_item<L, false>(R, I.a, I.c, s, R.tw);       \
-    else if (PASS == 1) fft2_rows_fwd_item<L, false, true>(R, I.a, I.c, s, R.tw); \
-    else fft2_cols_item<L, false>(R, I.a, I.c, s, R.tw);                    \
+    if (PASS == 0) fft2_rows_inv_item<L, false>(CtaTeam(), R, I.a, I.c, s, R.tw);       \
+    else if (PASS == 1) fft2_rows_fwd_item<L, false, true>(CtaTeam(), R, I.a, I.c, s, R.tw); \
+    else fft2_cols_item<L, false>(CtaTeam(), R, I.a, I.c, s, R.tw);                    \
     break;
     BD_PIPE_SIZES(BD_CASE)
 #undef BD_CASE
@@ -1321,7 +673,7 @@ __device__ __forceinline__ void scan_chunk_item(const RunDesc& R, int c, int* s_
   int cv[PER];
 #pragma unroll
   for (int k = 0; k < PER; k++) cv[k] = c0 + k < ncells ? R.count[c0 + k] : 0;
-  scan_chunk_store(R, c, ncells, cv, off, s_tmp);
+  scan_chunk_store<SCAN_CHUNK / 256>(CtaTeam(), R, c, ncells, cv, off, s_tmp);
 }
 
 // PIPE_SCAN_GROUP chunks of one run per CTA (Item.a: the first): the counts
@@ -1508,304 +860,6 @@ __global__ void k_green(float* __restrict__ green, float* __restrict__ sxt,
 }
 
 // ---------------------------------------------------------------------------
-// Fused step: one run on a power-of-two mesh up to 1024^2 with a fixed dt.
-// Every stage of the step runs in one cooperative launch (all CTAs
-// resident), separated by grid-wide barriers: the launch and drain gaps
-// between the stage kernels disappear, which is most of a step's time on
-// meshes this small. Data written within the launch is read
-// with plain (coherent) loads, never through the read-only cache.
-
-constexpr unsigned BAR_MAX_POLLS = 1u << 22;
-// set in the arrival counter by a CTA whose wait gave up: every CTA that
-// sees it fails the barrier
-constexpr unsigned BAR_POISON = 0x80000000u;
-
-// Grid-wide barrier: bar[0] counts arrivals (a release add; waiters poll it
-// with acquire loads until it reaches target = barriers so far x grid), so
-// the writes of every CTA before the barrier are visible to all after it.
-// bar[1] counts CTAs leaving the launch; the last one clears both words for
-// the next launch. A wait gives up after max_polls polls: it sets the poison
-// bit with a compare-and-swap that succeeds only while the count is short of
-// the target, so either the last arrival comes first and every CTA passes,
-// or the poison comes first and every CTA (late arrivals included) fails
-// this barrier and returns: no CTA runs past a failed barrier. The failure
-// is reported as E_BARRIER_TIMEOUT; the host clears the words.
-__device__ bool grid_barrier(unsigned* bar, unsigned target, unsigned max_polls, int* err, int* s_ok) {
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    cuda::atomic_ref<unsigned, cuda::thread_scope_device> c(bar[0]);
-    c.fetch_add(1u, cuda::memory_order_release);
-    int ok = 1;
-    for (unsigned polls = 0;; polls++) {
-      unsigned v = c.load(cuda::memory_order_acquire);
-      if (v & BAR_POISON) {
-        ok = 0;
-        break;
-      }
-      if (v >= target) break;
-      if (polls >= max_polls) {
-        while (!(v & BAR_POISON) && v < target)
-          if (c.compare_exchange_weak(v, v | BAR_POISON, cuda::memory_order_acq_rel, cuda::memory_order_acquire))
-            v |= BAR_POISON;
-        if (v & BAR_POISON) {
-          ok = 0;
-          atomicOr(err, E_BARRIER_TIMEOUT);
-        }
-        break;
-      }
-      __nanosleep(20);
-    }
-    *s_ok = ok;
-  }
-  __syncthreads();
-  return *s_ok != 0;
-}
-
-__device__ void grid_exit(unsigned* bar) {
-  if (threadIdx.x == 0 && atomicAdd(&bar[1], 1u) == gridDim.x - 1) {
-    atomicExch(&bar[0], 0u);
-    atomicExch(&bar[1], 0u);
-  }
-}
-
-constexpr size_t FUSED_TW_BYTES(int lz) { return (((size_t)8 << lz) + 255) & ~(size_t)255; }
-
-// The run's description is a kernel parameter (constant bank), so its fields
-// take no registers across the phases.
-__device__ __forceinline__ unsigned long long global_ns() {
-  unsigned long long t;
-  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-  return t;
-}
-
-// Bring this CTA's share (1/G, 256-byte aligned pieces) of a device array
-// into L2 with one bulk prefetch (no data moves to the SM; the base must be
-// 16-byte aligned, as cudaMalloc's are). Issued by one thread.
-__device__ __forceinline__ void l2_prefetch_share(const void* base, size_t bytes, int b, int G) {
-  const size_t per = ((bytes + G - 1) / G + 255) & ~(size_t)255;
-  const size_t off = (size_t)b * per;
-  if (off >= bytes) return;
-  const size_t len = (bytes - off < per ? bytes - off : per) & ~(size_t)15;
-  if (len == 0) return;
-  asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"((const char*)base + off), "r"((unsigned)len)
-               : "memory");
-}
-
-// ts (optional, FUSED_PHASES + 1 entries): CTA 0 records the global timer
-// at the start and after every phase's barrier.
-template <int LZ>
-__global__ void __launch_bounds__(256, 2) k_fused(const __grid_constant__ RunDesc R, RunDyn* __restrict__ dyn,
-                                               const __grid_constant__ FusedPlan P, unsigned* bar,
-                                               unsigned long long* ts) {
-  extern __shared__ __align__(16) unsigned char smem[];
-  __shared__ int s_tmp[32];
-  __shared__ int s_ok;
-  constexpr int Z = 1 << LZ;
-  RunDyn& D = dyn[0];
-  volatile RunDyn& Dv = dyn[0];
-  // the spectrum rows of this CTA's inverse row item go to L2 first, then the
-  // twiddles are requested together with the step budget (independent loads,
-  // all from DRAM after the caches were flushed)
-  if (threadIdx.x == 0 && (int)blockIdx.x < P.nri)
-    l2_prefetch_share(R.spec2 + ((size_t)blockIdx.x << P.lri) * (Z / 2), ((size_t)1 << P.lri) * (Z / 2) * sizeof(float4),
-                      0, 1);
-  constexpr int TWR = (Z + 255) / 256;
-  float2 twr[TWR];
-#pragma unroll
-  for (int k = 0; k < TWR; k++)
-    if (threadIdx.x + 256 * k < Z) twr[k] = R.tw[threadIdx.x + 256 * k];
-  // the budget is checked after the inverse row pass (which only rebuilds
-  // the force grid from the unchanged spectrum), so its load does not hold up
-  // the start; nothing in this launch changes it before the end
-  const long long steps_left = Dv.steps_left;
-  // What the later phases read first from memory (particles, cell starts and
-  // counts in the particle pass, and the density accumulator its move adds
-  // to; the Green's tables in the column pass) is requested into L2 now,
-  // behind the inverse row pass.
-  if (threadIdx.x == 0) {
-    const int nZ = (1 << LZ) / 2 + 1;
-    l2_prefetch_share(R.green, (size_t)(1 << LZ) * nZ * sizeof(float), blockIdx.x, gridDim.x);
-    l2_prefetch_share(R.recA, (size_t)R.N * sizeof(Rec), blockIdx.x, gridDim.x);
-    l2_prefetch_share(R.start, ((size_t)R.C * R.C + 1) * sizeof(int), blockIdx.x, gridDim.x);
-    l2_prefetch_share(R.count, (size_t)R.C * R.C * sizeof(int), blockIdx.x, gridDim.x);
-    l2_prefetch_share(R.dacc, ((size_t)1 << (2 * LZ)) * sizeof(unsigned long long), blockIdx.x, gridDim.x);
-    if (blockIdx.x == 0) {
-      l2_prefetch_share(R.sxt, (size_t)(1 << LZ) * sizeof(float), 0, 1);
-      l2_prefetch_share(R.syt, (size_t)nZ * sizeof(float), 0, 1);
-    }
-  }
-  float2* tws = (float2*)smem;
-  float2* work = (float2*)(smem + FUSED_TW_BYTES(LZ));
-#pragma unroll
-  for (int k = 0; k < TWR; k++)
-    if (threadIdx.x + 256 * k < Z) tws[threadIdx.x + 256 * k] = twr[k];
-  const unsigned G = gridDim.x;
-  // each CTA takes an equal contiguous share of the particles (the busiest
-  // SM then holds two shares, not two full CTAs of 256 while others hold one)
-  const int per = (R.N + (int)G - 1) / (int)G;
-  const int ncells = R.C * R.C;
-  const int b = blockIdx.x;
-  unsigned ep = 0;
-  int ph = 0;
-  const bool rec = ts && b == 0 && threadIdx.x == 0;
-  if (rec) ts[ph] = global_ns();
-  const unsigned maxp = P.max_polls ? P.max_polls : BAR_MAX_POLLS;
-  // next grid barrier; false: it failed, the CTA returns. The recovery-path
-  // test makes one CTA leave instead of arriving (CTA-uniform condition).
-  auto barrier = [&]() -> bool {
-    if (P.skip_barrier == (int)ep + 1 && b == P.skip_cta) return false;
-    return grid_barrier(bar, ++ep * G, maxp, &D.err, &s_ok);
-  };
-#define BD_BARRIER()        \
-  if (!barrier()) return; \
-  if (rec) ts[++ph] = global_ns()
-  // The mesh transform is pipelined across the step boundary: this step's
-  // density was deposited by the previous step's move and its forward row
-  // and column passes ran beside that step's scan and scatter (or, after the
-  // positions changed elsewhere, the host ran them before this launch). The
-  // step starts at the inverse row pass. A transform item runs at most once
-  // per call site and CTA (the host sizes them so; a loop around a transform
-  // would make the compiler keep the addresses of all its passes live).
-  if (b < P.nri) fft2_rows_inv_item<LZ, true>(R, b << P.lri, P.lri, work, tws);
-  BD_BARRIER();
-  if (steps_left <= 0) {  // uniform
-    grid_exit(bar);
-    return;
-  }
-  // forces, noise, move, re-binning, counts, the next step's density
-  for (int i = threadIdx.x; i < per; i += blockDim.x) {
-    const int gi = b * per + i;
-    if (gi < R.N) particle_item<false, true>(R, D, gi, MODE_STEP, 7);
-  }
-  BD_BARRIER();
-  // chunk offsets: each CTA sums the totals before its chunk (few chunks),
-  // else CTA 0 scans them first
-  const bool own = P.nch <= 512;
-  if (!own) {
-    if (b == 0) {
-      int loc = 0;
-      const int per = (P.nch + blockDim.x - 1) / blockDim.x, k0 = threadIdx.x * per;
-      for (int k = 0; k < per; k++)
-        if (k0 + k < P.nch) loc += R.chunk_sum[k0 + k];
-      int ex = block_excl_scan(loc, s_tmp);
-      for (int k = 0; k < per; k++)
-        if (k0 + k < P.nch) {
-          const int v = R.chunk_sum[k0 + k];
-          R.chunk_off[k0 + k] = ex;
-          ex += v;
-        }
-    }
-    if (!barrier()) return;
-  }
-  for (int c = b; c < P.nch; c += G) {
-    int off;
-    if (own) {
-      int loc = 0;
-      for (int k = threadIdx.x; k < c; k += blockDim.x) loc += R.chunk_sum[k];
-      const int ex = block_excl_scan(loc, s_tmp);
-      __syncthreads();  // every thread has read s_tmp
-      if (threadIdx.x == blockDim.x - 1) s_tmp[0] = ex + loc;
-      __syncthreads();
-      off = s_tmp[0];
-      __syncthreads();
-    } else {
-      off = R.chunk_off[c];
-    }
-    constexpr int PER = SCAN_CHUNK / 256;
-    const int c0 = c * SCAN_CHUNK + threadIdx.x * PER;
-    int v[PER];
-#pragma unroll
-    for (int k = 0; k < PER; k++) v[k] = c0 + k < ncells ? R.count[c0 + k] : 0;
-    scan_chunk_store(R, c, ncells, v, off, s_tmp);
-  }
-  // beside the scan: the next step's forward row pass over the density the
-  // move deposited (items on the CTAs from the top down, the scan's chunks
-  // are on the lowest)
-  {
-    const int it = (int)G - 1 - b;
-    if (it < P.nrf) fft2_rows_fwd_item<LZ, true, true>(R, it << P.lrf, P.lrf, work, tws);
-  }
-  BD_BARRIER();
-  for (int i = threadIdx.x; i < per; i += blockDim.x) {
-    const int gi = b * per + i;
-    if (gi < R.N) scatter_particle(R, gi);
-  }
-  // beside the scatter: the next step's column pass and Green's multiply
-  {
-    const int it = (int)G - 1 - b;
-    if (it < P.ncl) fft2_cols_item<LZ, true>(R, it << P.lw, P.lw, work, tws);
-  }
-  if (b == 0) {
-    for (int k = threadIdx.x; k < P.nch; k += blockDim.x) R.chunk_sum[k] = 0;
-    if (threadIdx.x == 0) end_step(R, D, 0);
-  }
-  if (ts) {
-    // the last phase ends when every CTA has scattered and transformed
-    if (!barrier()) return;
-    if (rec) ts[++ph] = global_ns();
-  }
-  grid_exit(bar);
-#undef BD_BARRIER
-}
-
-#define BD_FUSED_SIZES(X) X(3) X(4) X(5) X(6) X(7) X(8) X(9) X(10)
-
-int fused_configure(FusedPlan& P, int device) {
-  const int Z = 1 << P.lz, n = Z / 2;
-  const size_t rf = (size_t)(1 << P.lrf) * fft2_stride(n) * 8;
-  const size_t cl = (size_t)2 * (1 << P.lw) * fft2_stride(Z) * 8;
-  const size_t ri = (size_t)(1 << P.lri) * fft2_stride(Z) * 8;
-  P.smem = FUSED_TW_BYTES(P.lz) + std::max(rf, std::max(cl, ri));
-  int nsm = 0, per = 0;
-  cudaError_t e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, device);
-  if (e != cudaSuccess) return (int)e;
-  switch (P.lz) {
-#define BD_CASE(L)                                                                                \
-  case L:                                                                                         \
-    e = cudaFuncSetAttribute(k_fused<L>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)P.smem); \
-    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_fused<L>, 256, P.smem); \
-    break;
-    BD_FUSED_SIZES(BD_CASE)
-#undef BD_CASE
-    default:
-      return (int)cudaErrorInvalidValue;
-  }
-  if (e != cudaSuccess) return (int)e;
-  if (per <= 0) return (int)cudaErrorInvalidConfiguration;
-  // two CTAs per SM: more make every grid barrier slower than they gain
-  P.grid = std::min(per, 2) * nsm;
-  return 0;
-}
-
-int launch_fused(const RunDesc& run, RunDyn* dyn, const FusedPlan& P, unsigned* bar, cudaStream_t s,
-                 unsigned long long* ts) {
-  cudaError_t e;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(P.grid);
-  cfg.blockDim = dim3(256);
-  cfg.dynamicSmemBytes = P.smem;
-  cfg.stream = s;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeCooperative;
-  attr[0].val.cooperative = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  RunDesc rd = run;
-  rd.dacc = P.dacc;  // only the fused kernel's copy carries the accumulator
-  switch (P.lz) {
-#define BD_CASE(L)                                                 \
-  case L:                                                          \
-    e = cudaLaunchKernelEx(&cfg, k_fused<L>, rd, dyn, P, bar, ts); \
-    break;
-    BD_FUSED_SIZES(BD_CASE)
-#undef BD_CASE
-    default:
-      return (int)cudaErrorInvalidValue;
-  }
-  return (int)e;
-}
-
-// ---------------------------------------------------------------------------
 // Two-launch pipelined step (any number of runs on power-of-two meshes with a
 // fixed dt): the particle kernel, then one cooperative launch that holds the
 // rest of the step and the start of the next, its phases separated by grid
@@ -1822,7 +876,6 @@ int launch_fused(const RunDesc& run, RunDyn* dyn, const FusedPlan& P, unsigned* 
 // run beside the bandwidth-bound sort, which two kernels on two streams did
 // not: the first kernel's CTAs filled the GPU before the second's started.
 
-
 // meshes of the two-launch form (the host keeps larger ones on six launches)
 #define BD_TAIL_FFT_SIZES(X) X(3) X(4) X(5) X(6) X(7) X(8) X(9) X(10)
 
@@ -1835,9 +888,9 @@ template <int PASS, int L>
 __device__ __noinline__ void tail_fft_sized(const RunDesc* R, int a, int c) {
   extern __shared__ __align__(16) unsigned char smem[];
   float2* s = (float2*)smem;
-  if (PASS == 0) fft2_rows_inv_item<L, false>(*R, a, c, s, R->tw);
-  else if (PASS == 1) fft2_rows_fwd_item<L, false, true>(*R, a, c, s, R->tw);
-  else fft2_cols_item<L, false>(*R, a, c, s, R->tw);
+  if (PASS == 0) fft2_rows_inv_item<L, false>(CtaTeam(), *R, a, c, s, R->tw);
+  else if (PASS == 1) fft2_rows_fwd_item<L, false, true>(CtaTeam(), *R, a, c, s, R->tw);
+  else fft2_cols_item<L, false>(CtaTeam(), *R, a, c, s, R->tw);
 }
 
 template <int PASS>
@@ -2402,8 +1455,8 @@ static int launch_fft2(int pass, int lz, const RunDesc* runs, const RunDyn* dyn,
 }
 
 int launch_fft(const RunDesc* runs, const RunDyn* dyn, const FftPass gen[3], const Fft2Group* g2, int ng2,
-               int require_active, cudaStream_t s, cudaEvent_t* ev, int npass) {
-  for (int pass = 0; pass < npass && pass < 3; pass++) {
+               int require_active, cudaStream_t s, cudaEvent_t* ev, int first, int last) {
+  for (int pass = first; pass <= last; pass++) {
     const FftPass& g = gen[pass];
     if (g.n > 0) {
       if (pass == 0)
@@ -2424,7 +1477,18 @@ int launch_fft(const RunDesc* runs, const RunDyn* dyn, const FftPass gen[3], con
 }
 
 int launch_particles(const RunDesc* runs, RunDyn* dyn, const Item* items, int n, int mode,
-                     int mask, int require_active, cudaStream_t s, int deposit, int shape) {
+                     int mask, int require_active, cudaStream_t s, int shape) {
+  if (n <= 0) return 0;
+  const int g = grid_for(n, 65535);
+  if (shape == PART_SHAPE_5CTA)
+    k_particles<5><<<g, 256, 0, s>>>(runs, dyn, items, n, mode, mask, require_active);
+  else
+    k_particles<4><<<g, 256, 0, s>>>(runs, dyn, items, n, mode, mask, require_active);
+  BD_LAUNCH_CHECK();
+  return 0;
+}
+
+int launch_step(const RunDesc* runs, RunDyn* dyn, const Item* items, int n, int deposit, cudaStream_t s, int shape) {
   if (n <= 0) return 0;
   // The pipelined step (deposit): one wave of resident CTAs, each taking
   // items blockIdx.x, +gridDim.x, ... (256-run ensemble: particle phase
@@ -2436,15 +1500,18 @@ int launch_particles(const RunDesc* runs, RunDyn* dyn, const Item* items, int n,
   const int sh = shape == PART_SHAPE_5CTA ? 1 : 0;
   if (!resident[sh]) {
     int per = 0;
-    const cudaError_t e = sh ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_particles<5>, 256, 0)
-                             : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_particles<4>, 256, 0);
+    const cudaError_t e = sh ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_step<5, true>, 256, 0)
+                             : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_step<4, true>, 256, 0);
     resident[sh] = (e == cudaSuccess && per > 0) ? per : 1;
   }
   const int g = deposit ? grid_for(n, resident[sh] * sm_count()) : grid_for(n, 65535);
-  if (sh)
-    k_particles<5><<<g, 256, 0, s>>>(runs, dyn, items, n, mode, mask, require_active, deposit);
-  else
-    k_particles<4><<<g, 256, 0, s>>>(runs, dyn, items, n, mode, mask, require_active, deposit);
+  if (deposit) {
+    if (sh) k_step<5, true><<<g, 256, 0, s>>>(runs, dyn, items, n);
+    else k_step<4, true><<<g, 256, 0, s>>>(runs, dyn, items, n);
+  } else {
+    if (sh) k_step<5, false><<<g, 256, 0, s>>>(runs, dyn, items, n);
+    else k_step<4, false><<<g, 256, 0, s>>>(runs, dyn, items, n);
+  }
   BD_LAUNCH_CHECK();
   return 0;
 }
@@ -2526,7 +1593,6 @@ int launch_sort(const RunDesc* runs, RunDyn* dyn, int run0, int nruns, const Ite
   }
   return 0;
 }
-
 
 int launch_interp(const RunDesc* runs, const Item* items, int n, int scheme, cudaStream_t s) {
   if (n <= 0) return 0;

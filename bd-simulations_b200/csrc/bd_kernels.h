@@ -4,11 +4,9 @@
 #include <cstddef>
 #include <cuda_runtime.h>
 
-namespace bd {
+#include "bd_common.cuh"
 
-struct RunDesc;
-struct RunDyn;
-struct Rec;
+namespace bd {
 
 // Work item of a batched launch: run index plus up to three coordinates
 // whose meaning depends on the kernel (tile, row group, block, chunk).
@@ -45,19 +43,22 @@ struct Fft2Group {
 
 // rows forward, columns + Green, rows inverse: gen[] the kernels for meshes
 // with a factor 3 (radix 4/2/3), g2[] one group per power-of-two mesh size;
-// ev[0..2] (optional) recorded after each pass; npass < 3 stops early
+// ev[0..2] (optional) recorded after each pass; passes first .. last of 0 .. 2
 int launch_fft(const RunDesc* runs, const RunDyn* dyn, const FftPass gen[3], const Fft2Group* g2, int ng2,
-               int require_active, cudaStream_t s, cudaEvent_t* ev = nullptr, int npass = 3);
-// deposit (MODE_STEP): also add the new positions to each run's R.dacc.
-// shape: the compiled form of the particle kernel (same arithmetic):
+               int require_active, cudaStream_t s, cudaEvent_t* ev = nullptr, int first = 0, int last = 2);
+// shape: the compiled form of a particle kernel (same arithmetic):
 // PART_SHAPE_DEFAULT (registers for four 256-thread CTAs per SM) or
 // PART_SHAPE_5CTA (for five)
 enum PartShape { PART_SHAPE_DEFAULT = 0, PART_SHAPE_5CTA = 1 };
+// forces only: MODE_SET, MODE_ADD (mask: pair types) and MODE_FORCES
 int launch_particles(const RunDesc* runs, RunDyn* dyn, const Item* items, int n, int mode,
-                     int mask, int require_active, cudaStream_t s, int deposit = 0,
-                     int shape = PART_SHAPE_DEFAULT);
+                     int mask, int require_active, cudaStream_t s, int shape = PART_SHAPE_DEFAULT);
+// forces and move of the runs whose step budget is not used up; deposit: also
+// add the new positions to each run's R.dacc
+int launch_step(const RunDesc* runs, RunDyn* dyn, const Item* items, int n, int deposit, cudaStream_t s,
+                int shape = PART_SHAPE_DEFAULT);
 // Pipelined stage step (power-of-two meshes, fixed dt, every run with its
-// R.dacc): particles (launch_particles with deposit), then the scan and the
+// R.dacc): particles (launch_step with deposit), then the scan and the
 // scatter with the step end beside the transform of the new density:
 // forward rows (pass 1), columns + Green (pass 2), inverse rows (pass 0).
 // Transform items carry log2 Z in Item.b; smem is the largest item's shared
@@ -74,7 +75,7 @@ constexpr int PIPE_SCATTER_UNIT = 1024;
 int launch_pipe_scan(const RunDesc* runs, RunDyn* dyn, const Item* groups, int ngroup, cudaStream_t s);
 int launch_pipe_scatter(const RunDesc* runs, RunDyn* dyn, const Item* units, int nunit, const Item* chunks,
                         int nchunk, cudaStream_t s);
-// Two-launch form of the pipelined step: launch_particles (with deposit),
+// Two-launch form of the pipelined step: launch_step (with deposit),
 // then one cooperative launch of the sort and the transforms, phases C (scan
 // chunks and next forward rows), D (scatter, next columns + Green, step end)
 // and A (inverse rows: the next step's force grids). Unit lists:
@@ -110,41 +111,45 @@ int launch_records_by_pid(const Rec* src, Rec* dst, int n, cudaStream_t s);
 int launch_sort(const RunDesc* runs, RunDyn* dyn, int run0, int nruns, const Item* chunks, int nchunks,
                 const Item* parts, int nparts, int end_step_flag, int adaptive, int require_active, cudaStream_t s,
                 cudaEvent_t* ev = nullptr);
-// Fused step (one run, power-of-two mesh 2^lz with lz in [3, 10], fixed dt):
-// work sizes of its phases
-struct FusedPlan {
-  int lz;
-  int lrf, nrf;    // row items: 2^lrf rows, nrf items
-  int lw, ncl;     // column items
-  int lri, nri;    // inverse row items
-  int nch;         // scan chunks
-  size_t smem;     // dynamic shared memory
-  int grid;        // CTAs (all resident: cooperative launch)
-  unsigned long long* dacc;  // Z*Z density accumulator, zero between fused steps
+// phases of one step whose ends a single run's resident launch can time:
+// [0] inverse row FFT [1] particles (forces, noise, move, next density)
+// [2] cell-count scan + next row FFT [3] scatter + next column FFT + Green
+constexpr int FUSED_PHASES = 4;
+// Resident step (bd_resident.cuh): A.nsteps steps (at most each run's step
+// budget) of one run (SINGLE) or of every run of A.items in one launch.
+__host__ __device__ constexpr int res_threads(bool single) { return single ? 1024 : 512; }
+constexpr size_t res_max_smem(bool single) { return (single ? 200 : 112) * 1024; }  // one or two CTAs per SM
+constexpr int res_pcap(bool single) { return single ? 2048 : 1536; }  // particles of a CTA kept in shared memory
+__host__ __device__ constexpr int res_side(int lz) { return lz >= 16 ? 3 << (lz - 16) : lz ? 1 << lz : 0; }
+constexpr size_t RES_DESC_BYTES = 1024;   // the run's description
+__host__ __device__ constexpr size_t RES_TW_BYTES(int Z) {  // twiddles and sine tables
+  return ((size_t)8 * Z + 4 * (Z + Z / 2 + 1) + 255) & ~(size_t)255;
+}
+struct ResArgs {
+  RunDesc one;             // the single run (its dacc set)
+  Item one_item;           // its item: run 0, a/b/c = log2 rows forward, columns, rows inverse per item
+  const RunDesc* runs;     // run table (descriptions with dacc set)
+  RunDyn* dyn;
+  const Item* items;       // one per cluster: run, item sizes as above
+  int nsteps;
+  int part_off, pcap;      // the particles' place in shared memory and their number
+  int grid_mode;           // single run: the whole cooperative grid instead of one cluster
+  unsigned* bar;           // grid mode's two barrier words (zero; each launch leaves them zero)
   // grid-barrier waits give up after this many polls (0: the default bound,
   // about a second); a wait that gives up fails that barrier for every CTA
   unsigned max_polls;
   // recovery-path test: CTA skip_cta returns instead of arriving at barrier
   // skip_barrier (1-based; 0: none), so every other CTA's wait gives up
   int skip_barrier, skip_cta;
+  unsigned long long* ts;  // single run: FUSED_PHASES + 1 timestamps of one step (may be null)
 };
-// fills smem and grid (occupancy of the cooperative kernel); returns 0 or a
-// cudaError_t
-int fused_configure(FusedPlan& P, int device);
-// one step of one run (its description by value, its state in *dyn); bar:
-// the two device words of the grid barrier, zero before the first launch
-// (each launch leaves them zero). The FFT item counts nrf, ncl, nri must not
-// exceed grid. The step starts from the column-transformed, Green-multiplied
-// spectrum of the current positions (spec2), which the previous fused step
-// leaves behind; otherwise deposit + forward row and column passes must run
-// first (the stage kernels). It leaves the same for the next step, with the
-// accumulator dacc cleared again.
-// ts (optional): FUSED_PHASES + 1 device timestamps (ns) of the phase ends:
-// [0] inverse row FFT [1] particles (forces, noise, move, next density)
-// [2] cell-count scan + next row FFT [3] scatter + next column FFT + Green
-constexpr int FUSED_PHASES = 4;
-int launch_fused(const RunDesc& run, RunDyn* dyn, const FusedPlan& P, unsigned* bar, cudaStream_t s,
-                 unsigned long long* ts = nullptr);
+// lz: the mesh side: 2^lz (3..10), 3 * 2^(lz - 16) (20..24: 48 to 768), 0:
+// other meshes with a factor 3 and ideal-gas runs. cs: CTAs per cluster, 0: cooperative grid (single run).
+// resident_configure: attributes for smem bytes of dynamic shared memory;
+// *n: resident CTAs (cs 0) or clusters the device can hold at once
+int resident_configure(int lz, bool single, size_t smem, int cs, int device, int* n);
+int launch_resident(int lz, bool single, const ResArgs& A, int nclusters, int cs, int grid, size_t smem,
+                    cudaStream_t s);
 // TimestepInfo reductions of run 0 into acc (diag_bytes() of device memory):
 // energy, virial (double), largest |F|^2 << 32 | index of WCA, capillary,
 // noise forces (uint64 x 3), examined WCA pairs (uint64)

@@ -1,0 +1,45 @@
+// Dispatch of the resident step kernels by mesh size.
+#include "bd_kernels.h"
+
+namespace bd {
+
+template <int LZ, bool SINGLE>
+int resident_configure_t(size_t smem, int cs, int nsm, int* grid);
+template <int LZ, bool SINGLE>
+int launch_resident_t(const ResArgs& A, int nclusters, int cs, int grid, size_t smem, cudaStream_t s);
+
+#define BD_RES_SIZES(X) \
+  X(0) X(3) X(4) X(5) X(6) X(7) X(8) X(9) X(10) X(20) X(21) X(22) X(23) X(24)
+
+int resident_configure(int lz, bool single, size_t smem, int cs, int device, int* n) {
+  *n = 0;
+  int nsm = 0;
+  cudaError_t e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, device);
+  if (e != cudaSuccess) return (int)e;
+  switch (lz) {
+#define BD_CASE(L)                                                       \
+  case L:                                                                \
+    return single ? resident_configure_t<L, true>(smem, cs, nsm, n)      \
+                  : resident_configure_t<L, false>(smem, cs, nsm, n);
+    BD_RES_SIZES(BD_CASE)
+#undef BD_CASE
+    default:
+      return (int)cudaErrorInvalidValue;
+  }
+}
+
+int launch_resident(int lz, bool single, const ResArgs& A, int nclusters, int cs, int grid, size_t smem,
+                    cudaStream_t s) {
+  switch (lz) {
+#define BD_CASE(L)                                                             \
+  case L:                                                                      \
+    return single ? launch_resident_t<L, true>(A, nclusters, cs, grid, smem, s) \
+                  : launch_resident_t<L, false>(A, nclusters, cs, grid, smem, s);
+    BD_RES_SIZES(BD_CASE)
+#undef BD_CASE
+    default:
+      return (int)cudaErrorInvalidValue;
+  }
+}
+
+}  // namespace bd

@@ -1,7 +1,7 @@
 // Serving: a request loop with continuous batching. Requests (parameter set,
 // seed, step count) queue on the host; each tick admits queued requests
 // whose device footprint fits the HBM budget, advances every resident run by
-// up to steps_per_tick fused steps in one batched launch sequence, copies out
+// up to steps_per_tick steps in one batched launch sequence, copies out
 // due snapshots and retires finished runs, freeing their memory for the
 // queue. A run's result does not depend on which other runs share its
 // launches: every kernel works per run, noise is keyed by (seed, particle,
@@ -426,7 +426,7 @@ static int serve_tick(bd_server* s, int* active) {
     cudaEventRecord(s->ev[1], s->e.stream);
     std::vector<bd::RunDyn> y;
     RK(s->e.get_dyn_all(y));
-    // a grid-barrier wait that gave up leaves the fused step's barrier words
+    // a grid-barrier wait that gave up leaves the resident step's barrier words
     // set: the engine clears them and returns the run to its state before
     // the failed step (the request still ends with BD_ERR_TIMEOUT)
     for (const bd::RunDyn& d : y)

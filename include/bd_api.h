@@ -151,11 +151,13 @@ int bd_berechne_zufallskraefte(bd_ctx* c);
 int bd_optimaler_zeitschritt(bd_ctx* c, double* dt);
 /* refresh_erwNachbar (:216-325) */
 int bd_refresh_erwNachbar(bd_ctx* c);
-/* zeitschritt (:74-163): one fused step; *dt_out = the step length used
+/* zeitschritt (:74-163): one step; *dt_out = the step length used
  * (tmax is ignored as in the reference; tmax <= 0 returns BD_ERR_ARG and
  * *dt_out = 1e10) */
 int bd_zeitschritt(bd_ctx* c, double tmax, double* dt_out);
-/* nsteps fused steps replayed from captured CUDA graphs; *t_out = simulated time */
+/* nsteps steps, many per launch where the run qualifies for the resident step
+ * (bd_launches_per_step), else replayed from captured CUDA graphs;
+ * *t_out = simulated time */
 int bd_zeitschritte(bd_ctx* c, long long nsteps, double* t_out);
 /* zeitschritte_bis_obs (:444-455): steps until the time since the last
  * observation point reaches obs_dt; *nsteps_out = steps taken */
@@ -342,10 +344,13 @@ int bd_gridDensity_noalloc(const bd_params* p, int scheme, const int32_t* git1, 
 /* the cudaStream_t the context launches on, for CUDA-event timing */
 int bd_get_stream(bd_ctx* c, void** stream);
 int bd_batch_get_stream(bd_batch* b, void** stream);
-/* kernel launches one fused step makes (all runs of a batch together) */
+/* kernel launches one step taken by itself makes (all runs of a batch
+ * together). 1: the run steps with the resident kernel, which takes many steps
+ * per launch when asked for them. A batch whose runs qualify does too for
+ * calls of two or more steps; the number is that of a call of one step. */
 int bd_launches_per_step(bd_ctx* c, int* n);
 int bd_batch_launches_per_step(bd_batch* b, int* n);
-/* runs nsteps fused steps with CUDA events between the stages and returns
+/* runs nsteps steps of the stage kernels with CUDA events between the stages and returns
  * the mean device time per step of each stage in ms:
  * [0] deposit [1] row FFT [2] column FFT + Green [3] inverse row FFT
  * [4] per-particle forces/update [5] cell-count scan (+ step end)
@@ -409,14 +414,15 @@ int bd_batch_autotune(bd_batch* b, int reps, bd_tune_result* out);
  * is larger than 1024^2). BD_ERR_ARG for other values. */
 int bd_batch_set_step_form(bd_batch* b, int form, int ctas_per_sm);
 /* one run on a power-of-two mesh up to 1024^2 with a fixed dt steps in one
- * cooperative launch per step (the fused step); bd_launches_per_step then
- * reports 1 and bd_stage_times times the stage kernels instead. Runs on
+ * cooperative launch (the fused step: the resident kernel, many steps per
+ * launch when asked for them); bd_launches_per_step then reports 1 and
+ * bd_stage_times times the stage kernels instead. Runs on
  * power-of-two meshes with a fixed dt otherwise (a batch of two or more of
  * them) step in six launches per step (the pipelined stage step;
  * bd_launches_per_step reports 6): the particle kernel, then the cell sort
  * beside the transform of the new density on a second stream. This runs
  * nsteps steps and returns the mean time per step of each phase in ms (the
- * fused step: device timestamps at its grid-wide barriers; the pipelined
+ * fused step: device timestamps at its barriers, one step per launch; the pipelined
  * step: CUDA events on the library stream). The mesh transform is pipelined
  * across steps (the next step's density is deposited by the move):
  * fused step: [0] inverse row FFT [1] per-particle forces/update/next

@@ -1,0 +1,128 @@
+"""The resident step (many steps of a run in one launch) against the stage
+kernels, bit for bit: every mesh class (powers of two, 3 * 2^k, other factors
+of 3), fixed and adaptive dt, one cluster and the whole grid, one lane and
+several lanes per particle, particles beyond a CTA's shared memory, and
+batches of them. The sums are integers and every transform rounds as the
+stage kernels' does, so the tolerance is zero."""
+import numpy as np
+import pytest
+
+import configs as C
+
+pytestmark = pytest.mark.gpu
+
+
+def _params(gpu, n1, n2, mesh, adaptive, scheme=2, rho=0.2, **kw):
+    L = max(12.0, ((n1 + n2) / rho) ** 0.5)
+    return dict(C.CONFIGS["c1_cic"], N1=n1, N2=n2, L=L, FFT_samples=mesh, densGrid_Schema=scheme,
+                lambda_kapillar=L / 9, f2_f1=-0.7, T=2.0, dt_max=2e-3 if adaptive else 1e-4,
+                max_reisedistanz=0.1 if adaptive else 1e30, noise_kind=gpu.NOISE_DISK, **kw)
+
+
+def _lattice(p, seed):
+    """Sites of a square lattice in random order, each moved by up to what
+    keeps pairs 0.9 apart."""
+    rng = np.random.default_rng(seed)
+    n, L = p["N1"] + p["N2"], p["L"]
+    m = int(np.ceil(np.sqrt(n)))
+    site = rng.permutation(m * m)[:n]
+    x = np.mod(np.stack([site // m, site % m], 1) * (L / m) + rng.random((n, 2)) * max(0.0, L / m - 0.9), L)
+    Cc = int(L / 2 ** (1 / 6))
+    B = L / Cc
+    git = np.minimum((x / B).astype(np.int32), Cc - 1)
+    rel = np.clip(x - git * B, 0.0, np.float32(B) * (1 - 1e-6))
+    return {0: (git[:p["N1"]], rel[:p["N1"]]), 1: (git[p["N1"]:], rel[p["N1"]:])}
+
+
+def _same(a, b):
+    for s in (0, 1):
+        assert np.array_equal(a[s][0], b[s][0])
+        assert np.array_equal(a[s][1], b[s][1])
+
+
+# smallest and largest compiled meshes of every class, 144 and 648 through the
+# run-time transform, 864 beyond the resident step; 3000 and 3001 particles on
+# 128^2 either side of the cluster / grid rule
+SIZES = [(40, 17, 8), (300, 201, 16), (300, 200, 24), (700, 333, 48), (1500, 1500, 128), (1500, 1501, 128),
+         (1001, 999, 96), (900, 800, 144), (2000, 2500, 192), (5000, 4001, 256), (3000, 2999, 384),
+         (9001, 6000, 512), (9001, 6000, 648), (9001, 6000, 768), (20000, 19999, 1024), (2000, 1000, 864)]
+
+
+@pytest.mark.parametrize("adaptive", [False, True])
+@pytest.mark.parametrize("n1,n2,mesh", SIZES)
+def test_resident_equals_stage_kernels(gpu, n1, n2, mesh, adaptive):
+    p = _params(gpu, n1, n2, mesh, adaptive, scheme=(n1 + mesh) % 3)
+    start = _lattice(p, 5)
+    a, b = gpu.Run(p, seed=21), gpu.Run(p, seed=21)
+    for r in (a, b):
+        r.set_positions_all(start)
+    a.zeitschritte(12)
+    a.zeitschritt()
+    a.zeitschritte(6)
+    b.stage_times(19)
+    _same(a.get_positions(), b.get_positions())
+    assert a.time() == b.time() and a.step_count() == b.step_count()
+    if adaptive:  # the last step's forces stay readable
+        fa, fb = a.get_forces(), b.get_forces()
+        for k in fa:
+            assert np.array_equal(fa[k], fb[k])
+    a.close()
+    b.close()
+
+
+def test_resident_beyond_shared_particles(gpu):
+    """More particles per CTA than its shared memory holds (2048 on 148 SMs)."""
+    p = _params(gpu, 200000, 150001, 256, False, rho=0.25)
+    start = _lattice(p, 6)
+    a, b = gpu.Run(p, seed=3), gpu.Run(p, seed=3)
+    for r in (a, b):
+        r.set_positions_all(start)
+    a.zeitschritte(5)
+    b.stage_times(5)
+    _same(a.get_positions(), b.get_positions())
+
+
+def test_resident_many_launches_and_other_steps(gpu):
+    """More steps than one launch takes (1024 for a small run), and the forms
+    of stepping after one another on one run."""
+    p = _params(gpu, 250, 150, 32, False, scheme=1)
+    start = _lattice(p, 7)
+    a, b = gpu.Run(p, seed=8), gpu.Run(p, seed=8)
+    for r in (a, b):
+        r.set_positions_all(start)
+    a.zeitschritte(1030)
+    for n in (1000, 29, 1):
+        b.zeitschritte(n)
+    _same(a.get_positions(), b.get_positions())
+    a.zeitschritte(3)
+    a.stage_times(2)
+    a.zeitschritt_debug(0.05)
+    a.zeitschritte(4)
+    b.stage_times(5)
+    b.zeitschritt_debug(0.05)
+    b.stage_times(4)
+    _same(a.get_positions(), b.get_positions())
+
+
+@pytest.mark.parametrize("adaptive", [False, True])
+def test_resident_batch_equals_stage_kernels(gpu, adaptive):
+    """A batch of uneven runs on clusters of several sizes, steps of both
+    forms in turn (one step at a time takes the launch-per-step form)."""
+    sizes = [(400, 300, 64), (1000, 900, 128), (600, 601, 96), (150, 0, 32), (700, 700, 192), (300, 100, 144)]
+    if not adaptive:
+        sizes = [(n1, n2, m) for n1, n2, m in sizes if m & (m - 1) == 0]
+    runs = [_params(gpu, n1, n2, m, adaptive and k % 2 == 0, scheme=k % 3) for k, (n1, n2, m) in enumerate(sizes)]
+    if adaptive:
+        runs.append(dict(runs[0], idgas_only=1))
+    seeds = list(range(len(runs)))
+    a, b = gpu.Batch(runs, seeds), gpu.Batch(runs, seeds)
+    for x in (a, b):
+        for k, p in enumerate(runs):
+            x.set_positions(k, _lattice(p, 40 + k))
+    a.step(9)
+    a.step(1)
+    a.step(20)
+    b.stage_times(30)
+    for k in range(len(runs)):
+        _same(a.get_positions(k), b.get_positions(k))
+        assert a.time(k) == b.time(k)
