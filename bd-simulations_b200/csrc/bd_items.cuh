@@ -519,7 +519,7 @@ __device__ inline float dt_bound(float F, float nz, float mrd, float T) {
 }
 
 
-template <bool NC, bool DEP>
+template <bool NC>
 __device__ inline void finish_particle(const RunDesc& R, RunDyn& D, const unsigned long long& step, int mode, int mask,
                                        const Rec& p, int ic, int jc, int gi, float2 Fw);
 
@@ -632,7 +632,7 @@ __device__ __forceinline__ void wca_row(const RunDesc& R, const WcaP& W, const R
 
 // Forces and (MODE_STEP) the move of the particle at sorted index gi; DEP:
 // the move also deposits the new position into R.dacc.
-template <bool NC, bool DEP>
+template <bool NC>
 __device__ __forceinline__ void particle_item(const RunDesc& R, RunDyn& D, const unsigned long long& step, int gi, int mode,
                                               int mask) {
   const Rec p = ldrec<NC>(&R.recA[gi]);
@@ -642,25 +642,26 @@ __device__ __forceinline__ void particle_item(const RunDesc& R, RunDyn& D, const
   if (mode == MODE_SET) m &= p.pid >= R.N1 ? 2 : 1;
   if (R.flags & F_IDGAS) m = 0;
   const float2 Fw = m ? wca_direct<NC>(R, p, ic, jc, gi, m) : make_float2(0.f, 0.f);
-  finish_particle<NC, DEP>(R, D, step, mode, mask, p, ic, jc, gi, Fw);
+  finish_particle<NC>(R, D, step, mode, mask, p, ic, jc, gi, Fw);
 }
 
-// Count particle gi into its new cell (an add whose result nobody waits for;
+// Count a particle into its new cell (an add whose result nobody waits for;
 // the scatter takes the slots) and into the per-chunk total for the scan,
 // added once per group of lanes in the same chunk (neighbouring particles of
 // the cell-sorted order mostly share one). The cell is the key: the scatter
 // reads it from the record recB[gi].
-__device__ __forceinline__ void count_into_cell(const RunDesc& R, int gi, int key) {
+// act: the lanes of the warp that call, converged.
+__device__ __forceinline__ void count_into_cell(const RunDesc& R, int key, unsigned act) {
   red_add(&R.count[key], 1);
   const int ch = key / SCAN_CHUNK;
-  const unsigned grp = __match_any_sync(__activemask(), ch);
+  const unsigned grp = __match_any_sync(act, ch);
   if ((threadIdx.x & 31) == __ffs(grp) - 1) red_add(&R.chunk_sum[ch], __popc(grp));
 }
 
 // Everything after the WCA sum: store it (MODE_SET/ADD), or add the mesh
 // force and the noise and store the forces (MODE_FORCES) or move and re-bin
 // (MODE_STEP).
-template <bool NC, bool DEP>
+template <bool NC>
 __device__ inline void finish_particle(const RunDesc& R, RunDyn& D, const unsigned long long& step, int mode, int mask,
                                        const Rec& p, int ic, int jc, int gi, float2 Fw) {
   const bool sp2 = p.pid >= R.N1;
@@ -687,14 +688,33 @@ __device__ inline void finish_particle(const RunDesc& R, RunDyn& D, const unsign
     if (bnd < R.dt_max) atomicMin(&D.dt_bits, __float_as_uint(bnd));
     return;
   }
-  // MODE_STEP
-  const float2 F = make_float2(Fw.x + Fk.x, Fw.y + Fk.y);
-  const Rec np = move_particle(R, p, F, xi, R.dt_max, &D.err);
+}
+
+// Forces, noise and move of the particle at sorted index gi, its counts and
+// (DEP) its deposit. act: the lanes of the warp that call. The lanes are
+// brought together again behind the neighbour loops, the noise's rejections
+// and the re-binning: left to the compiler, what follows ran for parts of the
+// warp in turn (lanes that leave a loop early going ahead).
+template <bool NC, bool DEP>
+__device__ __forceinline__ void step_particle(const RunDesc& R, RunDyn& D, const unsigned long long& step, int gi,
+                                              unsigned act) {
+  const Rec p = ldrec<NC>(&R.recA[gi]);
+  int ic, jc;
+  cell_ij(R, p.cell, ic, jc);
+  const bool gas = (R.flags & F_IDGAS) != 0;
+  const float2 Fw = gas ? make_float2(0.f, 0.f) : wca_direct<NC>(R, p, ic, jc, gi, 7);
+  __syncwarp(act);
+  const float2 Fk = gas ? make_float2(0.f, 0.f) : mesh_force<NC>(R, p, ic, jc, R.scheme);
+  float2 xi = make_float2(0.f, 0.f);
+  if (!(R.flags & F_NOWCA)) xi = particle_noise(R.noise, R.seed, step, (uint32_t)p.pid);
+  __syncwarp(act);
+  const Rec np = move_particle(R, p, make_float2(Fw.x + Fk.x, Fw.y + Fk.y), xi, R.dt_max, &D.err);
+  __syncwarp(act);
   R.recB[gi] = np;
-  count_into_cell(R, gi, np.cell);
+  count_into_cell(R, np.cell, act);
   // the resident and the pipelined step: the next step's density
   if constexpr (DEP) deposit_acc<1>(R, np);
-  if (np.cell != p.cell) atomicAdd(&D.moved[sp2 ? 1 : 0], 1);  // num_Zellwechsel of TimestepInfo
+  if (np.cell != p.cell) atomicAdd(&D.moved[p.pid >= R.N1 ? 1 : 0], 1);  // num_Zellwechsel of TimestepInfo
 }
 
 // End of a step (one thread per run): advance the Philox step counter, the

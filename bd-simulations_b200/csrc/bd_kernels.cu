@@ -426,8 +426,8 @@ __global__ void __launch_bounds__(256, MINB) k_step(const RunDesc* __restrict__ 
     if (!on) continue;
     const RunDesc& R = runs[I.run];
     const int gi = I.a * blockDim.x + threadIdx.x;
-    if (gi >= R.N) continue;
-    particle_item<true, DEP>(R, dyn[I.run], dyn[I.run].step, gi, MODE_STEP, 7);
+    const unsigned act = __ballot_sync(0xffffffffu, gi < R.N);
+    if (gi < R.N) step_particle<true, DEP>(R, dyn[I.run], dyn[I.run].step, gi, act);
   }
 }
 
@@ -444,7 +444,7 @@ __global__ void __launch_bounds__(256, MINB) k_particles(const RunDesc* __restri
     const RunDesc& R = runs[I.run];
     const int gi = I.a * blockDim.x + threadIdx.x;
     if (gi >= R.N) continue;
-    particle_item<true, false>(R, dyn[I.run], dyn[I.run].step, gi, mode, mask);
+    particle_item<true>(R, dyn[I.run], dyn[I.run].step, gi, mode, mask);
   }
 }
 
@@ -461,6 +461,7 @@ __global__ void __launch_bounds__(256) k_move(const RunDesc* __restrict__ runs,
     const RunDesc& R = runs[I.run];
     RunDyn& D = dyn[I.run];
     const int gi = I.a * blockDim.x + threadIdx.x;
+    const unsigned act = __ballot_sync(0xffffffffu, gi < R.N);
     if (gi >= R.N) continue;
     const Rec p = R.recA[gi];
     Rec np;
@@ -472,7 +473,8 @@ __global__ void __launch_bounds__(256) k_move(const RunDesc* __restrict__ runs,
       np = move_particle(R, p, make_float2(Fw.x + Fk.x, Fw.y + Fk.y), xi, dt, &D.err);
     }
     R.recB[gi] = np;
-    count_into_cell(R, gi, np.cell);
+    __syncwarp(act);
+    count_into_cell(R, np.cell, act);
     if (np.cell != p.cell) atomicAdd(&D.moved[p.pid >= R.N1 ? 1 : 0], 1);
   }
 }
@@ -484,8 +486,8 @@ __global__ void __launch_bounds__(256) k_count(const RunDesc* __restrict__ runs,
     const Item I = items[it];
     const RunDesc& R = runs[I.run];
     const int gi = I.a * blockDim.x + threadIdx.x;
-    if (gi >= R.N) continue;
-    count_into_cell(R, gi, R.recB[gi].cell);
+    const unsigned act = __ballot_sync(0xffffffffu, gi < R.N);
+    if (gi < R.N) count_into_cell(R, R.recB[gi].cell, act);
   }
 }
 

@@ -568,15 +568,26 @@ __device__ __forceinline__ float2 res_mesh(const RunDesc& R, const Rec& p) {
   return mesh_force<false>(R, p, ic, jc, R.scheme);
 }
 
+// The lanes of this thread's warp that work on one of n things, LANES lanes
+// for each, i (< n) this thread's.
+template <int LANES>
+__device__ __forceinline__ unsigned lanes_below(int i, int n) {
+  const int lane = (int)threadIdx.x & 31;
+  const int k = (n - (i - lane / LANES)) * LANES;  // lanes of the warp in use
+  return k >= 32 ? 0xffffffffu : (1u << k) - 1u;
+}
+
 // The move of particle p with its counts and its deposit, LANES lanes per
 // particle: each computes the move, the lanes share the deposit's points and
-// lane 0 counts.
+// lane 0 counts. act: the lanes of the warp that call.
 template <int LANES>
 __device__ __forceinline__ Rec res_move(const RunDesc& R, RunDyn* D, const Rec& p, float2 F, float2 xi, float dt,
-                                        float sq, bool mesh, int sub) {
+                                        float sq, bool mesh, int sub, unsigned act) {
   const Rec np = move_particle_sq(R, p, F, xi, dt, sq, &D->err, true, sub == 0);
+  __syncwarp(act);
   if (sub == 0) {
-    count_into_cell(R, 0, np.cell);
+    constexpr unsigned first = LANES == 1 ? 0xffffffffu : LANES == 2 ? 0x55555555u : 0x11111111u;
+    count_into_cell(R, np.cell, act & first);
     if (np.cell != p.cell) atomicAdd(&D->moved[p.pid >= R.N1 ? 1 : 0], 1);
   }
   if (mesh) deposit_acc<LANES>(R, np, sub);
@@ -702,7 +713,8 @@ __device__ __noinline__ void res_step(RunDyn* D, unsigned long long step, int g0
   for (int i = (int)threadIdx.x / LANES; i < nc; i += 2 * NT / LANES) {
     const Rec p = S.rec[i];
     const float2 Fk = res_mesh(R, p), Fw = S.F[i];
-    const Rec np = res_move<LANES>(R, D, p, make_float2(Fw.x + Fk.x, Fw.y + Fk.y), S.xi[i], R.dt_max, sq, mesh, sub);
+    const Rec np = res_move<LANES>(R, D, p, make_float2(Fw.x + Fk.x, Fw.y + Fk.y), S.xi[i], R.dt_max, sq, mesh, sub,
+                                   lanes_below<LANES>(i, nc));
     if constexpr (LANES > 1) {
       // every lane of the particle has read its record
       const unsigned lane = threadIdx.x & 31u;
@@ -712,8 +724,8 @@ __device__ __noinline__ void res_step(RunDyn* D, unsigned long long step, int g0
   }
   if constexpr (LANES == 1)
     for (int gi = g0 + nc + (int)threadIdx.x; gi < g1; gi += 2 * NT) {
-      if (mesh) particle_item<false, true>(R, *D, step, gi, MODE_STEP, 7);
-      else particle_item<false, false>(R, *D, step, gi, MODE_STEP, 7);
+      if (mesh) step_particle<false, true>(R, *D, step, gi, lanes_below<1>(gi, g1));
+      else step_particle<false, false>(R, *D, step, gi, lanes_below<1>(gi, g1));
     }
 }
 
@@ -746,11 +758,12 @@ __device__ __noinline__ void res_adaptive_move(RunDyn* D, int g0, int g1, int nc
   const float dt = fminf(R.dt_max, __uint_as_float(((volatile RunDyn*)D)->dt_bits));
   const float sq = sqrtf(2.0f * R.T * dt);
   for (int i = (int)threadIdx.x; i < nc; i += 2 * NT)
-    S.rec[i] = res_move<1>(R, D, S.rec[i], S.F[i], S.xi[i], dt, sq, mesh, 0);
+    S.rec[i] = res_move<1>(R, D, S.rec[i], S.F[i], S.xi[i], dt, sq, mesh, 0, lanes_below<1>(i, nc));
   for (int gi = g0 + nc + (int)threadIdx.x; gi < g1; gi += 2 * NT) {
     const Rec p = ldrec<false>(&R.recA[gi]);
     const float2 Fw = R.Fw[p.pid], Fk = R.Fk[p.pid];
-    R.recB[gi] = res_move<1>(R, D, p, make_float2(Fw.x + Fk.x, Fw.y + Fk.y), R.Fn[p.pid], dt, sq, mesh, 0);
+    R.recB[gi] = res_move<1>(R, D, p, make_float2(Fw.x + Fk.x, Fw.y + Fk.y), R.Fn[p.pid], dt, sq, mesh, 0,
+                             lanes_below<1>(gi, g1));
   }
 }
 
