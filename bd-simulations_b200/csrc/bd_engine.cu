@@ -803,10 +803,7 @@ int Engine::build_plan() {
   // take as many sequences per item as FFT2_THREADS threads transform at
   // once (Z/16 threads per length-Z sequence).
   const size_t nr = runs.size();
-  // the pipelined stage step (decided below) runs every transform item with
-  // FFT2_THREADS threads; the classic column pass of meshes of 2048 and more
-  // takes FFT2_WIDE_THREADS, so an item holds several columns
-  bool pipe_runs = nr >= 2;
+  bool pipe_runs = nr >= 2 || (nr == 1 && runs[0]->Z > 1024);
   for (auto* r : runs) pipe_runs = pipe_runs && r->d.dacc != nullptr;
   std::vector<int> lrf(nr), lri(nr), lw(nr);
   for (size_t k = 0; k < nr; k++) {
@@ -817,8 +814,7 @@ int Engine::build_plan() {
       lrf[k] = std::min(ilog2(FFT2_THREADS / fft2_tps(lz - 1)), lz);
       lri[k] = std::min(ilog2(FFT2_THREADS / fft2_tps(lz)), lz);
       // columns per item: both inverse transforms of the item run at once
-      const int cthr = (lz >= 11 && !pipe_runs) ? FFT2_WIDE_THREADS : FFT2_THREADS;
-      lw[k] = std::min(ilog2(cthr / (2 * fft2_tps(lz))), lz - 1);
+      lw[k] = std::min(ilog2(std::max(1, FFT2_THREADS / (2 * fft2_tps(lz)))), lz - 1);
     } else {
       lrf[k] = r.lrf;
       lri[k] = r.lri;
@@ -877,8 +873,7 @@ int Engine::build_plan() {
         fsm[P][2] = std::max(fsm[P][2], (size_t)(1 << lri[k]) * fft2_stride(Z) * 8);
         fthr[P][0] = std::max(fthr[P][0], (1 << lrf[k]) * fft2_tps(lz - 1));
         // both inverse column transforms at once when the threads allow
-        fthr[P][1] = std::max(fthr[P][1], std::min(lz >= 11 && !pipe_runs ? FFT2_WIDE_THREADS : FFT2_THREADS,
-                                                   2 * (1 << lw[k]) * fft2_tps(lz)));
+        fthr[P][1] = std::max(fthr[P][1], std::min(FFT2_THREADS, 2 * (1 << lw[k]) * fft2_tps(lz)));
         fthr[P][2] = std::max(fthr[P][2], (1 << lri[k]) * fft2_tps(lz));
       } else {
         fsm[0][0] = std::max(fsm[0][0], (size_t)(1 << lrf[k]) * n * 8);
@@ -907,7 +902,7 @@ int Engine::build_plan() {
       put(fl[P][q], f.off[q], f.n[q]);
       f.sm[q] = fsm[P][q];
       // whole warps, at least one
-      f.thr[q] = P ? std::max(32, std::min(q == 1 ? FFT2_WIDE_THREADS : FFT2_THREADS, (fthr[P][q] + 31) / 32 * 32))
+      f.thr[q] = P ? std::max(32, std::min(FFT2_THREADS, (fthr[P][q] + 31) / 32 * 32))
                    : FFT_THREADS;
     }
     if (P) fft_p2.push_back(f);
@@ -917,10 +912,16 @@ int Engine::build_plan() {
   put(chunk, off_chunk, n_chunk);
   off_part_all = off_part;
   n_part_all = n_part;
-  // pipelined stage step: several runs, every one depositing in the move. A
-  // single run takes the resident step (mesh up to 1024^2) or the classic stage
-  // kernels: alone on a large mesh, the tile deposit is cheaper than the
-  // move's atomics and its transforms leave the sort nothing to overlap with
+  // the particle kernel's form: for runs of 131 072 particles and more on
+  // average, whose arrays do not stay in L2 from one kernel to the next.
+  // Measured, us per step (that form | the other), runs x particles, mesh:
+  // 2 x 100 000, 256^2 36.7 | 35.6; 4 x 100 000 50.8 | 52.3; 2 x 250 000, 512^2
+  // 59.9 | 64.2; 8 x 250 000 200 | 258; 4 x 600 000 206 | 280; 1 x 2 000 000,
+  // 2048^2 247 | 351; the 256-run ensemble (24 000 on average) 562 | 537
+  part_large = n_part >= (int)nr * 512 ? 1 : 0;
+  // pipelined stage step: several runs, every one depositing in the move, or
+  // one on a mesh beyond the resident step's (1024^2): 2.1 M particles on
+  // 2048^2, 335 us per step with the stage kernels, 252 pipelined
   piped = pipe_runs;
   if (piped) {
     std::vector<Item> pl[3];
@@ -1008,7 +1009,7 @@ int Engine::enqueue_step(cudaStream_t s, cudaEvent_t* ev) {
     RK(launch_particles(d_runs, d_dyn, it(off_part), n_part, MODE_FORCES, 7, 1, s, part_shape));
     RK(launch_move(d_runs, d_dyn, it(off_part), n_part, 1, 0, s));
   } else {
-    RK(launch_step(d_runs, d_dyn, it(off_part), n_part, 0, s, part_shape));
+    RK(launch_step(d_runs, d_dyn, it(off_part), n_part, 0, part_large, s, part_shape));
   }
   if (ev) cudaEventRecord(ev[5], s);
   RK(launch_sort(d_runs, d_dyn, 0, (int)runs.size(), it(off_chunk), n_chunk, it(off_part), n_part, 1,
@@ -1032,7 +1033,7 @@ int Engine::enqueue_step(cudaStream_t s, cudaEvent_t* ev) {
 int Engine::enqueue_pipe(cudaStream_t s, cudaEvent_t* ev) {
   if (ev) CK(cudaEventRecord(ev[0], s));
   if (ev) CK(cudaEventRecord(ev[1], s));
-  RK(launch_step(d_runs, d_dyn, it(off_part), n_part, 1, s, part_shape));
+  RK(launch_step(d_runs, d_dyn, it(off_part), n_part, 1, part_large, s, part_shape));
   if (ev) CK(cudaEventRecord(ev[2], s));
   CK(cudaEventRecord(ev_fork[0], s));
   CK(cudaStreamWaitEvent(stream2, ev_fork[0], 0));
@@ -1052,7 +1053,7 @@ int Engine::enqueue_pipe(cudaStream_t s, cudaEvent_t* ev) {
 // cooperative tail (scan | next forward rows, scatter | next columns, step
 // end, the next step's inverse rows). ts (optional): the tail's timestamps.
 int Engine::enqueue_pipe2(cudaStream_t s, unsigned long long* ts) {
-  RK(launch_step(d_runs, d_dyn, it(off_part), n_part, 1, s, part_shape));
+  RK(launch_step(d_runs, d_dyn, it(off_part), n_part, 1, part_large, s, part_shape));
   return launch_pipe_tail(d_runs, d_dyn, tplan, d_bar, s, ts) ? BD_ERR_CUDA : BD_OK;
 }
 
@@ -1418,7 +1419,7 @@ int Engine::pipe2_phase_times(int nsteps, double* ms, int nphases) {
   for (int k = 0; k < nsteps && st == BD_OK; k++) {
     if (cudaEventRecord(ev[0], stream) != cudaSuccess) st = BD_ERR_CUDA;
     if (st == BD_OK)
-      st = launch_step(d_runs, d_dyn, it(off_part), n_part, 1, stream, part_shape)
+      st = launch_step(d_runs, d_dyn, it(off_part), n_part, 1, part_large, stream, part_shape)
                ? BD_ERR_CUDA
                : BD_OK;
     if (st == BD_OK && cudaEventRecord(ev[1], stream) != cudaSuccess) st = BD_ERR_CUDA;
@@ -1512,7 +1513,7 @@ int Engine::time_particles(int shape, int reps, cudaEvent_t e0, cudaEvent_t e1, 
   for (int k = 0; k <= reps; k++) {
     if (k == 1) CK(cudaEventRecord(e0, stream));
     if (split) RK(launch_particles(d_runs, d_dyn, it(off_part), n_part, MODE_FORCES, 7, 1, stream, shape));
-    else RK(launch_step(d_runs, d_dyn, it(off_part), n_part, piped ? 1 : 0, stream, shape));
+    else RK(launch_step(d_runs, d_dyn, it(off_part), n_part, piped ? 1 : 0, part_large, stream, shape));
   }
   CK(cudaEventRecord(e1, stream));
   CK(cudaEventSynchronize(e1));

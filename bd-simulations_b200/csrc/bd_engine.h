@@ -124,6 +124,7 @@ class Engine {
   int dep_tiles_min = 148, fft_items_min = 296;
   // compiled form of the step's particle kernel (PartShape; autotune() picks it)
   int part_shape = PART_SHAPE_DEFAULT;
+  int part_large = 0;  // the particle kernel's form for large runs (launch_step)
   // form of the pipelined step (set_step_form; same bits either way):
   // PIPE_SIX: six launches on two streams; PIPE_TWO: the particle kernel and
   // one cooperative launch of everything else
@@ -221,7 +222,8 @@ class Engine {
   // of the API: bd_fused_phase_times, bd_inject_barrier_timeout)
   bool fused = false;
   unsigned* d_bar = nullptr;
-  // pipelined stage step (power-of-two meshes, fixed dt, two or more runs):
+  // pipelined stage step (power-of-two meshes, fixed dt, two or more runs or one
+  // on a mesh of 2048 or 4096):
   // six launches per step, the density deposited in the move, its transform
   // beside the cell sort. Its transform items of every mesh size (log2 Z in
   // Item.b) and their shared memory:

@@ -207,6 +207,73 @@ struct Fft2Sched<LOGN, LOGN, TWS> {
 // place (sg = -1 forward, +1 inverse, unnormalised) with nseq * N/E threads;
 // the caller syncs before, the last pass ends with a barrier.
 
+// The transform with its first pass reading through ld(b, e) (element e of
+// sequence b, straight from global memory: no copy to shared memory and no
+// barrier ahead of it) and its last one writing through st(b, e, value). The
+// arithmetic is Fft2Sched's. ILV: neighbouring threads take the same elements
+// of different sequences (b = thread mod nseq), for sources stored by column.
+// OUT_SHARED: st writes shared memory (the reads of the last pass end first).
+// 2^lseq sequences, 2^lseq * N/E threads at most; every thread calls; ends
+// with a barrier unless the last pass leaves shared memory alone.
+// IN_SHARED: the sequences are in shared memory already (ld is not used).
+template <int LOGN, int DONE, bool ILV, bool IN_SHARED, bool OUT_SHARED, class Ld, class St>
+__device__ __forceinline__ void fft2_through(float2* s, int ss, int lseq, const float2* __restrict__ tw, int lz,
+                                             float sg, const Ld& ld, const St& st) {
+  constexpr int rem = LOGN - DONE, left = (rem + 3) / 4, LOGR = (rem + left - 1) / left;
+  constexpr bool FIRST = DONE == 0 && !IN_SHARED, LAST = DONE + LOGR == LOGN;
+  constexpr int N = 1 << LOGN, R = 1 << LOGR, E = fft2_e(LOGN), TPS = N / E, NB = E / R, NR = N / R;
+  const int g = threadIdx.x;
+  const int b = ILV ? g & ((1 << lseq) - 1) : g / TPS, i = ILV ? g >> lseq : g - b * TPS;
+  const bool act = ILV ? i < TPS : b < (1 << lseq);
+  float2* q = s + b * ss;
+  float2 v[E];
+#pragma unroll
+  for (int t = 0; t < E; t++) v[t] = make_float2(0.f, 0.f);
+  if (act) {
+#pragma unroll
+    for (int u = 0; u < NB; u++)
+#pragma unroll
+      for (int t = 0; t < R; t++) {
+        const int e = u * TPS + i + t * NR;
+        if constexpr (FIRST) v[u * R + t] = ld(b, e);
+        else v[u * R + t] = q[pad16(e)];
+      }
+  }
+  if (!FIRST && (!LAST || OUT_SHARED)) __syncthreads();
+  if (act) {
+#pragma unroll
+    for (int u = 0; u < NB; u++) {
+      const int j = u * TPS + i;
+      const int k = j & ((1 << DONE) - 1);
+      if (DONE > 0) {
+        const int sh = lz - DONE - LOGR;
+        float2 w[R];
+#pragma unroll
+        for (int t = 1; t < R; t++) {
+          if ((t & (t - 1)) == 0) {
+            w[t] = __ldg(&tw[(k * t) << sh]);
+            if (sg > 0.f) w[t].y = -w[t].y;
+          } else {
+            const int hb = 1 << (31 - __clz(t));
+            w[t] = cmul(w[hb], w[t - hb]);
+          }
+          v[u * R + t] = cmul(v[u * R + t], w[t]);
+        }
+      }
+      dftr<R>(&v[u * R], sg);
+      const int d = ((j >> DONE) << (DONE + LOGR)) + k;
+#pragma unroll
+      for (int t = 0; t < R; t++) {
+        const int e = d + (t << DONE);
+        if constexpr (LAST) st(b, e, v[u * R + t]);
+        else q[pad16(e)] = v[u * R + t];
+      }
+    }
+  }
+  if (!LAST || OUT_SHARED) __syncthreads();
+  if constexpr (!LAST) fft2_through<LOGN, DONE + LOGR, ILV, IN_SHARED, OUT_SHARED>(s, ss, lseq, tw, lz, sg, ld, st);
+}
+
 // The same transform with four elements per thread (N/4 threads per
 // sequence), for the resident step, whose transforms are bound by the length
 // of one thread's instruction chain: a radix-16 butterfly is shared by four

@@ -317,6 +317,122 @@ __device__ __forceinline__ void fft2_rows_inv_item(const Team& T, const RunDesc&
   T.sync();
 }
 
+// The three passes of meshes of 2048 and 4096 points a side (256 threads): the
+// first transform pass of each reads global memory and the last one writes it
+// (fft2_through), and spec2 is stored by column, point (slot j, row k) at
+// j*Z + k, so that a column is written whole whatever number of columns an item
+// has; the inverse rows read two rows of a column in one 32-byte sector.
+// 2048^2, us per pass alone, columns 51 (1024 threads, four columns an item) and
+// inverse rows 32 before.
+template <int LZ, bool FROM_ACC>
+__device__ __forceinline__ void big_rows_fwd_item(const RunDesc& R, int row0, int lr, float2* s, const float2* tw) {
+  constexpr int Z = 1 << LZ, n = Z >> 1, ln = LZ - 1;
+  constexpr int ss = fft2_stride(n);
+  float2* rho = reinterpret_cast<float2*>(R.rho) + (size_t)row0 * n;
+  ulonglong2* acc = reinterpret_cast<ulonglong2*>(R.dacc) + (size_t)row0 * n;
+  const double inv = pow2_double(-R.fx_shift);
+  auto ld = [&](int b, int m) {
+    const int i = b * n + m;
+    if constexpr (!FROM_ACC) return rho[i];
+    const ulonglong2 a = acc[i];
+    const float2 v = make_float2((float)((double)(long long)a.x * inv), (float)((double)(long long)a.y * inv));
+    rho[i] = v;
+    acc[i] = make_ulonglong2(0ull, 0ull);
+    return v;
+  };
+  auto st = [&](int b, int j, float2 v) { s[b * ss + pad16(j)] = v; };
+  fft2_through<LZ - 1, 0, false, false, true>(s, ss, lr, tw, LZ, -1.f, ld, st);
+  const int lrb = lr < 2 ? lr : 2;
+  const int rbm = (1 << lrb) - 1;
+  for (int i = threadIdx.x; i < (n << lr); i += blockDim.x) {
+    const int rest = i >> lrb;
+    const int j = rest & (n - 1), b = ((rest >> ln) << lrb) + (i & rbm);
+    const float2 zj = s[b * ss + pad16(j)];
+    const float2 zc = s[b * ss + pad16((n - j) & (n - 1))];
+    float2 out;
+    if (j == 0) {
+      out = make_float2(zj.x + zj.y, zj.x - zj.y);
+    } else {
+      const float2 E = make_float2(0.5f * (zj.x + zc.x), 0.5f * (zj.y - zc.y));
+      const float2 O = make_float2(0.5f * (zj.y + zc.y), -0.5f * (zj.x - zc.x));
+      out = cadd(E, cmul(__ldg(&tw[j]), O));
+    }
+    R.spec[(size_t)j * Z + row0 + b] = out;
+  }
+}
+
+template <int LZ>
+__device__ __forceinline__ void big_cols_item(const RunDesc& R, int col0, int lw, float2* sA, const float2* tw) {
+  constexpr int Z = 1 << LZ, n = Z >> 1;
+  constexpr int ss = fft2_stride(Z);
+  const int W = 1 << lw;
+  float2* sB = sA + W * ss;
+  const float2* src = R.spec + (size_t)col0 * Z;
+  auto ld = [&](int c, int k) { return src[c * Z + k]; };
+  auto green = [&](int c, int kx, float2 v) {
+    const int j = col0 + c, a = c * ss + pad16(kx);
+    if (j == 0) {
+      sA[a] = v;
+      return;
+    }
+    const float g = __ldg(&R.green[(size_t)j * Z + kx]);
+    const float gx = __ldg(&R.sxt[kx]) * g;
+    const float gy = __ldg(&R.syt[j]) * g;
+    sA[a] = make_float2(-gx * v.y, gx * v.x);
+    sB[a] = make_float2(-gy * v.y, gy * v.x);
+  };
+  fft2_through<LZ, 0, false, false, true>(sA, ss, lw, tw, LZ, -1.f, ld, green);
+  if (col0 == 0) {
+    const float sy0 = __ldg(&R.syt[0]), syn = __ldg(&R.syt[n]);
+    for (int kx = threadIdx.x; kx <= n; kx += blockDim.x) {
+      const int km = (Z - kx) & (Z - 1);
+      const float2 Ck = sA[pad16(kx)], Cm = sA[pad16(km)];
+      float2 P, Q;
+      packed_green(R, kx, Ck, Cm, n, Z, sy0, syn, P, Q);
+      sA[pad16(kx)] = P;
+      sB[pad16(kx)] = Q;
+      if (km != kx) {
+        packed_green(R, km, Cm, Ck, n, Z, sy0, syn, P, Q);
+        sA[pad16(km)] = P;
+        sB[pad16(km)] = Q;
+      }
+    }
+    __syncthreads();
+  }
+  // sequences 0 .. W-1 the x fields, W .. 2W-1 the y fields
+  float2* dst = reinterpret_cast<float2*>(R.spec2 + (size_t)col0 * Z);
+  auto inverse = [&](int s0, int ls) {
+    auto st = [&](int b, int k, float2 v) {
+      const int q = s0 + b;
+      dst[2 * ((size_t)(q & (W - 1)) * Z + k) + (q >> lw)] = v;
+    };
+    fft2_through<LZ, 0, false, true, false>(sA + s0 * ss, ss, ls, tw, LZ, 1.f, ld, st);
+  };
+  if ((2 << lw) * fft2_tps(LZ) <= (int)blockDim.x) {
+    inverse(0, lw + 1);
+  } else {
+    inverse(0, lw);
+    inverse(W, lw);
+  }
+}
+
+template <int LZ>
+__device__ __forceinline__ void big_rows_inv_item(const RunDesc& R, int row0, int lr, float2* s, const float2* tw) {
+  constexpr int Z = 1 << LZ, n = Z >> 1;
+  constexpr int ss = fft2_stride(Z);
+  const float4* src = R.spec2 + row0;
+  auto ld = [&](int b, int j) {
+    const float4 v = src[(size_t)(j < n ? j : (Z - j) & (n - 1)) * Z + b];
+    return j == 0   ? make_float2(v.x, v.z)
+           : j == n ? make_float2(v.y, v.w)
+           : j < n  ? make_float2(v.x - v.w, v.y + v.z)
+                    : make_float2(v.x + v.w, -v.y + v.z);
+  };
+  float2* dst = R.H + (size_t)row0 * Z;
+  auto st = [&](int b, int l, float2 v) { dst[(size_t)b * Z + l] = v; };
+  fft2_through<LZ, 0, true, false, false>(s, ss, lr, tw, LZ, 1.f, ld, st);
+}
+
 // ---------------------------------------------------------------------------
 // Per-particle physics shared by the staged and the global neighbour paths.
 

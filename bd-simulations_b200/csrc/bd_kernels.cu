@@ -346,11 +346,12 @@ __global__ void __launch_bounds__(FFT_THREADS) k_fft_rows_inv(const RunDesc* __r
   }
 }
 
-// The three passes as kernels, one item per CTA (an item loop around the
+// The three passes as kernels (meshes of 2048 and more: four CTAs per SM, 64
+// registers; columns 55 -> 47 us at 2048^2), one item per CTA (an item loop around the
 // transform with twiddles from global memory makes the compiler hoist the
 // twiddle loads of every pass and spill).
 template <int LZ>
-__global__ void __launch_bounds__(FFT2_THREADS) k_fft2_rows_fwd(const RunDesc* __restrict__ runs,
+__global__ void __launch_bounds__(FFT2_THREADS, LZ >= 11 ? 4 : 1) k_fft2_rows_fwd(const RunDesc* __restrict__ runs,
                                                          const RunDyn* __restrict__ dyn,
                                                          const Item* __restrict__ items, int nitems,
                                                          int require_active) {
@@ -359,11 +360,12 @@ __global__ void __launch_bounds__(FFT2_THREADS) k_fft2_rows_fwd(const RunDesc* _
   const Item I = items[blockIdx.x];
   if (require_active && !run_active(dyn, I.run)) return;
   const RunDesc& R = runs[I.run];
-  fft2_rows_fwd_item<LZ, false, false>(CtaTeam(), R, I.a, I.c, (float2*)smem, R.tw);
+  if constexpr (LZ >= 11) big_rows_fwd_item<LZ, false>(R, I.a, I.c, (float2*)smem, R.tw);
+  else fft2_rows_fwd_item<LZ, false, false>(CtaTeam(), R, I.a, I.c, (float2*)smem, R.tw);
 }
 
 template <int LZ>
-__global__ void __launch_bounds__(FFT2_THREADS) k_fft2_cols(const RunDesc* __restrict__ runs,
+__global__ void __launch_bounds__(FFT2_THREADS, LZ >= 11 ? 4 : 1) k_fft2_cols(const RunDesc* __restrict__ runs,
                                                      const RunDyn* __restrict__ dyn,
                                                      const Item* __restrict__ items, int nitems,
                                                      int require_active) {
@@ -372,28 +374,12 @@ __global__ void __launch_bounds__(FFT2_THREADS) k_fft2_cols(const RunDesc* __res
   const Item I = items[blockIdx.x];
   if (require_active && !run_active(dyn, I.run)) return;
   const RunDesc& R = runs[I.run];
-  fft2_cols_item<LZ, false>(CtaTeam(), R, I.a, I.c, (float2*)smem, R.tw);
-}
-
-// Meshes of 2048 and more: the column pass with 1024 threads, so that an
-// item holds 2-4 adjacent columns (a 2048-point column alone needs 128
-// threads per transform and 256 for the joint inverse) and each row's read
-// of the half spectrum fills a 32-byte sector instead of a quarter of one.
-template <int LZ>
-__global__ void __launch_bounds__(FFT2_WIDE_THREADS) k_fft2_cols_wide(const RunDesc* __restrict__ runs,
-                                                                      const RunDyn* __restrict__ dyn,
-                                                                      const Item* __restrict__ items, int nitems,
-                                                                      int require_active) {
-  extern __shared__ __align__(16) unsigned char smem[];
-  if ((int)blockIdx.x >= nitems) return;
-  const Item I = items[blockIdx.x];
-  if (require_active && !run_active(dyn, I.run)) return;
-  const RunDesc& R = runs[I.run];
-  fft2_cols_item<LZ, false>(CtaTeam(), R, I.a, I.c, (float2*)smem, R.tw);
+  if constexpr (LZ >= 11) big_cols_item<LZ>(R, I.a, I.c, (float2*)smem, R.tw);
+  else fft2_cols_item<LZ, false>(CtaTeam(), R, I.a, I.c, (float2*)smem, R.tw);
 }
 
 template <int LZ>
-__global__ void __launch_bounds__(FFT2_THREADS) k_fft2_rows_inv(const RunDesc* __restrict__ runs,
+__global__ void __launch_bounds__(FFT2_THREADS, LZ >= 11 ? 4 : 1) k_fft2_rows_inv(const RunDesc* __restrict__ runs,
                                                          const RunDyn* __restrict__ dyn,
                                                          const Item* __restrict__ items, int nitems,
                                                          int require_active) {
@@ -402,7 +388,8 @@ __global__ void __launch_bounds__(FFT2_THREADS) k_fft2_rows_inv(const RunDesc* _
   const Item I = items[blockIdx.x];
   if (require_active && !run_active(dyn, I.run)) return;
   const RunDesc& R = runs[I.run];
-  fft2_rows_inv_item<LZ, false>(CtaTeam(), R, I.a, I.c, (float2*)smem, R.tw);
+  if constexpr (LZ >= 11) big_rows_inv_item<LZ>(R, I.a, I.c, (float2*)smem, R.tw);
+  else fft2_rows_inv_item<LZ, false>(CtaTeam(), R, I.a, I.c, (float2*)smem, R.tw);
 }
 
 // The step's particle kernel: forces, noise, move, re-binning and counts, one
@@ -413,11 +400,47 @@ __global__ void __launch_bounds__(FFT2_THREADS) k_fft2_rows_inv(const RunDesc* _
 // MINB: CTAs per SM the compiler keeps registers for (4: at most 64
 // registers; 5: at most 51, more warps resident, a few values reloaded from
 // local memory); the batch autotuner picks one, the arithmetic is the same.
-template <int MINB, bool DEP>
+// AHEAD > 0: every block requests into L2 what the block AHEAD items on reads
+// first. A large run's arrays stream through memory with the cell order, and
+// each of a particle's dependent reads (record, cell starts, neighbours, force
+// grid, accumulator) waited for DRAM: 2.1 M particles, 2048^2, 207 -> 143 us.
+// Runs of a batch that fit L2 gain nothing and pay for the requests (256-run
+// ensemble 333 -> 343 us).
+
+// Part of an array of `total` elements, [at, at + n), into L2.
+__device__ __forceinline__ void l2_prefetch_part(const void* base, size_t elem, size_t at, size_t n, size_t total) {
+  if (at >= total) return;
+  const size_t lo = (at * elem) & ~(size_t)15, hi = (min(at + n, total) * elem) & ~(size_t)15;
+  if (hi <= lo) return;
+  asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"((const char*)base + lo), "r"((unsigned)(hi - lo)));
+}
+
+// What block a (256 particles) of run R reads first. Its cells and mesh points
+// are guessed from its place in the cell order, as for a uniform density (a
+// wrong guess costs the request); the rows behind them are in L2 already.
+template <bool DEP>
+__device__ __forceinline__ void prefetch_block(const RunDesc& R, int a) {
+  const size_t g = (size_t)a * 256, cc = (size_t)R.C * R.C;
+  const float f = (float)g / (float)R.N, w = 256.f / (float)R.N;
+  l2_prefetch_part(R.recA, sizeof(Rec), g, 256, R.N);
+  const size_t c0 = (size_t)(f * (float)cc), cn = (size_t)(w * (float)cc) + 8;
+  l2_prefetch_part(R.start, sizeof(int), c0 + R.C, cn, cc + 1);
+  l2_prefetch_part(R.count, sizeof(int), c0, cn, cc);
+  if (R.flags & F_IDGAS) return;
+  const size_t zz = (size_t)R.Z * R.Z, z0 = (size_t)(f * (float)zz), zn = (size_t)(w * (float)zz) + 8;
+  l2_prefetch_part(R.H, sizeof(float2), z0 + 2 * R.Z, zn, zz);
+  if (DEP) l2_prefetch_part(R.dacc, sizeof(unsigned long long), z0 + 2 * R.Z, zn, zz);
+}
+
+template <int MINB, bool DEP, int AHEAD>
 __global__ void __launch_bounds__(256, MINB) k_step(const RunDesc* __restrict__ runs, RunDyn* __restrict__ dyn,
                                                     const Item* __restrict__ items, int nitems) {
   for (int it = blockIdx.x; it < nitems; it += gridDim.x) {
     const Item I = items[it];
+    if (AHEAD > 0 && threadIdx.x == 32 && it + AHEAD < nitems) {
+      const Item J = items[it + AHEAD];
+      prefetch_block<DEP>(runs[J.run], J.a);
+    }
     const bool on = run_active(dyn, I.run);
     // the pipelined step: the run's first block records whether the run takes
     // part in this step, for the sort and transform kernels that follow (the
@@ -624,14 +647,25 @@ __global__ void __launch_bounds__(256) k_scatter(const RunDesc* __restrict__ run
 #define BD_PIPE_SIZES(X) X(3) X(4) X(5) X(6) X(7) X(8) X(9) X(10) X(11) X(12)
 
 // pass 0: inverse rows, 1: forward rows from R.dacc, 2: columns + Green
+template <int PASS, int L>
+__device__ __forceinline__ void pipe_fft_sized(const RunDesc& R, const Item& I, float2* s) {
+  if constexpr (L >= 11) {
+    if (PASS == 0) big_rows_inv_item<L>(R, I.a, I.c, s, R.tw);
+    else if (PASS == 1) big_rows_fwd_item<L, true>(R, I.a, I.c, s, R.tw);
+    else big_cols_item<L>(R, I.a, I.c, s, R.tw);
+  } else {
+    if (PASS == 0) fft2_rows_inv_item<L, false>(CtaTeam(), R, I.a, I.c, s, R.tw);
+    else if (PASS == 1) fft2_rows_fwd_item<L, false, true>(CtaTeam(), R, I.a, I.c, s, R.tw);
+    else fft2_cols_item<L, false>(CtaTeam(), R, I.a, I.c, s, R.tw);
+  }
+}
+
 template <int PASS>
 __device__ __forceinline__ void pipe_fft_item(const RunDesc& R, const Item& I, float2* s) {
   switch (I.b) {
-#define BD_CASE(L)                                                      \
-  case L:                                                               \
-    if (PASS == 0) fft2_rows_inv_item<L, false>(CtaTeam(), R, I.a, I.c, s, R.tw);       \
-    else if (PASS == 1) fft2_rows_fwd_item<L, false, true>(CtaTeam(), R, I.a, I.c, s, R.tw); \
-    else fft2_cols_item<L, false>(CtaTeam(), R, I.a, I.c, s, R.tw);                    \
+#define BD_CASE(L)                   \
+  case L:                            \
+    pipe_fft_sized<PASS, L>(R, I, s); \
     break;
     BD_PIPE_SIZES(BD_CASE)
 #undef BD_CASE
@@ -1440,10 +1474,7 @@ static int launch_fft2(int pass, int lz, const RunDesc* runs, const RunDyn* dyn,
     if (pass == 0)                                                                                      \
       k_fft2_rows_fwd<L><<<p.n, p.threads, p.smem, s>>>(runs, dyn, p.items, p.n, require_active);      \
     else if (pass == 1)                                                                                 \
-      if (p.threads > FFT2_THREADS)                                                                      \
-        k_fft2_cols_wide<L><<<p.n, p.threads, p.smem, s>>>(runs, dyn, p.items, p.n, require_active);   \
-      else                                                                                              \
-        k_fft2_cols<L><<<p.n, p.threads, p.smem, s>>>(runs, dyn, p.items, p.n, require_active);        \
+      k_fft2_cols<L><<<p.n, p.threads, p.smem, s>>>(runs, dyn, p.items, p.n, require_active);        \
     else                                                                                                \
       k_fft2_rows_inv<L><<<p.n, p.threads, p.smem, s>>>(runs, dyn, p.items, p.n, require_active);      \
     break;
@@ -1490,29 +1521,36 @@ int launch_particles(const RunDesc* runs, RunDyn* dyn, const Item* items, int n,
   return 0;
 }
 
-int launch_step(const RunDesc* runs, RunDyn* dyn, const Item* items, int n, int deposit, cudaStream_t s, int shape) {
+int launch_step(const RunDesc* runs, RunDyn* dyn, const Item* items, int n, int deposit, int large,
+                cudaStream_t s, int shape) {
   if (n <= 0) return 0;
-  // The pipelined step (deposit): one wave of resident CTAs, each taking
-  // items blockIdx.x, +gridDim.x, ... (256-run ensemble: particle phase
-  // 0.429 -> 0.407 ms). Otherwise one CTA per item: for one large run the
-  // resident wave was slower (0.152 -> 0.190 ms; two waves 0.179).
-  // resident CTAs per SM of each shape, asked once per process (every
-  // device of one process is taken to be the same GPU model)
-  static int resident[2] = {0, 0};
-  const int sh = shape == PART_SHAPE_5CTA ? 1 : 0;
-  if (!resident[sh]) {
-    int per = 0;
-    const cudaError_t e = sh ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_step<5, true>, 256, 0)
-                             : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_step<4, true>, 256, 0);
-    resident[sh] = (e == cudaSuccess && per > 0) ? per : 1;
-  }
-  const int g = deposit ? grid_for(n, resident[sh] * sm_count()) : grid_for(n, 65535);
-  if (deposit) {
-    if (sh) k_step<5, true><<<g, 256, 0, s>>>(runs, dyn, items, n);
-    else k_step<4, true><<<g, 256, 0, s>>>(runs, dyn, items, n);
+  const bool five = shape == PART_SHAPE_5CTA;
+  if (large) {
+    // one CTA per item, four per SM: the block that starts when this one ends
+    constexpr int ahead = 592;
+    const int g = grid_for(n, 65535);
+    if (deposit) k_step<4, true, ahead><<<g, 256, 0, s>>>(runs, dyn, items, n);
+    else k_step<4, false, ahead><<<g, 256, 0, s>>>(runs, dyn, items, n);
   } else {
-    if (sh) k_step<5, false><<<g, 256, 0, s>>>(runs, dyn, items, n);
-    else k_step<4, false><<<g, 256, 0, s>>>(runs, dyn, items, n);
+    // one wave of resident CTAs, each taking items blockIdx.x, +gridDim.x, ...
+    // (256-run ensemble: 398 us with one CTA per item, 333 us)
+    // resident CTAs per SM of each shape, asked once per process (every
+    // device of one process is taken to be the same GPU model)
+    static int resident[2] = {0, 0};
+    if (!resident[five]) {
+      int per = 0;
+      const cudaError_t e = five ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_step<5, true, 0>, 256, 0)
+                                 : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_step<4, true, 0>, 256, 0);
+      resident[five] = (e == cudaSuccess && per > 0) ? per : 1;
+    }
+    const int g = deposit ? grid_for(n, resident[five] * sm_count()) : grid_for(n, 65535);
+    if (deposit) {
+      if (five) k_step<5, true, 0><<<g, 256, 0, s>>>(runs, dyn, items, n);
+      else k_step<4, true, 0><<<g, 256, 0, s>>>(runs, dyn, items, n);
+    } else {
+      if (five) k_step<5, false, 0><<<g, 256, 0, s>>>(runs, dyn, items, n);
+      else k_step<4, false, 0><<<g, 256, 0, s>>>(runs, dyn, items, n);
+    }
   }
   BD_LAUNCH_CHECK();
   return 0;
@@ -1638,8 +1676,6 @@ int set_kernel_attributes() {
   e = cudaFuncSetAttribute(k_fft2_rows_fwd<L>, cudaFuncAttributeMaxDynamicSharedMemorySize, MAX_FFT_SMEM); \
   if (e != cudaSuccess) return (int)e;                                                                  \
   e = cudaFuncSetAttribute(k_fft2_cols<L>, cudaFuncAttributeMaxDynamicSharedMemorySize, MAX_FFT_SMEM);     \
-  if (e != cudaSuccess) return (int)e;                                                                  \
-  e = cudaFuncSetAttribute(k_fft2_cols_wide<L>, cudaFuncAttributeMaxDynamicSharedMemorySize, MAX_FFT_SMEM); \
   if (e != cudaSuccess) return (int)e;                                                                  \
   e = cudaFuncSetAttribute(k_fft2_rows_inv<L>, cudaFuncAttributeMaxDynamicSharedMemorySize, MAX_FFT_SMEM); \
   if (e != cudaSuccess) return (int)e;

@@ -19,7 +19,6 @@ enum CellblockMode { MODE_STEP = 0, MODE_SET = 1, MODE_ADD = 2, MODE_FORCES = 3 
 constexpr int SCAN_CHUNK = 2048;
 constexpr int FFT_THREADS = 512;
 constexpr int FFT2_THREADS = 256;  // power-of-two path (register-radix transform)
-constexpr int FFT2_WIDE_THREADS = 1024;  // column pass of meshes of 2048 and more (several columns per item)
 constexpr int MAX_FFT_SMEM = 200 * 1024;
 
 // One FFT launch: its items, dynamic shared memory and threads per CTA.
@@ -54,9 +53,10 @@ enum PartShape { PART_SHAPE_DEFAULT = 0, PART_SHAPE_5CTA = 1 };
 int launch_particles(const RunDesc* runs, RunDyn* dyn, const Item* items, int n, int mode,
                      int mask, int require_active, cudaStream_t s, int shape = PART_SHAPE_DEFAULT);
 // forces and move of the runs whose step budget is not used up; deposit: also
-// add the new positions to each run's R.dacc
-int launch_step(const RunDesc* runs, RunDyn* dyn, const Item* items, int n, int deposit, cudaStream_t s,
-                int shape = PART_SHAPE_DEFAULT);
+// add the new positions to each run's R.dacc; large: the form for runs whose
+// arrays do not stay in L2 (shape is not used)
+int launch_step(const RunDesc* runs, RunDyn* dyn, const Item* items, int n, int deposit, int large,
+                cudaStream_t s, int shape = PART_SHAPE_DEFAULT);
 // Pipelined stage step (power-of-two meshes, fixed dt, every run with its
 // R.dacc): particles (launch_step with deposit), then the scan and the
 // scatter with the step end beside the transform of the new density:

@@ -126,3 +126,34 @@ def test_resident_batch_equals_stage_kernels(gpu, adaptive):
     for k in range(len(runs)):
         _same(a.get_positions(k), b.get_positions(k))
         assert a.time(k) == b.time(k)
+
+
+@pytest.mark.parametrize("mesh", [2048, 4096])
+def test_large_mesh_pipelined_equals_stage_kernels(gpu, mesh):
+    """One run on a mesh beyond the resident step's: the pipelined step (its
+    transforms read and write global memory in their outer passes, the
+    spectrum by column) against the stage kernels and, after new positions,
+    again; 140 000 particles take the particle kernel's form for large runs."""
+    p = _params(gpu, 80000, 60001, mesh, False, scheme=2, rho=0.05)
+    start, other = _lattice(p, 11), _lattice(p, 12)
+    a, b = gpu.Run(p, seed=5), gpu.Run(p, seed=5)
+    assert a.launches_per_step() == 6
+    for r, steps in ((a, a.zeitschritte), (b, b.stage_times)):
+        r.set_positions_all(start)
+        steps(4)
+        r.set_positions_all(other)
+        steps(3)
+        r.zeitschritt()
+        steps(2)
+    _same(a.get_positions(), b.get_positions())
+    assert a.time() == b.time()
+    a.forces()
+    fa = a.get_forces()
+    import oracle
+    o = oracle.Oracle(p, 1)
+    pos = a.get_positions()
+    o.set_positions(pos)
+    fo = o.forces()
+    for s in (0, 1):  # FP32 transforms of 2^22 points and more: 1e-5 as the parity tests
+        d = np.linalg.norm(fa[("kap", s)] - fo[("kap", s)]) / np.linalg.norm(fo[("kap", s)])
+        assert d <= 1e-5
