@@ -283,9 +283,8 @@ int bd_zeitschritte(bd_ctx* c, long long nsteps, double* t_out) {
   bd::RunDyn y0;
   RK(c->e.get_dyn(0, &y0));
   RK(c->e.step(nsteps));
-  RK(c->e.sync_check());
   bd::RunDyn y;
-  RK(c->e.get_dyn(0, &y));
+  RK(c->e.sync_check(&y));
   c->t_obs += (long double)(y.t - y0.t);
   if (t_out) *t_out = y.t;
   return BD_OK;

@@ -7,6 +7,8 @@
 #include <climits>
 #include <cmath>
 #include <cstring>
+#include <map>
+#include <tuple>
 
 #include "bd_fft2.cuh"
 #include "bd_host.h"
@@ -175,6 +177,7 @@ Engine::~Engine() {
   }
   if (stream) cudaStreamSynchronize(stream);
   if (h_stage) cudaFreeHost(h_stage);
+  if (h_dyn) cudaFreeHost(h_dyn);
   if (ev_stage) cudaEventDestroy(ev_stage);
   for (auto& e : ev_piece)
     if (e) cudaEventDestroy(e);
@@ -473,25 +476,23 @@ static Item resident_item(const RunHost& r, int run, int G, int nt, size_t* smem
   return I;
 }
 
-// Clusters of cs (1, 2, 4, 8, 16) CTAs of the many-run kernels that the device
-// holds at once: every mesh's kernel has the same threads, register bound and
-// largest shared memory, so one of them is asked, once per process, device and
-// size (an occupancy query takes a few hundred microseconds).
-static int clusters_fit(int cs, int device) {
+// Whether a resident kernel can run: its attributes set, the CTAs (cs 0) or
+// clusters of cs CTAs that the device holds at once at the kernels' largest
+// shared memory (0: none). Asked once per process, device and kernel: the
+// queries take a few hundred microseconds, a served mix plans every tick.
+static int resident_fit(int lz, bool single, int cs, int device) {
   static std::mutex mu;
-  static int fit[64][5] = {};
-  if (device < 0 || device >= 64) return 0;
-  const int k = ilog2(cs);
+  static std::map<std::tuple<int, int, bool, int>, int> known;  // a few hundred entries at most
   std::lock_guard<std::mutex> g(mu);
-  if (!fit[device][k]) {
-    int n = 0;
-    if (resident_configure(7, false, res_max_smem(false), cs, device, &n) || n <= 0) {
-      cudaGetLastError();
-      n = -1;
-    }
-    fit[device][k] = n;
+  const auto key = std::make_tuple(device, lz, single, cs);
+  const auto f = known.find(key);
+  if (f != known.end()) return f->second;
+  int n = 0;
+  if (resident_configure(lz, single, res_max_smem(single), cs, device, &n) || n < 0) {
+    cudaGetLastError();
+    n = 0;
   }
-  return std::max(0, fit[device][k]);
+  return known[key] = n;
 }
 
 // The resident step's work items, appended to the plan's lists (several
@@ -534,7 +535,7 @@ void Engine::resident_items(std::vector<Item>& all) {
     e.cs = cs;
     e.I = resident_item(r, (int)k, cs, res_threads(false) / 2, &e.smem);
     e.load = weight(r) / cs;
-    const int n = e.smem + (size_t)res_pcap(false) * 32 <= res_max_smem(false) ? clusters_fit(cs, device) : 0;
+    const int n = e.smem + (size_t)res_pcap(false) * 32 <= res_max_smem(false) ? resident_fit(e.lz, false, cs, device) : 0;
     e.share = n > 0 ? 1.0 / n : 1e9;
     return e;
   };
@@ -597,15 +598,8 @@ int Engine::plan_resident() {
     CK(cudaMemsetAsync(d_bar, 0, 2 * sizeof(unsigned), stream));
   }
   if (runs.size() > 1) {
-    for (const ResGroup& g : res_groups) {
-      if (res_configured.count(g.lz)) continue;
-      int n = 0;
-      if (resident_configure(g.lz, false, g.smem + (size_t)res_pcap(false) * 32, g.cs, device, &n) || n <= 0) {
-        cudaGetLastError();
-        return BD_OK;
-      }
-      res_configured.insert(g.lz);
-    }
+    for (const ResGroup& g : res_groups)
+      if (resident_fit(g.lz, false, g.cs, device) <= 0) return BD_OK;
     while (res_streams.size() + 1 < res_groups.size()) {
       cudaStream_t s = nullptr;
       CK(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
@@ -632,15 +626,10 @@ int Engine::plan_resident() {
   rone_grid = resident_item(r, 0, want, res_threads(true) / 2, &sm_g);
   const size_t work = std::max(sm_c, sm_g);
   rone_smem = work + (size_t)res_pcap(true) * 32;
-  int n = 0;
-  if (res_cs && (resident_configure(rone_lz, true, rone_smem, res_cs, device, &n) || n <= 0)) {
-    cudaGetLastError();
-    res_cs = 0;
-  }
-  if (resident_configure(rone_lz, true, rone_smem, 0, device, &n) || n <= 0) {
-    cudaGetLastError();
-    return BD_OK;
-  }
+  if (rone_smem > res_max_smem(true)) return BD_OK;
+  if (res_cs && resident_fit(rone_lz, true, res_cs, device) <= 0) res_cs = 0;
+  const int n = resident_fit(rone_lz, true, 0, device);
+  if (n <= 0) return BD_OK;
   res_grid = std::min(n, want);
   rone = ResArgs{};
   rone.one = table_desc(0);
@@ -772,13 +761,25 @@ int Engine::stage_buffer(size_t bytes, void** out) {
   return BD_OK;
 }
 
+int Engine::fetch_dyn(size_t first, size_t n) {
+  if (n > h_dyn_cap) {
+    if (h_dyn) CK(cudaFreeHost(h_dyn));
+    h_dyn = nullptr;
+    h_dyn_cap = 0;
+    const size_t cap = n + n / 2 + 4;
+    CK(cudaHostAlloc((void**)&h_dyn, cap * sizeof(RunDyn), cudaHostAllocDefault));
+    h_dyn_cap = cap;
+  }
+  if (n) CK(cudaMemcpyAsync(h_dyn, d_dyn + first, n * sizeof(RunDyn), cudaMemcpyDeviceToHost, stream));
+  CK(cudaStreamSynchronize(stream));
+  return BD_OK;
+}
+
 // the device state of every run back into the host mirrors (one copy)
 int Engine::download_dyn() {
   if (!tables_ok || runs.empty()) return BD_OK;
-  std::vector<RunDyn> hy(runs.size());
-  CK(cudaStreamSynchronize(stream));
-  CK(d2h(stream, hy.data(), d_dyn, hy.size() * sizeof(RunDyn)));
-  for (size_t k = 0; k < runs.size(); k++) runs[k]->dyn = hy[k];
+  RK(fetch_dyn(0, runs.size()));
+  for (size_t k = 0; k < runs.size(); k++) runs[k]->dyn = h_dyn[k];
   return BD_OK;
 }
 
@@ -1677,15 +1678,18 @@ int Engine::step(long long nsteps) {
   return BD_OK;
 }
 
-int Engine::sync_check() {
+int Engine::sync_check(RunDyn* dd) {
   CK(cudaSetDevice(device));
-  CK(cudaStreamSynchronize(stream));
-  if (!tables_ok) return BD_OK;
-  std::vector<RunDyn> hy(runs.size());
-  if (!runs.empty()) CK(d2h(stream, hy.data(), d_dyn, hy.size() * sizeof(RunDyn)));
-  for (auto& y : hy) {
-    if (y.err & E_NONFINITE) return BD_ERR_NONFINITE;
-    if (y.err & E_BARRIER_TIMEOUT) {
+  if (!tables_ok) {
+    CK(cudaStreamSynchronize(stream));
+    if (dd && !runs.empty()) *dd = runs[0]->dyn;
+    return BD_OK;
+  }
+  RK(fetch_dyn(0, runs.size()));
+  if (dd && !runs.empty()) *dd = h_dyn[0];
+  for (size_t k = 0; k < runs.size(); k++) {
+    if (h_dyn[k].err & E_NONFINITE) return BD_ERR_NONFINITE;
+    if (h_dyn[k].err & E_BARRIER_TIMEOUT) {
       RK(recover_fused());
       return BD_ERR_TIMEOUT;
     }
@@ -1748,8 +1752,8 @@ int Engine::get_dyn(size_t run, RunDyn* dd) {
     *dd = runs[run]->dyn;
     return BD_OK;
   }
-  CK(cudaStreamSynchronize(stream));
-  CK(d2h(stream, dd, d_dyn + run, sizeof(RunDyn)));
+  RK(fetch_dyn(run, 1));
+  *dd = h_dyn[0];
   return BD_OK;
 }
 
@@ -1789,8 +1793,8 @@ int Engine::get_dyn_all(std::vector<RunDyn>& out) {
     for (size_t k = 0; k < runs.size(); k++) out[k] = runs[k]->dyn;
     return BD_OK;
   }
-  CK(cudaStreamSynchronize(stream));
-  CK(d2h(stream, out.data(), d_dyn, runs.size() * sizeof(RunDyn)));
+  RK(fetch_dyn(0, runs.size()));
+  std::copy(h_dyn, h_dyn + runs.size(), out.begin());
   return BD_OK;
 }
 
@@ -2213,19 +2217,44 @@ int Engine::fused_prologue(bool grids) {
   return BD_OK;
 }
 
+// A force array of one species through the pinned staging buffer, in pieces
+// that are widened to double on the host pool as their copies end (as the
+// positions; pageable copies and one host thread before: 65 536 particles,
+// four arrays and their evaluation 1.2 ms).
 int Engine::get_forces(int kind, int species, double* out) {
   if (runs.empty() || species < 0 || species > 1 || kind < 0 || kind > 2) return BD_ERR_ARG;
   RunHost& r = *runs[0];
-  CK(cudaStreamSynchronize(stream));
-  const int lo = species == 0 ? 0 : r.p.N1;
-  const int cnt = species == 0 ? r.p.N1 : r.p.N2;
-  std::vector<float2> h(cnt + 1);
-  const float2* src = kind == 0 ? r.d.Fw : kind == 1 ? r.d.Fk : r.d.Fn;
-  if (cnt > 0) CK(d2h(stream, h.data(), src + lo, cnt * sizeof(float2)));
-  for (int i = 0; i < cnt; i++) {
-    out[2 * i] = h[i].x;
-    out[2 * i + 1] = h[i].y;
+  CK(cudaSetDevice(device));
+  const long long lo = species == 0 ? 0 : r.p.N1;
+  const long long cnt = species == 0 ? r.p.N1 : r.p.N2;
+  const float2* src = (kind == 0 ? r.d.Fw : kind == 1 ? r.d.Fk : r.d.Fn) + lo;
+  void* buf = nullptr;
+  RK(stage_buffer((size_t)std::max(cnt, 1ll) * sizeof(float2), &buf));
+  float2* h = static_cast<float2*>(buf);
+  const int np = copy_pieces(cnt);
+  const long long per = np > 0 ? (cnt + np - 1) / np : 0;
+  for (int k = 0; k < np; k++) {
+    const long long t0 = k * per, t1 = std::min(cnt, t0 + per);
+    if (t0 >= t1) break;
+    CK(cudaMemcpyAsync(h + t0, src + t0, (size_t)(t1 - t0) * sizeof(float2), cudaMemcpyDeviceToHost, stream));
+    CK(cudaEventRecord(ev_piece[k], stream));
   }
+  if (np == 0) CK(cudaStreamSynchronize(stream));
+  std::vector<cudaError_t> err(np, cudaSuccess);
+  const int dev = device;
+  host_pool().run(np, [&](int k) {
+    const long long t0 = k * per, t1 = std::min(cnt, t0 + per);
+    if (t0 >= t1) return;
+    cudaError_t e = cudaSetDevice(dev);
+    if (e == cudaSuccess) e = cudaEventSynchronize(ev_piece[k]);
+    err[k] = e;
+    if (e == cudaSuccess)
+      for (long long i = t0; i < t1; i++) {
+        out[2 * i] = h[i].x;
+        out[2 * i + 1] = h[i].y;
+      }
+  });
+  for (int k = 0; k < np; k++) CK(err[k]);
   return BD_OK;
 }
 

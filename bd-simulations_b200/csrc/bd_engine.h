@@ -8,7 +8,6 @@
 #include <memory>
 #include <mutex>
 #include <random>
-#include <set>
 #include <string>
 #include <thread>
 #include <vector>
@@ -95,7 +94,8 @@ class Engine {
   int sort_uploaded_run(size_t run);
 
   int step(long long nsteps);  // fused steps for every run
-  int sync_check();            // synchronise and report run errors
+  // synchronise and report run errors; dd: also the first run's state
+  int sync_check(RunDyn* dd = nullptr);
   int get_dyn(size_t run, RunDyn* d);
   int set_dyn_field_step(size_t run, unsigned long long step);
   int set_dyn_time(size_t run, double t, float dt);
@@ -181,6 +181,11 @@ class Engine {
   size_t h_stage_cap = 0;
   cudaEvent_t ev_stage = nullptr;
   int stage_buffer(size_t bytes, void** out);
+  // pinned copies of the run states (RunDyn), read back after most calls: a
+  // copy into pageable memory is staged by the driver and waits twice
+  RunDyn* h_dyn = nullptr;
+  size_t h_dyn_cap = 0;
+  int fetch_dyn(size_t first, size_t n);  // states [first, first + n) into h_dyn, after everything queued
   // the device -> host copies of a run's records go in up to this many
   // pieces, each with its event, converted as they arrive
   static constexpr int MAX_COPY_PIECES = 64;
@@ -205,7 +210,6 @@ class Engine {
     double load;  // particles per CTA of its largest run
   };
   std::vector<ResGroup> res_groups;
-  std::set<int> res_configured;           // mesh classes whose kernel attributes are set
   std::vector<cudaStream_t> res_streams;  // for the second and later groups
   cudaEvent_t ev_res = nullptr;
   ResArgs rone{};
