@@ -466,10 +466,10 @@ static Item resident_item(const RunHost& r, int run, int G, int nt, size_t* smem
                       std::max((size_t)2 * (1 << I.b) * fft2_stride(Z), (size_t)(1 << I.c) * fft2_stride(Z))) *
              8;
   } else {
-    // up to two butterflies per thread and stage
-    I.a = size(Z, n, n / 8);
-    I.b = size(n, 2 * Z, Z / 4);
-    I.c = size(Z, Z, Z / 8);
+    // 12 to 16 elements per thread (two stages a pass, fftc_stage2)
+    I.a = size(Z, n, n / 12);
+    I.b = size(n, 2 * Z, Z / 6);
+    I.c = size(Z, Z, Z / 12);
     *smem += std::max((size_t)n << I.a, std::max((size_t)(2 * Z) << I.b, (size_t)Z << I.c)) * 8;
   }
   *smem = (*smem + 255) & ~(size_t)255;
