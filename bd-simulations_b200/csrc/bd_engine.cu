@@ -480,15 +480,15 @@ static Item resident_item(const RunHost& r, int run, int G, int nt, size_t* smem
 // clusters of cs CTAs that the device holds at once at the kernels' largest
 // shared memory (0: none). Asked once per process, device and kernel: the
 // queries take a few hundred microseconds, a served mix plans every tick.
-static int resident_fit(int lz, bool single, int cs, int device) {
+static int resident_fit(int lz, int kind, int cs, int device) {
   static std::mutex mu;
-  static std::map<std::tuple<int, int, bool, int>, int> known;  // a few hundred entries at most
+  static std::map<std::tuple<int, int, int, int>, int> known;  // a few hundred entries at most
   std::lock_guard<std::mutex> g(mu);
-  const auto key = std::make_tuple(device, lz, single, cs);
+  const auto key = std::make_tuple(device, lz, kind, cs);
   const auto f = known.find(key);
   if (f != known.end()) return f->second;
   int n = 0;
-  if (resident_configure(lz, single, res_max_smem(single), cs, device, &n) || n < 0) {
+  if (resident_configure(lz, kind, res_max_smem(kind), cs, device, &n) || n < 0) {
     cudaGetLastError();
     n = 0;
   }
@@ -501,6 +501,7 @@ void Engine::resident_items(std::vector<Item>& all) {
   resident = false;
   fused = false;
   res_groups.clear();
+  res_share_grid = 0;
   if (runs.empty()) return;
   for (auto* r : runs)
     if (!resident_run(*r)) return;
@@ -521,9 +522,8 @@ void Engine::resident_items(std::vector<Item>& all) {
   std::vector<Ent> v;
   // load: particles and a quarter of the mesh points per CTA
   auto weight = [&](const RunHost& r) { return r.N + (r.idgas ? 0.0 : 0.25 * r.Z * r.Z); };
-  const double limit = piped ? 800.0 : 20000.0;
-  for (auto* r : runs)
-    if (weight(*r) > 16 * limit) return;
+  long long particles = 0;
+  for (auto* r : runs) particles += r->N;
   // every run on clusters of one size, the largest at which the whole batch
   // is resident at once; then larger clusters for runs that would hold the
   // others up, while there is room to spare. share: the part of the GPU one
@@ -533,9 +533,9 @@ void Engine::resident_items(std::vector<Item>& all) {
     Ent e{};
     e.lz = resident_lz(r);
     e.cs = cs;
-    e.I = resident_item(r, (int)k, cs, res_threads(false) / 2, &e.smem);
+    e.I = resident_item(r, (int)k, cs, res_threads(RES_CLUSTERS) / 2, &e.smem);
     e.load = weight(r) / cs;
-    const int n = e.smem + (size_t)res_pcap(false) * 32 <= res_max_smem(false) ? resident_fit(e.lz, false, cs, device) : 0;
+    const int n = e.smem + (size_t)res_pcap(RES_CLUSTERS) * 32 <= res_max_smem(RES_CLUSTERS) ? resident_fit(e.lz, RES_CLUSTERS, cs, device) : 0;
     e.share = n > 0 ? 1.0 / n : 1e9;
     return e;
   };
@@ -564,13 +564,52 @@ void Engine::resident_items(std::vector<Item>& all) {
       v.swap(w);
     }
   }
-  // loads where the launch-per-step forms are the better ones. Measured, us per step
-  // (resident | other), runs x particles: pipelined step 8 x 4000 16 | 23,
-  // 32 x 4000 24 | 28, 64 x 2000 25 | 29 (loads to 760), 64 x 4000 41 | 40,
-  // 32 x 8000 40 | 38 (from 1260 on). Stage kernels (adaptive dt or meshes
-  // with a factor 3): 16 x 8000 84 | 208, 64 x 32 000 522 | 912 (load 17 000,
-  // the largest measured)
-  if (v.empty() || most > limit) return;
+  // the same for groups of CTAs of one cooperative grid, a CTA at a time to
+  // the run with the largest load
+  int nsm = 0;
+  if (cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) nsm = 0;
+  const int fit = (int)runs.size() <= std::min(nsm, (int)BAR_GROUPS) ? resident_fit(-1, RES_GROUPS, 0, device) : 0;
+  const int slots = std::min(nsm, fit);
+  std::vector<int> share(runs.size(), 1);
+  double most_g = 1e30;
+  if (slots >= (int)runs.size()) {
+    auto top = [&]() {
+      size_t t = 0;
+      for (size_t k = 1; k < runs.size(); k++)
+        if (weight(*runs[k]) / share[k] > weight(*runs[t]) / share[t]) t = k;
+      return t;
+    };
+    for (int left = slots - (int)runs.size(); left > 0; left--) share[top()]++;
+    const size_t t = top();
+    most_g = weight(*runs[t]) / share[t];
+  }
+  // Which form: estimates of a step in us, fitted to measurements of 1 to 128
+  // runs of 1000 to 250 000 particles (clusters 12-60, groups 14-45, the
+  // pipelined step 20-110; the stage kernels, 45-900, were never the fastest)
+  const double t_clusters = v.empty() ? 1e30 : 8.0 + 0.025 * most;
+  const double t_groups = 14.0 + 0.016 * most_g;
+  const double t_piped = piped ? 19.0 + 8e-5 * particles : 1e30;
+  if (std::min(t_clusters, t_groups) > t_piped) return;
+  if (t_groups < t_clusters) {
+    off_share = (int)all.size();
+    res_share_smem = 0;
+    for (size_t k = 0; k < runs.size(); k++) {
+      size_t sm = 0;
+      const Item I = resident_item(*runs[k], (int)k, share[k], res_threads(RES_GROUPS) / 2, &sm);
+      res_share_smem = std::max(res_share_smem, sm);
+      for (int c = 0; c < share[k]; c++) {
+        all.push_back(I);
+        all.push_back({resident_lz(*runs[k]), (int)k, c, share[k]});
+        res_share_grid++;
+      }
+    }
+    if (res_share_smem + (size_t)res_pcap(RES_GROUPS) * 32 > res_max_smem(RES_GROUPS)) {
+      res_share_grid = 0;
+      return;
+    }
+    resident = true;
+    return;
+  }
   std::stable_sort(v.begin(), v.end(), [](const Ent& a, const Ent& b) {
     return a.lz != b.lz ? a.lz < b.lz : a.cs != b.cs ? a.cs > b.cs : a.load > b.load;
   });
@@ -594,12 +633,12 @@ int Engine::plan_resident() {
   if (!resident) return BD_OK;
   resident = false;
   if (!d_bar) {
-    CK(cudaMalloc(&d_bar, 2 * sizeof(unsigned)));
-    CK(cudaMemsetAsync(d_bar, 0, 2 * sizeof(unsigned), stream));
+    CK(cudaMalloc(&d_bar, 2 * BAR_GROUPS * sizeof(unsigned)));
+    CK(cudaMemsetAsync(d_bar, 0, 2 * BAR_GROUPS * sizeof(unsigned), stream));
   }
   if (runs.size() > 1) {
     for (const ResGroup& g : res_groups)
-      if (resident_fit(g.lz, false, g.cs, device) <= 0) return BD_OK;
+      if (resident_fit(g.lz, RES_CLUSTERS, g.cs, device) <= 0) return BD_OK;
     while (res_streams.size() + 1 < res_groups.size()) {
       cudaStream_t s = nullptr;
       CK(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
@@ -622,13 +661,13 @@ int Engine::plan_resident() {
   // arrivals
   const int want = std::max(32, std::min(nsm, std::max((r.N + 63) / 64, r.idgas ? 0 : r.Z / 3)));
   size_t sm_c = 0, sm_g = 0;
-  rone_cluster = resident_item(r, 0, 16, res_threads(true) / 2, &sm_c);
-  rone_grid = resident_item(r, 0, want, res_threads(true) / 2, &sm_g);
+  rone_cluster = resident_item(r, 0, 16, res_threads(RES_SINGLE) / 2, &sm_c);
+  rone_grid = resident_item(r, 0, want, res_threads(RES_SINGLE) / 2, &sm_g);
   const size_t work = std::max(sm_c, sm_g);
-  rone_smem = work + (size_t)res_pcap(true) * 32;
-  if (rone_smem > res_max_smem(true)) return BD_OK;
-  if (res_cs && resident_fit(rone_lz, true, res_cs, device) <= 0) res_cs = 0;
-  const int n = resident_fit(rone_lz, true, 0, device);
+  rone_smem = work + (size_t)res_pcap(RES_SINGLE) * 32;
+  if (rone_smem > res_max_smem(RES_SINGLE)) return BD_OK;
+  if (res_cs && resident_fit(rone_lz, RES_SINGLE, res_cs, device) <= 0) res_cs = 0;
+  const int n = resident_fit(rone_lz, RES_SINGLE, 0, device);
   if (n <= 0) return BD_OK;
   res_grid = std::min(n, want);
   rone = ResArgs{};
@@ -636,7 +675,7 @@ int Engine::plan_resident() {
   rone.dyn = d_dyn;
   rone.bar = d_bar;
   rone.part_off = (int)work;
-  rone.pcap = res_pcap(true);
+  rone.pcap = res_pcap(RES_SINGLE);
   resident = true;
   fused = r.d.dacc != nullptr;
   return BD_OK;
@@ -665,7 +704,7 @@ int Engine::launch_one(int nsteps, bool fault, unsigned long long* ts) {
     A.max_polls = fault_polls;
     fault_barrier = 0;
   }
-  return launch_resident(rone_lz, true, A, 1, cs, res_grid, rone_smem, stream) ? BD_ERR_CUDA : BD_OK;
+  return launch_resident(rone_lz, RES_SINGLE, A, 1, cs, res_grid, rone_smem, stream) ? BD_ERR_CUDA : BD_OK;
 }
 
 // nsteps resident steps of every run, at most res_chunk per launch. Several
@@ -684,6 +723,21 @@ int Engine::step_resident(long long nsteps) {
     }
     return BD_OK;
   }
+  if (res_share_grid > 0) {
+    ResArgs A{};
+    A.runs = d_runs;
+    A.dyn = d_dyn;
+    A.items = it(off_share);
+    A.bar = d_bar;
+    A.part_off = (int)res_share_smem;
+    A.pcap = res_pcap(RES_GROUPS);
+    while (nsteps > 0) {
+      A.nsteps = (int)std::min<long long>(nsteps, res_chunk);
+      RK(launch_resident(-1, RES_GROUPS, A, 0, 0, res_share_grid, res_share_smem + (size_t)A.pcap * 32, stream));
+      nsteps -= A.nsteps;
+    }
+    return BD_OK;
+  }
   const size_t ng = res_groups.size();
   if (ng > 1) {
     CK(cudaEventRecord(ev_res, stream));
@@ -698,8 +752,8 @@ int Engine::step_resident(long long nsteps) {
       const ResGroup& q = res_groups[g];
       A.items = it(q.off);
       A.part_off = (int)q.smem;
-      A.pcap = res_pcap(false);
-      RK(launch_resident(q.lz, false, A, q.n, q.cs, 0, q.smem + (size_t)A.pcap * 32, g ? res_streams[g - 1] : stream));
+      A.pcap = res_pcap(RES_CLUSTERS);
+      RK(launch_resident(q.lz, RES_CLUSTERS, A, q.n, q.cs, 0, q.smem + (size_t)A.pcap * 32, g ? res_streams[g - 1] : stream));
     }
     nsteps -= A.nsteps;
   }
@@ -1090,8 +1144,8 @@ int Engine::plan_tail() {
     return BD_OK;
   }
   if (!d_bar) {
-    CK(cudaMalloc(&d_bar, 2 * sizeof(unsigned)));
-    CK(cudaMemsetAsync(d_bar, 0, 2 * sizeof(unsigned), stream));
+    CK(cudaMalloc(&d_bar, 2 * BAR_GROUPS * sizeof(unsigned)));
+    CK(cudaMemsetAsync(d_bar, 0, 2 * BAR_GROUPS * sizeof(unsigned), stream));
   }
   tplan = P;
   tail_ok = true;
@@ -1708,7 +1762,7 @@ int Engine::sync_check(RunDyn* dd) {
 // of the unchanged records; the next step recomputes the spectrum (prologue).
 // The step can then be taken again with the same bits.
 int Engine::recover_fused() {
-  if (d_bar) CK(cudaMemsetAsync(d_bar, 0, 2 * sizeof(unsigned), stream));
+  if (d_bar) CK(cudaMemsetAsync(d_bar, 0, 2 * BAR_GROUPS * sizeof(unsigned), stream));
   for (size_t k = 0; k < runs.size(); k++) {
     RunDesc& d = runs[k]->d;
     const size_t cc = (size_t)runs[k]->C * runs[k]->C;

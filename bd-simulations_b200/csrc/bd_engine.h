@@ -202,7 +202,8 @@ class Engine {
   // resident step (bd_resident.cuh): the step loop of a run in one launch.
   // resident: every run qualifies; one run: rone (cluster of res_cs CTAs, or
   // the cooperative grid of res_grid CTAs when res_cs is 0); several runs:
-  // one launch per group (mesh size, cluster size), on streams of their own
+  // one launch per group (mesh size, cluster size), on streams of their own, or
+  // (res_share_grid > 0) one cooperative launch of that many CTAs shared out
   bool resident = false;
   struct ResGroup {
     int lz, cs, off, n;
@@ -216,6 +217,8 @@ class Engine {
   Item rone_cluster{}, rone_grid{};  // item sizes of the two modes
   int rone_lz = 0, res_cs = 0, res_grid = 0;
   size_t rone_smem = 0;
+  int res_share_grid = 0, off_share = 0;
+  size_t res_share_smem = 0;
   int res_chunk = 1;  // steps per launch
   void resident_items(std::vector<Item>& all);
   int plan_resident();
@@ -225,7 +228,8 @@ class Engine {
   // one run on a power-of-two mesh with a fixed dt, resident (the fused step
   // of the API: bd_fused_phase_times, bd_inject_barrier_timeout)
   bool fused = false;
-  unsigned* d_bar = nullptr;
+  unsigned* d_bar = nullptr;  // barrier words, two per group of CTAs (BAR_GROUPS of them)
+  static constexpr int BAR_GROUPS = 256;
   // pipelined stage step (power-of-two meshes, fixed dt, two or more runs or one
   // on a mesh of 2048 or 4096):
   // six launches per step, the density deposited in the move, its transform

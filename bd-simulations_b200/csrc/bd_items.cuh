@@ -937,8 +937,9 @@ __device__ inline bool grid_barrier(unsigned* bar, unsigned target, unsigned max
   return *s_ok != 0;
 }
 
-__device__ inline void grid_exit(unsigned* bar) {
-  if (threadIdx.x == 0 && atomicAdd(&bar[1], 1u) == gridDim.x - 1) {
+// G: the CTAs that share the words
+__device__ inline void grid_exit(unsigned* bar, unsigned G) {
+  if (threadIdx.x == 0 && atomicAdd(&bar[1], 1u) == G - 1) {
     atomicExch(&bar[0], 0u);
     atomicExch(&bar[1], 0u);
   }

@@ -994,7 +994,7 @@ __global__ void __launch_bounds__(256, MINB) k_pipe_tail(const RunDesc* __restri
     if (!grid_barrier(bar, ++ep * G, maxp, &dyn[0].err, &s_ok)) return;
     if (rec) ts[3] = global_ns();
   }
-  grid_exit(bar);
+  grid_exit(bar, G);
 }
 
 #define BD_TAIL_SHAPES(X) X(2) X(3) X(4)

@@ -117,10 +117,11 @@ int launch_sort(const RunDesc* runs, RunDyn* dyn, int run0, int nruns, const Ite
 constexpr int FUSED_PHASES = 4;
 // Resident step (bd_resident.cuh): A.nsteps steps (at most each run's step
 // budget) of one run (SINGLE) or of every run of A.items in one launch.
-__host__ __device__ constexpr int res_threads(bool single) { return single ? 1024 : 512; }
-constexpr size_t res_max_smem(bool single) { return (single ? 200 : 112) * 1024; }  // one or two CTAs per SM
-constexpr int res_pcap(bool single) { return single ? 2048 : 1536; }  // particles of a CTA kept in shared memory
-__host__ __device__ constexpr int res_side(int lz) { return lz >= 16 ? 3 << (lz - 16) : lz ? 1 << lz : 0; }
+enum ResKind { RES_CLUSTERS = 0, RES_SINGLE = 1, RES_GROUPS = 2 };
+__host__ __device__ constexpr int res_threads(int kind) { return kind == RES_CLUSTERS ? 512 : 1024; }
+constexpr size_t res_max_smem(int kind) { return (kind == RES_CLUSTERS ? 112 : 200) * 1024; }  // two CTAs per SM, or one
+constexpr int res_pcap(int kind) { return kind == RES_CLUSTERS ? 1536 : 2048; }  // particles of a CTA kept in shared memory
+__host__ __device__ constexpr int res_side(int lz) { return lz >= 16 ? 3 << (lz - 16) : lz > 0 ? 1 << lz : 0; }
 constexpr size_t RES_DESC_BYTES = 1024;   // the run's description
 __host__ __device__ constexpr size_t RES_TW_BYTES(int Z) {  // twiddles and sine tables
   return ((size_t)8 * Z + 4 * (Z + Z / 2 + 1) + 255) & ~(size_t)255;
@@ -130,7 +131,7 @@ struct ResArgs {
   Item one_item;           // its item: run 0, a/b/c = log2 rows forward, columns, rows inverse per item
   const RunDesc* runs;     // run table (descriptions with dacc set)
   RunDyn* dyn;
-  const Item* items;       // one per cluster: run, item sizes as above
+  const Item* items;       // one per cluster: run, item sizes as above; groups: two per CTA (k_resident)
   int nsteps;
   int part_off, pcap;      // the particles' place in shared memory and their number
   int grid_mode;           // single run: the whole cooperative grid instead of one cluster
@@ -143,12 +144,13 @@ struct ResArgs {
   int skip_barrier, skip_cta;
   unsigned long long* ts;  // single run: FUSED_PHASES + 1 timestamps of one step (may be null)
 };
+// kind: one run, one cluster per run, or groups of CTAs of one cooperative grid.
 // lz: the mesh side: 2^lz (3..10), 3 * 2^(lz - 16) (20..24: 48 to 768), 0:
-// other meshes with a factor 3 and ideal-gas runs. cs: CTAs per cluster, 0: cooperative grid (single run).
+// other meshes with a factor 3 and ideal-gas runs, -1: any (groups). cs: CTAs per cluster, 0: cooperative grid (single run).
 // resident_configure: attributes for smem bytes of dynamic shared memory;
 // *n: resident CTAs (cs 0) or clusters the device can hold at once
-int resident_configure(int lz, bool single, size_t smem, int cs, int device, int* n);
-int launch_resident(int lz, bool single, const ResArgs& A, int nclusters, int cs, int grid, size_t smem,
+int resident_configure(int lz, int kind, size_t smem, int cs, int device, int* n);
+int launch_resident(int lz, int kind, const ResArgs& A, int nclusters, int cs, int grid, size_t smem,
                     cudaStream_t s);
 // TimestepInfo reductions of run 0 into acc (diag_bytes() of device memory):
 // energy, virial (double), largest |F|^2 << 32 | index of WCA, capillary,

@@ -3,24 +3,25 @@
 
 namespace bd {
 
-template <int LZ, bool SINGLE>
+template <int LZ, int KIND>
 int resident_configure_t(size_t smem, int cs, int nsm, int* grid);
-template <int LZ, bool SINGLE>
+template <int LZ, int KIND>
 int launch_resident_t(const ResArgs& A, int nclusters, int cs, int grid, size_t smem, cudaStream_t s);
 
 #define BD_RES_SIZES(X) \
   X(0) X(3) X(4) X(5) X(6) X(7) X(8) X(9) X(10) X(20) X(21) X(22) X(23) X(24)
 
-int resident_configure(int lz, bool single, size_t smem, int cs, int device, int* n) {
+int resident_configure(int lz, int kind, size_t smem, int cs, int device, int* n) {
   *n = 0;
   int nsm = 0;
   cudaError_t e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, device);
   if (e != cudaSuccess) return (int)e;
+  if (kind == RES_GROUPS) return resident_configure_t<-1, RES_GROUPS>(smem, 0, nsm, n);
   switch (lz) {
 #define BD_CASE(L)                                                       \
   case L:                                                                \
-    return single ? resident_configure_t<L, true>(smem, cs, nsm, n)      \
-                  : resident_configure_t<L, false>(smem, cs, nsm, n);
+    return kind == RES_SINGLE ? resident_configure_t<L, RES_SINGLE>(smem, cs, nsm, n)      \
+                              : resident_configure_t<L, RES_CLUSTERS>(smem, cs, nsm, n);
     BD_RES_SIZES(BD_CASE)
 #undef BD_CASE
     default:
@@ -28,13 +29,14 @@ int resident_configure(int lz, bool single, size_t smem, int cs, int device, int
   }
 }
 
-int launch_resident(int lz, bool single, const ResArgs& A, int nclusters, int cs, int grid, size_t smem,
+int launch_resident(int lz, int kind, const ResArgs& A, int nclusters, int cs, int grid, size_t smem,
                     cudaStream_t s) {
+  if (kind == RES_GROUPS) return launch_resident_t<-1, RES_GROUPS>(A, 0, 0, grid, smem, s);
   switch (lz) {
 #define BD_CASE(L)                                                             \
   case L:                                                                      \
-    return single ? launch_resident_t<L, true>(A, nclusters, cs, grid, smem, s) \
-                  : launch_resident_t<L, false>(A, nclusters, cs, grid, smem, s);
+    return kind == RES_SINGLE ? launch_resident_t<L, RES_SINGLE>(A, nclusters, cs, grid, smem, s) \
+                              : launch_resident_t<L, RES_CLUSTERS>(A, nclusters, cs, grid, smem, s);
     BD_RES_SIZES(BD_CASE)
 #undef BD_CASE
     default:

@@ -816,20 +816,59 @@ __device__ __noinline__ void res_place(RunDyn* D, int b, int g0, int g1, int nc,
   }
 }
 
-// LZ: the mesh side as res_side gives it, or 0: the other meshes with a factor
-// 3 and ideal-gas runs.
-// SINGLE: one run, described by the kernel parameter, 1024 threads per CTA
-// and one CTA per SM; else one cluster per entry of A.items, 512 threads and
-// two CTAs per SM.
-template <int LZ, bool SINGLE>
-__global__ void __launch_bounds__(SINGLE ? 1024 : 512, SINGLE ? 1 : 2) k_resident(const __grid_constant__ ResArgs A) {
-  constexpr int NT = SINGLE ? 512 : 256;
+// The transform phases with the mesh class known at run time (RES_GROUPS).
+#define BD_RES_SIZES(X) \
+  X(0) X(3) X(4) X(5) X(6) X(7) X(8) X(9) X(10) X(20) X(21) X(22) X(23) X(24)
+template <int LZ, int NT>
+__device__ __forceinline__ void res_inv_of(int lz, int b, int G, int lri, bool alias) {
+  if constexpr (LZ >= 0) res_inv<LZ, NT>(b, G, lri, alias);
+  else switch (lz) {
+#define BD_CASE(L) case L: res_inv<L, NT>(b, G, lri, alias); break;
+    BD_RES_SIZES(BD_CASE)
+#undef BD_CASE
+  }
+}
+template <int LZ, int NT>
+__device__ __forceinline__ void res_fwd_of(int lz, int b, int G, int lrf, bool alias) {
+  if constexpr (LZ >= 0) res_fwd<LZ, NT>(b, G, lrf, alias);
+  else switch (lz) {
+#define BD_CASE(L) case L: res_fwd<L, NT>(b, G, lrf, alias); break;
+    BD_RES_SIZES(BD_CASE)
+#undef BD_CASE
+  }
+}
+template <int LZ, int NT>
+__device__ __forceinline__ void res_cols_of(int lz, int b, int G, int lw) {
+  if constexpr (LZ >= 0) res_cols<LZ, NT>(b, G, lw);
+  else switch (lz) {
+#define BD_CASE(L) case L: res_cols<L, NT>(b, G, lw); break;
+    BD_RES_SIZES(BD_CASE)
+#undef BD_CASE
+  }
+}
+
+// LZ: the mesh side as res_side gives it; 0: the other meshes with a factor 3
+// and ideal-gas runs; -1 (RES_GROUPS): any, named by the items.
+// KIND: RES_SINGLE: one run, described by the kernel parameter, on one cluster
+// or on the whole cooperative grid, 1024 threads per CTA and one CTA per SM.
+// RES_CLUSTERS: one cluster per entry of A.items, 512 threads and two CTAs per
+// SM. RES_GROUPS: a cooperative grid shared out among the runs, a group of
+// CTAs of any size for each with barrier words of its own: CTA k's items
+// A.items[2k] (run, item sizes) and A.items[2k + 1] (mesh class, group, rank
+// in it, its CTAs); for few runs of uneven weight, which clusters of at most
+// 16 CTAs leave to the heaviest.
+template <int LZ, int KIND>
+__global__ void __launch_bounds__(res_threads(KIND), KIND == RES_CLUSTERS ? 2 : 1) k_resident(const __grid_constant__ ResArgs A) {
+  constexpr int NT = res_threads(KIND) / 2;
+  constexpr bool SINGLE = KIND == RES_SINGLE, GROUPS = KIND == RES_GROUPS;
   __shared__ int s_tmp[32];
   __shared__ int s_ok;
-  const bool grid = SINGLE && A.grid_mode;
-  const int G = grid ? (int)gridDim.x : (int)cluster_size();
-  const int b = grid ? (int)blockIdx.x : (int)cluster_rank();
-  const Item I = SINGLE ? A.one_item : A.items[blockIdx.x / (unsigned)G];
+  const bool grid = GROUPS || (SINGLE && A.grid_mode);
+  const Item J = GROUPS ? A.items[2 * blockIdx.x + 1] : Item{LZ, 0, 0, 0};
+  const int G = GROUPS ? J.c : grid ? (int)gridDim.x : (int)cluster_size();
+  const int b = GROUPS ? J.b : grid ? (int)blockIdx.x : (int)cluster_rank();
+  const Item I = SINGLE ? A.one_item : GROUPS ? A.items[2 * blockIdx.x] : A.items[blockIdx.x / (unsigned)G];
+  unsigned* bar = GROUPS ? A.bar + 2 * J.a : A.bar;
   {
     static_assert(sizeof(RunDesc) % 4 == 0 && sizeof(RunDesc) <= RES_DESC_BYTES, "copied by words");
     const int* src = SINGLE ? reinterpret_cast<const int*>(&A.one) : reinterpret_cast<const int*>(&A.runs[I.run]);
@@ -839,7 +878,7 @@ __global__ void __launch_bounds__(SINGLE ? 1024 : 512, SINGLE ? 1 : 2) k_residen
   const RunDesc& R = res_desc();
   RunDyn* D = A.dyn + I.run;
   const int Z = res_side(LZ) ? res_side(LZ) : R.Z, n = Z >> 1;
-  const bool mesh = LZ || !(R.flags & F_IDGAS);
+  const bool mesh = LZ > 0 || !(R.flags & F_IDGAS);
   // the accumulator shares spec2's memory: its clearing moves to the inverse rows
   const bool alias = (const void*)R.dacc == (const void*)R.spec2;
   const bool adaptive = (R.flags & F_ADAPTIVE) != 0;
@@ -880,7 +919,7 @@ __global__ void __launch_bounds__(SINGLE ? 1024 : 512, SINGLE ? 1 : 2) k_residen
       return true;
     }
     if (A.skip_barrier == (int)ep + 1 && b == A.skip_cta) return false;
-    return grid_barrier(A.bar, ++ep * (unsigned)G, maxp, &D->err, &s_ok);
+    return grid_barrier(bar, ++ep * (unsigned)G, maxp, &D->err, &s_ok);
   };
   const bool rec = SINGLE && A.ts && b == 0 && threadIdx.x == 0;
   int ph = 0;
@@ -892,7 +931,7 @@ __global__ void __launch_bounds__(SINGLE ? 1024 : 512, SINGLE ? 1 : 2) k_residen
 #pragma unroll 1
   for (int k = 0; k < nst; k++, step++) {
     if (!lower) res_pairs<NT>(step, g0, nc, k > 0 ? noise : nullptr, A.part_off, A.pcap);
-    else if (mesh) res_inv<LZ, NT>(b, G, I.c, alias);
+    else if (mesh) res_inv_of<LZ, NT>(J.run, b, G, I.c, alias);
     BD_BARRIER();
     if (!adaptive) {
       // a few particles: several lanes for each
@@ -906,30 +945,30 @@ __global__ void __launch_bounds__(SINGLE ? 1024 : 512, SINGLE ? 1 : 2) k_residen
     }
     BD_BARRIER();
     if (!lower) res_scan_phase<NT>(b, G, nch, s_tmp);
-    else if (mesh) res_fwd<LZ, NT>(b, G, I.a, alias);
+    else if (mesh) res_fwd_of<LZ, NT>(J.run, b, G, I.a, alias);
     BD_BARRIER();
     if (!lower) res_place<NT>(D, b, g0, g1, nc, nch, adaptive, k + 1 < nst ? noise : nullptr, step + 1, A.part_off, A.pcap);
-    else if (mesh) res_cols<LZ, NT>(b, G, I.b);
+    else if (mesh) res_cols_of<LZ, NT>(J.run, b, G, I.b);
     if (k + 1 < nst || (SINGLE && A.ts)) {
       BD_BARRIER();
     }
   }
 #undef BD_BARRIER
-  if (grid) grid_exit(A.bar);
+  if (grid) grid_exit(bar, (unsigned)G);
 }
 
 // sets the kernel's attributes for `smem` bytes; grid mode: fills *grid with
 // the CTAs that can be resident; cluster mode: *grid > 0 when clusters of
 // `cs` CTAs can be scheduled. Returns 0 or a cudaError_t.
-template <int LZ, bool SINGLE>
+template <int LZ, int KIND>
 int resident_configure_t(size_t smem, int cs, int nsm, int* grid) {
-  auto* f = k_resident<LZ, SINGLE>;
-  if (smem > res_max_smem(SINGLE)) return (int)cudaErrorInvalidValue;
-  cudaError_t e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)res_max_smem(SINGLE));
+  auto* f = k_resident<LZ, KIND>;
+  if (smem > res_max_smem(KIND)) return (int)cudaErrorInvalidValue;
+  cudaError_t e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)res_max_smem(KIND));
   if (e != cudaSuccess) return (int)e;
   if (cs == 0) {
     int per = 0;
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, f, res_threads(SINGLE), smem);
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, f, res_threads(KIND), smem);
     *grid = per * nsm;
     return (int)e;
   }
@@ -937,7 +976,7 @@ int resident_configure_t(size_t smem, int cs, int nsm, int* grid) {
   if (e != cudaSuccess) return (int)e;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(cs);
-  cfg.blockDim = dim3(res_threads(SINGLE));
+  cfg.blockDim = dim3(res_threads(KIND));
   cfg.dynamicSmemBytes = smem;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -948,11 +987,11 @@ int resident_configure_t(size_t smem, int cs, int nsm, int* grid) {
   return (int)cudaOccupancyMaxActiveClusters(grid, f, &cfg);
 }
 
-template <int LZ, bool SINGLE>
+template <int LZ, int KIND>
 int launch_resident_t(const ResArgs& A, int nclusters, int cs, int grid, size_t smem, cudaStream_t s) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(cs ? nclusters * cs : grid);
-  cfg.blockDim = dim3(res_threads(SINGLE));
+  cfg.blockDim = dim3(res_threads(KIND));
   cfg.dynamicSmemBytes = smem;
   cfg.stream = s;
   cudaLaunchAttribute attr[1];
@@ -966,13 +1005,14 @@ int launch_resident_t(const ResArgs& A, int nclusters, int cs, int grid, size_t 
   }
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  return (int)cudaLaunchKernelEx(&cfg, k_resident<LZ, SINGLE>, A);
+  return (int)cudaLaunchKernelEx(&cfg, k_resident<LZ, KIND>, A);
 }
 
-#define BD_RES_INSTANTIATE(L)                                                                              \
-  template int resident_configure_t<L, false>(size_t, int, int, int*);                                     \
-  template int resident_configure_t<L, true>(size_t, int, int, int*);                                      \
-  template int launch_resident_t<L, false>(const ResArgs&, int, int, int, size_t, cudaStream_t);           \
-  template int launch_resident_t<L, true>(const ResArgs&, int, int, int, size_t, cudaStream_t);
+#define BD_RES_INSTANTIATE_KIND(L, K)                           \
+  template int resident_configure_t<L, K>(size_t, int, int, int*); \
+  template int launch_resident_t<L, K>(const ResArgs&, int, int, int, size_t, cudaStream_t);
+#define BD_RES_INSTANTIATE(L)            \
+  BD_RES_INSTANTIATE_KIND(L, RES_CLUSTERS) \
+  BD_RES_INSTANTIATE_KIND(L, RES_SINGLE)
 
 }  // namespace bd

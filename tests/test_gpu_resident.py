@@ -157,3 +157,32 @@ def test_large_mesh_pipelined_equals_stage_kernels(gpu, mesh):
     for s in (0, 1):  # FP32 transforms of 2^22 points and more: 1e-5 as the parity tests
         d = np.linalg.norm(fa[("kap", s)] - fo[("kap", s)]) / np.linalg.norm(fo[("kap", s)])
         assert d <= 1e-5
+
+
+def test_groups_uneven_batch_equals_stage_kernels(gpu):
+    """Few runs of very uneven weight: groups of CTAs of one cooperative grid,
+    the smallest run on one CTA, the largest on most of them, with step
+    budgets of their own through the server."""
+    sizes = [(60, 41, 16), (3000, 2501, 384), (500, 400, 64), (9000, 8000, 256)]
+    runs = [_params(gpu, n1, n2, m, k != 3, scheme=2) for k, (n1, n2, m) in enumerate(sizes)]
+    a, b = gpu.Batch(runs, [3, 4, 5, 6]), gpu.Batch(runs, [3, 4, 5, 6])
+    for x in (a, b):
+        for k, p in enumerate(runs):
+            x.set_positions(k, _lattice(p, 70 + k))
+    a.step(13)
+    a.step(7)
+    b.stage_times(20)
+    for k in range(len(runs)):
+        _same(a.get_positions(k), b.get_positions(k))
+        assert a.time(k) == b.time(k)
+    runs = [dict(p, max_reisedistanz=1e30) for p in runs]  # the server steps with a fixed dt
+    srv = gpu.Server(steps_per_tick=9)
+    ids = [srv.submit(p, 90 + k, 5 + 11 * k) for k, p in enumerate(runs)]
+    for _ in range(1000):
+        srv.tick()
+        if all(srv.poll(i).state >= 2 for i in ids):
+            break
+    for k, p in enumerate(runs):
+        r = gpu.Run(p, seed=90 + k)
+        r.stage_times(5 + 11 * k)
+        _same(srv.result(ids[k]), r.get_positions())
