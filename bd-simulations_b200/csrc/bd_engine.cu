@@ -428,6 +428,16 @@ static bool resident_run(const RunHost& r) {
   return pow2(r.Z) ? r.Z >= 8 && r.Z <= 1024 : r.Z <= 648 || r.Z == 768;
 }
 
+// A single run that steps pipelined when asked for several steps (on a mesh
+// beyond the resident step's, always). Measured, us per step, 128 steps a call
+// (resident | pipelined | a launch per step), particles, mesh side:
+// 131 072, 256 27.5 | 29.3 | 31.0; 131 072, 512 32.5 | 31.6 | 35.4; 262 144, 512
+// 45.1 | 41.0 | 51.4; 524 288, 512 64.2 | 57.4 | 71.9; 131 072, 1024 60.5 | 49.3 |
+// 51.6; 262 144, 1024 72.9 | 59.9 | 64.1; 900 000, 1024 122 | 105 | 116
+static bool pipelined_single(const RunHost& r) {
+  return r.Z > 1024 || (r.N >= 131072 && r.Z >= 512) || r.N >= 262144;
+}
+
 static int resident_lz(const RunHost& r) {
   if (r.idgas) return 0;
   if (pow2(r.Z)) return ilog2(r.Z);
@@ -678,6 +688,11 @@ int Engine::plan_resident() {
   rone.pcap = res_pcap(RES_SINGLE);
   resident = true;
   fused = r.d.dacc != nullptr;
+  one_step = OneStepPlan{};
+  if (fused && one_step_plan(one_step, r.Z, r.N, r.C, device)) {
+    cudaGetLastError();
+    one_step = OneStepPlan{};
+  }
   return BD_OK;
 }
 
@@ -692,6 +707,8 @@ RunDesc Engine::table_desc(size_t k) const {
 // nsteps steps of the only run in one launch; fault: with the pending
 // recovery-path test (grid mode); ts: phase timestamps of one step.
 int Engine::launch_one(int nsteps, bool fault, unsigned long long* ts) {
+  if (nsteps == 1 && !fault && one_step.grid > 0)
+    return launch_one_step(rone.one, d_dyn, one_step, d_bar, stream, ts) ? BD_ERR_CUDA : BD_OK;
   ResArgs A = rone;
   A.nsteps = nsteps;
   A.ts = ts;
@@ -716,8 +733,12 @@ int Engine::step_resident(long long nsteps) {
       RK(launch_one(1, true, nullptr));
       nsteps--;
     }
+    // 1024^2: four elements per thread of half the CTAs' threads are short of
+    // the transforms' work, the launches cost less (65 536 particles, us per
+    // step: 55.6 resident, 43.9 a launch each)
+    const bool each = one_step.grid > 0 && (piped || runs[0]->Z == 1024);
     while (nsteps > 0) {
-      const int k = (int)std::min<long long>(nsteps, res_chunk);
+      const int k = each ? 1 : (int)std::min<long long>(nsteps, res_chunk);
       RK(launch_one(k, false, nullptr));
       nsteps -= k;
     }
@@ -858,7 +879,7 @@ int Engine::build_plan() {
   // take as many sequences per item as FFT2_THREADS threads transform at
   // once (Z/16 threads per length-Z sequence).
   const size_t nr = runs.size();
-  bool pipe_runs = nr >= 2 || (nr == 1 && runs[0]->Z > 1024);
+  bool pipe_runs = nr >= 2 || (nr == 1 && pipelined_single(*runs[0]));
   for (auto* r : runs) pipe_runs = pipe_runs && r->d.dacc != nullptr;
   std::vector<int> lrf(nr), lri(nr), lw(nr);
   for (size_t k = 0; k < nr; k++) {
@@ -975,8 +996,8 @@ int Engine::build_plan() {
   // 2048^2 247 | 351; the 256-run ensemble (24 000 on average) 562 | 537
   part_large = n_part >= (int)nr * 512 ? 1 : 0;
   // pipelined stage step: several runs, every one depositing in the move, or
-  // one on a mesh beyond the resident step's (1024^2): 2.1 M particles on
-  // 2048^2, 335 us per step with the stage kernels, 252 pipelined
+  // one large run (pipelined_single): 2.1 M particles on 2048^2, 335 us per step
+  // with the stage kernels, 252 pipelined
   piped = pipe_runs;
   if (piped) {
     std::vector<Item> pl[3];
@@ -1125,7 +1146,7 @@ int Engine::set_step_form(int form, int ctas) {
 // (the six-launch form runs instead).
 int Engine::plan_tail() {
   tail_ok = false;
-  if (!piped || pipe_form != PIPE_TWO) return BD_OK;
+  if (!piped || fused || pipe_form != PIPE_TWO) return BD_OK;
   for (auto* r : runs)
     if (r->Z > 1024) return BD_OK;  // the tail's transforms are compiled up to 1024 points
   PipeTail P{};
@@ -1408,7 +1429,7 @@ int Engine::fused_phase_times(int nsteps, double* ms, int nphases) {
     if (!r->has_pos) return BD_ERR_STATE;
   CK(cudaSetDevice(device));
   if (!planned) RK(build_plan());
-  if (piped) return pipe_phase_times(nsteps, ms, nphases);
+  if (piped && !fused) return pipe_phase_times(nsteps, ms, nphases);
   if (!fused) return BD_ERR_STATE;
   RK(fused_prologue(false));
   unsigned long long* d_ts = nullptr;
@@ -1715,8 +1736,11 @@ int Engine::step(long long nsteps) {
   if (!planned) RK(build_plan());
   if (runs.empty()) return BD_OK;
   if (nsteps == 0) return BD_OK;
-  // several runs: a call of one step takes the launch-per-step form
-  if (resident && (runs.size() == 1 || (nsteps > 1 && !(piped && pipe_form == PIPE_TWO)))) {
+  // several runs: a call of one step takes the launch-per-step form; one run
+  // that has the pipelined form too: from 8 steps on, which pay for the force
+  // grids it starts from
+  const bool single = runs.size() == 1 && !(piped && nsteps >= 8 && fault_barrier == 0);
+  if (resident && (single || (runs.size() > 1 && nsteps > 1 && !(piped && pipe_form == PIPE_TWO)))) {
     RK(fused_prologue(false));
     grids_valid = false;
     return step_resident(nsteps);

@@ -216,6 +216,7 @@ class Engine {
   ResArgs rone{};
   Item rone_cluster{}, rone_grid{};  // item sizes of the two modes
   int rone_lz = 0, res_cs = 0, res_grid = 0;
+  OneStepPlan one_step{};  // a call of one step of the only run (grid 0: the resident kernel)
   size_t rone_smem = 0;
   int res_share_grid = 0, off_share = 0;
   size_t res_share_smem = 0;
@@ -225,8 +226,9 @@ class Engine {
   int launch_one(int nsteps, bool fault, unsigned long long* ts);
   int step_resident(long long nsteps);
   RunDesc table_desc(size_t k) const;
-  // one run on a power-of-two mesh with a fixed dt, resident (the fused step
-  // of the API: bd_fused_phase_times, bd_inject_barrier_timeout)
+  // one run on a power-of-two mesh with a fixed dt, a step per launch or
+  // resident (the fused step of the API: bd_fused_phase_times,
+  // bd_inject_barrier_timeout)
   bool fused = false;
   unsigned* d_bar = nullptr;  // barrier words, two per group of CTAs (BAR_GROUPS of them)
   static constexpr int BAR_GROUPS = 256;

@@ -111,7 +111,7 @@ int launch_records_by_pid(const Rec* src, Rec* dst, int n, cudaStream_t s);
 int launch_sort(const RunDesc* runs, RunDyn* dyn, int run0, int nruns, const Item* chunks, int nchunks,
                 const Item* parts, int nparts, int end_step_flag, int adaptive, int require_active, cudaStream_t s,
                 cudaEvent_t* ev = nullptr);
-// phases of one step whose ends a single run's resident launch can time:
+// phases of one step whose ends a single run's launch of one step can time:
 // [0] inverse row FFT [1] particles (forces, noise, move, next density)
 // [2] cell-count scan + next row FFT [3] scatter + next column FFT + Green
 constexpr int FUSED_PHASES = 4;
@@ -152,6 +152,22 @@ struct ResArgs {
 int resident_configure(int lz, int kind, size_t smem, int cs, int device, int* n);
 int launch_resident(int lz, int kind, const ResArgs& A, int nclusters, int cs, int grid, size_t smem,
                     cudaStream_t s);
+// One step of one run on a power-of-two mesh up to 1024^2 with a fixed dt in
+// one launch of its own (bd_onestep.cu); run: its description, dacc set. bar:
+// two barrier words, zero before and after each launch. Starts and ends with
+// the resident step's state.
+struct OneStepPlan {
+  int lz;
+  int lrf, nrf;  // forward row items: 2^lrf rows, nrf items
+  int lw, ncl;   // column items
+  int lri, nri;  // inverse row items
+  int nch;       // scan chunks
+  size_t smem;   // dynamic shared memory
+  int grid;      // CTAs (all resident: cooperative launch); 0: no plan
+};
+int one_step_plan(OneStepPlan& P, int Z, int N, int C, int device);
+int launch_one_step(const RunDesc& run, RunDyn* dyn, const OneStepPlan& P, unsigned* bar, cudaStream_t s,
+                    unsigned long long* ts);
 // TimestepInfo reductions of run 0 into acc (diag_bytes() of device memory):
 // energy, virial (double), largest |F|^2 << 32 | index of WCA, capillary,
 // noise forces (uint64 x 3), examined WCA pairs (uint64)

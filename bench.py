@@ -261,8 +261,8 @@ def flusher(local):
 
 
 def timed_steps_flushed(run, K, local, buf):
-    """K fused steps (one graph launch each), the L2 flushed before every
-    step, CUDA events around each step on the library's stream."""
+    """K steps, one call each, the L2 flushed before every step, CUDA events
+    around each step on the library's stream."""
     import torch
     stream = torch.cuda.ExternalStream(run.stream(), device="cuda:%d" % local)
     evs = [(torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)) for _ in range(K)]
@@ -280,8 +280,8 @@ def timed_steps_flushed(run, K, local, buf):
 
 
 def fused_profile(run, K, local, buf):
-    """Phase times of the fused step (ms per step), L2 flushed before each
-    step; None when the run steps with the stage kernels."""
+    """Phase times of one-step calls (ms per step; pipelined: of its steps), L2 flushed
+    before each step; None when the run steps with the stage kernels."""
     import torch
     stream = torch.cuda.ExternalStream(run.stream(), device="cuda:%d" % local)
     acc = None
@@ -345,12 +345,12 @@ def gpu_arm(args):
     t_dev = dist_max(t_dev, ws)
     value = ws * N * K / t_dev
     launches = run.launches_per_step() * K
-    # roofline. Fused step: the one kernel is the whole step (its launch
+    # roofline. A call of one step: the one kernel is the whole step (its launch
     # time is the event-timed step), its phases from device timestamps.
     # Stage kernels: the dominant stage, algorithmic bytes / its event time.
     phases = fused_profile(run, min(K, 200), local, buf)
     if phases is not None:
-        dom = "k_fused (whole step in one cooperative launch)"
+        dom = "k_one_step (whole step in one cooperative launch)"
         achieved = step_bytes(p) / (t_dev / K) / 1e9
         stages = None
     else:

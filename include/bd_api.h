@@ -414,8 +414,8 @@ int bd_batch_autotune(bd_batch* b, int reps, bd_tune_result* out);
  * is larger than 1024^2). BD_ERR_ARG for other values. */
 int bd_batch_set_step_form(bd_batch* b, int form, int ctas_per_sm);
 /* one run on a power-of-two mesh up to 1024^2 with a fixed dt steps in one
- * cooperative launch (the fused step: the resident kernel, many steps per
- * launch when asked for them); bd_launches_per_step then reports 1 and
+ * cooperative launch (the fused step; calls of several steps: many steps per
+ * launch, or for large runs the pipelined step below); bd_launches_per_step then reports 1 and
  * bd_stage_times times the stage kernels instead. Runs on
  * power-of-two meshes with a fixed dt otherwise (a batch of two or more of
  * them, one on a larger mesh) step in six launches per step (the pipelined stage step;

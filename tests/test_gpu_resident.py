@@ -186,3 +186,52 @@ def test_groups_uneven_batch_equals_stage_kernels(gpu):
         r = gpu.Run(p, seed=90 + k)
         r.stage_times(5 + 11 * k)
         _same(srv.result(ids[k]), r.get_positions())
+
+
+def test_resident_adaptive_beyond_shared_particles(gpu):
+    p = _params(gpu, 170000, 150001, 96, True, rho=0.25)
+    start = _lattice(p, 6)
+    a, b = gpu.Run(p, seed=3), gpu.Run(p, seed=3)
+    for r in (a, b):
+        r.set_positions_all(start)
+    a.zeitschritte(4)
+    b.stage_times(4)
+    _same(a.get_positions(), b.get_positions())
+
+
+# smallest and largest mesh, meshes whose column items hold one and several
+# columns, one and two CTAs per SM (256 particles per CTA on 148 SMs), and
+# more than 512 scan chunks (a C of 1024 and more)
+@pytest.mark.parametrize("n1,n2,mesh", [(40, 17, 8), (300, 201, 32), (1500, 1501, 128), (18900, 18988, 256),
+                                        (18900, 18989, 512), (20000, 19999, 1024), (180001, 130000, 256)])
+def test_one_step_calls_equal_stage_kernels(gpu, n1, n2, mesh):
+    p = _params(gpu, n1, n2, mesh, False, scheme=(n1 + mesh) % 3, rho=0.2 if n1 < 100000 else 0.18)
+    start = _lattice(p, 15)
+    a, b = gpu.Run(p, seed=22), gpu.Run(p, seed=22)
+    for r in (a, b):
+        r.set_positions_all(start)
+    for _ in range(4):
+        a.zeitschritt()
+    a.zeitschritte(3)
+    a.zeitschritt()
+    b.stage_times(8)
+    _same(a.get_positions(), b.get_positions())
+    assert a.time() == b.time() and a.step_count() == b.step_count()
+
+
+@pytest.mark.parametrize("n1,n2,mesh", [(65536, 65535, 512), (65536, 65536, 512), (65536, 65536, 1024),
+                                        (131072, 131072, 64)])
+def test_large_single_run_forms_in_turn(gpu, n1, n2, mesh):
+    """Either side of the size from which calls of several steps take the
+    pipelined step; single steps, short and long calls after one another."""
+    p = _params(gpu, n1, n2, mesh, False, rho=0.25)
+    start = _lattice(p, 16)
+    a, b = gpu.Run(p, seed=23), gpu.Run(p, seed=23)
+    for r in (a, b):
+        r.set_positions_all(start)
+    for n in (20, 1, 7, 8, 1, 3):
+        a.zeitschritte(n)
+    b.stage_times(40)
+    _same(a.get_positions(), b.get_positions())
+    assert a.launches_per_step() == 1
+    assert a.time() == b.time() and a.step_count() == b.step_count()
