@@ -30,14 +30,21 @@ struct FftPlan {
 // with a named barrier of its own, so that the two halves of a resident CTA
 // work on different things between group barriers. tid: index in the team.
 struct CtaTeam {
+  static constexpr bool ONCE = false;  // no loop around the transforms
   int tid;
   __device__ __forceinline__ CtaTeam() : tid((int)threadIdx.x) {}
   __device__ __forceinline__ int nt() const { return (int)blockDim.x; }
   __device__ __forceinline__ void sync() const { __syncthreads(); }
 };
+// the CTA where no transform is in a loop: the values of idle threads need not
+// be set (one-step launch after an L2 flush, 65 536 particles 32.2 -> 31.5 us)
+struct OnceTeam : CtaTeam {
+  static constexpr bool ONCE = true;
+};
 // half ID (0: the lower threads) of a CTA of 2*NT threads, NT a power of two
 template <int ID, int NT>
 struct HalfTeam {
+  static constexpr bool ONCE = false;
   int tid;
   __device__ __forceinline__ HalfTeam() {
     // the index is opaque to the compiler: an item loop around a transform

@@ -141,8 +141,10 @@ __device__ __forceinline__ void fft2_pass(const Team& T, float2* s, int ss, int 
   float2 v[E];
   // set before the branch: left undefined on the idle threads' path, v is kept
   // in local memory across the barrier wherever a loop surrounds the pass
+  if constexpr (!Team::ONCE) {
 #pragma unroll
-  for (int t = 0; t < E; t++) v[t] = make_float2(0.f, 0.f);
+    for (int t = 0; t < E; t++) v[t] = make_float2(0.f, 0.f);
+  }
   if (act) {
 #pragma unroll
     for (int u = 0; u < NB; u++)

@@ -11,9 +11,9 @@
 // code (fetched from memory again when other work has used the L2). What
 // bounds it is the chain of launch, four phases and three grid barriers.
 // Measured, us per call of one step, L2 flushed before it (resident kernel |
-// this one): 2000 particles, 128^2 34.0 | 26.1; 16 384, 256^2 34.8 | 28.6; 65 536,
-// 512^2 42.4 | 32.3; 262 144, 1024^2 97.8 | 76.0; not flushed 23.2 | 25.3, 29.0 |
-// 27.6, 37.4 | 31.3, 86.0 | 67.9: every size takes this kernel.
+// this one): 2000 particles, 128^2 34.0 | 25.4; 16 384, 256^2 34.8 | 28.6; 65 536,
+// 512^2 42.4 | 31.5; 262 144, 1024^2 97.8 | 76.0; not flushed 23.2 | 25.2, 29.0 |
+// 27.6, 37.4 | 31.2, 86.0 | 67.9: every size takes this kernel.
 #include <algorithm>
 
 #include "bd_items.cuh"
@@ -75,7 +75,7 @@ __global__ void __launch_bounds__(256, 2) k_one_step(const __grid_constant__ Run
   if (rec) ts[++ph] = global_ns()
   // A transform item runs at most once per call site and CTA (the host sizes
   // them so): in a loop the compiler keeps the addresses of all its passes.
-  if (b < P.nri) fft2_rows_inv_item<LZ, true>(CtaTeam(), R, b << P.lri, P.lri, work, tws);
+  if (b < P.nri) fft2_rows_inv_item<LZ, true>(OnceTeam(), R, b << P.lri, P.lri, work, tws);
   BD_BARRIER();
   if (steps_left <= 0) {  // the same for every CTA
     grid_exit(bar, (unsigned)G);
@@ -133,13 +133,13 @@ __global__ void __launch_bounds__(256, 2) k_one_step(const __grid_constant__ Run
   }
   {
     const int it = G - 1 - b;
-    if (it < P.nrf) fft2_rows_fwd_item<LZ, true, true>(CtaTeam(), R, it << P.lrf, P.lrf, work, tws);
+    if (it < P.nrf) fft2_rows_fwd_item<LZ, true, true>(OnceTeam(), R, it << P.lrf, P.lrf, work, tws);
   }
   BD_BARRIER();
   for (int gi = g0 + threadIdx.x; gi < g1; gi += blockDim.x) scatter_particle(R, gi);
   {
     const int it = G - 1 - b;
-    if (it < P.ncl) fft2_cols_item<LZ, true>(CtaTeam(), R, it << P.lw, P.lw, work, tws);
+    if (it < P.ncl) fft2_cols_item<LZ, true>(OnceTeam(), R, it << P.lw, P.lw, work, tws);
   }
   if (b == 0) {
     for (int k = threadIdx.x; k < P.nch; k += blockDim.x) R.chunk_sum[k] = 0;
