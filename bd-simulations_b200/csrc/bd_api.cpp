@@ -681,6 +681,16 @@ int bd_inject_barrier_timeout(bd_ctx* c, int barrier, unsigned max_polls) {
   return c->e.inject_barrier_timeout(barrier, max_polls);
 }
 
+int bd_inject_wait_timeout(bd_ctx* c, int barrier, unsigned max_polls) {
+  if (!c) return BD_ERR_ARG;
+  return c->e.inject_wait_timeout(0, barrier, max_polls);
+}
+
+int bd_batch_inject_wait_timeout(bd_batch* b, int run, int barrier, unsigned max_polls) {
+  if (!b || run < 0) return BD_ERR_ARG;
+  return b->e.inject_wait_timeout((size_t)run, barrier, max_polls);
+}
+
 int bd_batch_stage_times(bd_batch* b, int nsteps, double* ms, int nstages) {
   if (!b || !ms) return BD_ERR_ARG;
   return b->e.stage_times(nsteps, ms, nstages);

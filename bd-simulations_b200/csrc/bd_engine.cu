@@ -580,7 +580,8 @@ void Engine::resident_items(std::vector<Item>& all) {
   if (cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) nsm = 0;
   const int fit = (int)runs.size() <= std::min(nsm, (int)BAR_GROUPS) ? resident_fit(-1, RES_GROUPS, 0, device) : 0;
   const int slots = std::min(nsm, fit);
-  std::vector<int> share(runs.size(), 1);
+  std::vector<int>& share = res_share;
+  share.assign(runs.size(), 1);
   double most_g = 1e30;
   if (slots >= (int)runs.size()) {
     auto top = [&]() {
@@ -707,8 +708,16 @@ RunDesc Engine::table_desc(size_t k) const {
 // nsteps steps of the only run in one launch; fault: with the pending
 // recovery-path test (grid mode); ts: phase timestamps of one step.
 int Engine::launch_one(int nsteps, bool fault, unsigned long long* ts) {
-  if (nsteps == 1 && !fault && one_step.grid > 0)
-    return launch_one_step(rone.one, d_dyn, one_step, d_bar, stream, ts) ? BD_ERR_CUDA : BD_OK;
+  if (nsteps == 1 && one_step.grid > 0) {
+    OneStepPlan P = one_step;
+    if (fault) {
+      P.skip_barrier = fault_barrier;
+      P.skip_cta = P.grid - 1;
+      P.max_polls = fault_polls;
+      fault_barrier = 0;
+    }
+    return launch_one_step(rone.one, d_dyn, P, d_bar, stream, ts) ? BD_ERR_CUDA : BD_OK;
+  }
   ResArgs A = rone;
   A.nsteps = nsteps;
   A.ts = ts;
@@ -729,9 +738,10 @@ int Engine::launch_one(int nsteps, bool fault, unsigned long long* ts) {
 // joined to the engine's stream once.
 int Engine::step_resident(long long nsteps) {
   if (runs.size() == 1) {
-    if (fault_barrier > 0 && nsteps > 0) {
-      RK(launch_one(1, true, nullptr));
-      nsteps--;
+    if (fault_barrier > 0) {
+      const int k = (int)std::min<long long>(nsteps, res_chunk);
+      RK(launch_one(k, true, nullptr));
+      nsteps -= k;
     }
     // 1024^2: four elements per thread of half the CTAs' threads are short of
     // the transforms' work, the launches cost less (65 536 particles, us per
@@ -752,10 +762,18 @@ int Engine::step_resident(long long nsteps) {
     A.bar = d_bar;
     A.part_off = (int)res_share_smem;
     A.pcap = res_pcap(RES_GROUPS);
+    if (fault_barrier > 0) {
+      A.skip_barrier = fault_barrier;
+      A.skip_group = (int)fault_run;
+      A.skip_cta = res_share[fault_run] - 1;
+      A.max_polls = fault_polls;
+      fault_barrier = 0;
+    }
     while (nsteps > 0) {
       A.nsteps = (int)std::min<long long>(nsteps, res_chunk);
       RK(launch_resident(-1, RES_GROUPS, A, 0, 0, res_share_grid, res_share_smem + (size_t)A.pcap * 32, stream));
       nsteps -= A.nsteps;
+      A.skip_barrier = 0;
     }
     return BD_OK;
   }
@@ -1130,7 +1148,14 @@ int Engine::enqueue_pipe(cudaStream_t s, cudaEvent_t* ev) {
 // end, the next step's inverse rows). ts (optional): the tail's timestamps.
 int Engine::enqueue_pipe2(cudaStream_t s, unsigned long long* ts) {
   RK(launch_step(d_runs, d_dyn, it(off_part), n_part, 1, part_large, s, part_shape));
-  return launch_pipe_tail(d_runs, d_dyn, tplan, d_bar, s, ts) ? BD_ERR_CUDA : BD_OK;
+  PipeTail P = tplan;
+  if (fault_barrier > 0) {
+    P.skip_barrier = fault_barrier;
+    P.skip_cta = P.grid - 1;
+    P.max_polls = fault_polls;
+    fault_barrier = 0;
+  }
+  return launch_pipe_tail(d_runs, d_dyn, P, d_bar, s, ts) ? BD_ERR_CUDA : BD_OK;
 }
 
 int Engine::set_step_form(int form, int ctas) {
@@ -1747,6 +1772,10 @@ int Engine::step(long long nsteps) {
   }
   if (piped) RK(fused_prologue(true));
   else RK(dep_invalidate());
+  if (fault_barrier > 0 && piped && pipe_form == PIPE_TWO && tail_ok) {
+    RK(enqueue_pipe2(stream));
+    nsteps--;
+  }
   if (!graphs_ok) RK(make_graphs());
   while (nsteps >= K) {
     CK(cudaGraphLaunch(gK, stream));
@@ -1820,6 +1849,23 @@ int Engine::inject_barrier_timeout(int barrier, unsigned max_polls) {
   if (!fused) return BD_ERR_STATE;
   fault_barrier = barrier;
   fault_polls = max_polls;
+  return BD_OK;
+}
+
+int Engine::inject_wait_timeout(size_t run, int barrier, unsigned max_polls) {
+  if (run >= runs.size() || barrier < 1 || max_polls == 0) return BD_ERR_ARG;
+  for (auto* r : runs)
+    if (!r->has_pos) return BD_ERR_STATE;
+  CK(cudaSetDevice(device));
+  if (!planned) RK(build_plan());
+  const bool waits = piped && pipe_form == PIPE_TWO && tail_ok ? barrier == 1
+                     : !resident                               ? false
+                     : runs.size() == 1                        ? true
+                                                               : res_share_grid > 0 && res_share[run] > 1;
+  if (!waits) return BD_ERR_STATE;
+  fault_barrier = barrier;
+  fault_polls = max_polls;
+  fault_run = run;
   return BD_OK;
 }
 
@@ -2105,7 +2151,7 @@ int Engine::sort_uploaded_run(size_t run) {
   Item* dp = r.d_sort;
   Item* dch = r.d_sort + r.n_sort_part;
   int st = BD_OK;
-  if (r.n_sort_part > 0) st = launch_count(d_runs, dp, r.n_sort_part, stream);
+  if (r.n_sort_part > 0) st = launch_count(d_runs, d_dyn, dp, r.n_sort_part, stream);
   if (!st)
     st = launch_sort(d_runs, d_dyn, (int)run, 1, dch, r.n_sort_chunk, dp, r.n_sort_part, 0, 0, 0, stream);
   if (!st) st = dep_invalidate();

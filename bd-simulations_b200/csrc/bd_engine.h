@@ -147,6 +147,9 @@ class Engine {
   // of arriving at grid barrier `barrier` (1..3) and every wait give up after
   // max_polls polls; BD_ERR_STATE without the fused step
   int inject_barrier_timeout(int barrier, unsigned max_polls);
+  // the same for every step with grid barriers: a single resident run (any
+  // dt, any mesh), the group of CTAs of run `run`, the cooperative tail
+  int inject_wait_timeout(size_t run, int barrier, unsigned max_polls);
 
  private:
   RunDesc* d_runs = nullptr;
@@ -220,6 +223,7 @@ class Engine {
   size_t rone_smem = 0;
   int res_share_grid = 0, off_share = 0;
   size_t res_share_smem = 0;
+  std::vector<int> res_share;  // CTAs of every run's group
   int res_chunk = 1;  // steps per launch
   void resident_items(std::vector<Item>& all);
   int plan_resident();
@@ -265,6 +269,7 @@ class Engine {
   // one-shot fault of the next fused launch (inject_barrier_timeout)
   int fault_barrier = 0;
   unsigned fault_polls = 0;
+  size_t fault_run = 0;
   // after a failed grid barrier: the run back at its state before the step
   int recover_fused();
   cudaGraphExec_t g1 = nullptr, gK = nullptr;

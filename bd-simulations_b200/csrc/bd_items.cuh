@@ -25,8 +25,16 @@ __device__ __forceinline__ int wrap1(int a, int m) {
   return a < 0 ? a + m : (a >= m ? a - m : a);
 }
 
+// A bounded wait of a step of this run gave up: its cell counts, chunk totals
+// and density sums may hold half a step. No step form and no sort touches the
+// run until the host has put it back (Engine::recover_fused); a second move
+// would count its particles twice and the scatter write past its records.
+__device__ __forceinline__ bool run_failed(const RunDyn* dyn, int run) {
+  return (dyn[run].err & E_BARRIER_TIMEOUT) != 0;
+}
+
 __device__ __forceinline__ bool run_active(const RunDyn* dyn, int run) {
-  return dyn[run].steps_left > 0;
+  return dyn[run].steps_left > 0 && !run_failed(dyn, run);
 }
 
 // Load of data that earlier kernels wrote: through the read-only cache when

@@ -480,7 +480,7 @@ __global__ void __launch_bounds__(256) k_move(const RunDesc* __restrict__ runs,
                                               int require_active, int refresh_only) {
   for (int it = blockIdx.x; it < nitems; it += gridDim.x) {
     const Item I = items[it];
-    if (require_active && !run_active(dyn, I.run)) continue;
+    if (require_active ? !run_active(dyn, I.run) : run_failed(dyn, I.run)) continue;
     const RunDesc& R = runs[I.run];
     RunDyn& D = dyn[I.run];
     const int gi = I.a * blockDim.x + threadIdx.x;
@@ -503,10 +503,11 @@ __global__ void __launch_bounds__(256) k_move(const RunDesc* __restrict__ runs,
 }
 
 // Keys of an unsorted upload in recB (initial sort).
-__global__ void __launch_bounds__(256) k_count(const RunDesc* __restrict__ runs,
+__global__ void __launch_bounds__(256) k_count(const RunDesc* __restrict__ runs, const RunDyn* __restrict__ dyn,
                                                const Item* __restrict__ items, int nitems) {
   for (int it = blockIdx.x; it < nitems; it += gridDim.x) {
     const Item I = items[it];
+    if (run_failed(dyn, I.run)) continue;
     const RunDesc& R = runs[I.run];
     const int gi = I.a * blockDim.x + threadIdx.x;
     const unsigned act = __ballot_sync(0xffffffffu, gi < R.N);
@@ -536,7 +537,7 @@ __global__ void __launch_bounds__(1024) k_chunk_scan(const RunDesc* __restrict__
   for (int run = run0 + blockIdx.x; run < run0 + nruns; run += gridDim.x) {
     // the scan and the scatter of this sort follow this decision, taken
     // before end_step changes the steps budget
-    const bool on = !require_active || run_active(dyn, run);
+    const bool on = require_active ? run_active(dyn, run) : !run_failed(dyn, run);
     __syncthreads();
     if (threadIdx.x == 0) dyn[run].sorting = on ? 1 : 0;
     if (!on) continue;
@@ -574,11 +575,11 @@ struct ScanChunk {
 };
 
 __device__ __forceinline__ void scan_load(const RunDesc* __restrict__ runs, const RunDyn* __restrict__ dyn,
-                                          const Item& I, int require_active, ScanChunk& S) {
+                                          const Item& I, ScanChunk& S) {
   constexpr int PER = SCAN_CHUNK / 256;
   S.R = &runs[I.run];
   S.chunk = I.a;
-  S.on = !require_active || dyn[I.run].sorting;
+  S.on = dyn[I.run].sorting;
   S.ncells = S.R->C * S.R->C;
   const int base = I.a * SCAN_CHUNK;
   const int c0 = base + threadIdx.x * PER;
@@ -595,16 +596,16 @@ __device__ __forceinline__ void scan_load(const RunDesc* __restrict__ runs, cons
 }
 
 __global__ void __launch_bounds__(256) k_scan(const RunDesc* __restrict__ runs, const RunDyn* __restrict__ dyn,
-                                              const Item* __restrict__ items, int nitems, int require_active) {
+                                              const Item* __restrict__ items, int nitems) {
   static_assert(SCAN_CHUNK == 2048, "eight counts per thread");
   __shared__ int sh[32];
   int it = blockIdx.x;
   if (it >= nitems) return;
   ScanChunk cur, nxt;
-  scan_load(runs, dyn, items[it], require_active, cur);
+  scan_load(runs, dyn, items[it], cur);
   for (;;) {
     const int itn = it + gridDim.x;
-    if (itn < nitems) scan_load(runs, dyn, items[itn], require_active, nxt);
+    if (itn < nitems) scan_load(runs, dyn, items[itn], nxt);
     if (cur.on) scan_chunk_store<SCAN_CHUNK / 256>(CtaTeam(), *cur.R, cur.chunk, cur.ncells, cur.v, cur.R->chunk_off[cur.chunk], sh);
     if (itn >= nitems) break;
     it = itn;
@@ -616,11 +617,10 @@ __global__ void __launch_bounds__(256) k_scan(const RunDesc* __restrict__ runs, 
 // order within a cell is arbitrary and no result depends on it).
 __global__ void __launch_bounds__(256) k_scatter(const RunDesc* __restrict__ runs,
                                                  const RunDyn* __restrict__ dyn,
-                                                 const Item* __restrict__ items, int nitems,
-                                                 int require_active) {
+                                                 const Item* __restrict__ items, int nitems) {
   for (int it = blockIdx.x; it < nitems; it += gridDim.x) {
     const Item I = items[it];
-    if (require_active && !dyn[I.run].sorting) continue;
+    if (!dyn[I.run].sorting) continue;
     const RunDesc& R = runs[I.run];
     const int gi = I.a * blockDim.x + threadIdx.x;
     if (gi >= R.N) continue;
@@ -962,6 +962,17 @@ __global__ void __launch_bounds__(256, MINB) k_pipe_tail(const RunDesc* __restri
   // before this launch; read with volatile loads (the run's state line may
   // sit in this SM's L1 while the step end in phase D changes it)
   volatile const RunDyn* dv = dyn;
+  // a failed barrier leaves every run that took part in mid-step: all of them
+  // are marked, so that no other form steps them before the host's recovery
+  auto barrier = [&]() -> bool {
+    if (P.skip_barrier == (int)ep + 1 && b == P.skip_cta) return false;
+    if (grid_barrier(bar, ++ep * G, maxp, &dyn[0].err, &s_ok)) return true;
+    for (int c = threadIdx.x; c < P.nchunk; c += nt) {
+      const Item I = P.chunks[c];
+      if (I.a == 0 && dv[I.run].sorting) atomicOr(&dyn[I.run].err, E_BARRIER_TIMEOUT);
+    }
+    return false;
+  };
   for (int u = b; u < P.ncu; u += G) {
     const Item I = P.cunits[u];
     if (!dv[I.run].sorting) continue;
@@ -969,7 +980,7 @@ __global__ void __launch_bounds__(256, MINB) k_pipe_tail(const RunDesc* __restri
     if (I.b < 0) scan_chunk_item(R, I.a, s_tmp);
     else tail_fft_item<1>(&R, I);
   }
-  if (!grid_barrier(bar, ++ep * G, maxp, &dyn[0].err, &s_ok)) return;
+  if (!barrier()) return;
   if (rec) ts[1] = global_ns();
   for (int u = b; u < P.ndu; u += G) {
     const Item I = P.dunits[u];
@@ -984,14 +995,14 @@ __global__ void __launch_bounds__(256, MINB) k_pipe_tail(const RunDesc* __restri
     runs[I.run].chunk_sum[I.a] = 0;
     if (I.a == 0) end_step(runs[I.run], dyn[I.run], 0);
   }
-  if (!grid_barrier(bar, ++ep * G, maxp, &dyn[0].err, &s_ok)) return;
+  if (!barrier()) return;
   if (rec) ts[2] = global_ns();
   for (int u = b; u < P.ninv; u += G) {
     const Item I = P.inv[u];
     if (dv[I.run].sorting) tail_fft_item<0>(&runs[I.run], I);
   }
   if (ts) {
-    if (!grid_barrier(bar, ++ep * G, maxp, &dyn[0].err, &s_ok)) return;
+    if (!barrier()) return;
     if (rec) ts[3] = global_ns();
   }
   grid_exit(bar, G);
@@ -1606,9 +1617,9 @@ int launch_records_by_pid(const Rec* src, Rec* dst, int n, cudaStream_t s) {
   return 0;
 }
 
-int launch_count(const RunDesc* runs, const Item* items, int n, cudaStream_t s) {
+int launch_count(const RunDesc* runs, const RunDyn* dyn, const Item* items, int n, cudaStream_t s) {
   if (n <= 0) return 0;
-  k_count<<<grid_for(n, 65535), 256, 0, s>>>(runs, items, n);
+  k_count<<<grid_for(n, 65535), 256, 0, s>>>(runs, dyn, items, n);
   BD_LAUNCH_CHECK();
   return 0;
 }
@@ -1619,12 +1630,12 @@ int launch_sort(const RunDesc* runs, RunDyn* dyn, int run0, int nruns, const Ite
   if (nchunks > 0) {
     k_chunk_scan<<<nruns, 1024, 0, s>>>(runs, dyn, run0, nruns, end_step_flag, adaptive, require_active);
     BD_LAUNCH_CHECK();
-    k_scan<<<grid_for(nchunks, 148 * 8), 256, 0, s>>>(runs, dyn, chunks, nchunks, require_active);
+    k_scan<<<grid_for(nchunks, 148 * 8), 256, 0, s>>>(runs, dyn, chunks, nchunks);
     BD_LAUNCH_CHECK();
   }
   if (ev) cudaEventRecord(ev[0], s);
   if (nparts > 0) {
-    k_scatter<<<grid_for(nparts, 65535), 256, 0, s>>>(runs, dyn, parts, nparts, require_active);
+    k_scatter<<<grid_for(nparts, 65535), 256, 0, s>>>(runs, dyn, parts, nparts);
     BD_LAUNCH_CHECK();
   }
   if (ev) {

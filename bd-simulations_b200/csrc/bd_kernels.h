@@ -91,6 +91,7 @@ struct PipeTail {
   const Item* inv;     // inverse row items
   int ninv;
   unsigned max_polls;  // grid-barrier poll bound (0: the default, about a second)
+  int skip_barrier, skip_cta;  // recovery-path test, as ResArgs
   size_t smem;    // the largest transform item's shared memory
   int minb;       // CTAs per SM the registers are bounded for (2, 3 or 4)
   int grid;       // filled by pipe_tail_configure
@@ -102,7 +103,7 @@ int launch_pipe_tail(const RunDesc* runs, RunDyn* dyn, const PipeTail& P, unsign
                      unsigned long long* ts = nullptr);
 int launch_move(const RunDesc* runs, RunDyn* dyn, const Item* items, int n, int require_active,
                 int refresh_only, cudaStream_t s);
-int launch_count(const RunDesc* runs, const Item* items, int n, cudaStream_t s);
+int launch_count(const RunDesc* runs, const RunDyn* dyn, const Item* items, int n, cudaStream_t s);
 // dst[src[i].pid] = src[i] for the n records of one run
 int launch_records_by_pid(const Rec* src, Rec* dst, int n, cudaStream_t s);
 // scan of the cell counts (chunk offsets of runs run0 .. run0+nruns-1, then
@@ -139,9 +140,10 @@ struct ResArgs {
   // grid-barrier waits give up after this many polls (0: the default bound,
   // about a second); a wait that gives up fails that barrier for every CTA
   unsigned max_polls;
-  // recovery-path test: CTA skip_cta returns instead of arriving at barrier
-  // skip_barrier (1-based; 0: none), so every other CTA's wait gives up
-  int skip_barrier, skip_cta;
+  // recovery-path test: CTA skip_cta (of group skip_group) returns instead of
+  // arriving at barrier skip_barrier (1-based; 0: none), so every other CTA's
+  // wait gives up; max_polls then bounds that group's waits only
+  int skip_barrier, skip_cta, skip_group;
   unsigned long long* ts;  // single run: FUSED_PHASES + 1 timestamps of one step (may be null)
 };
 // kind: one run, one cluster per run, or groups of CTAs of one cooperative grid.
@@ -162,6 +164,8 @@ struct OneStepPlan {
   int lw, ncl;   // column items
   int lri, nri;  // inverse row items
   int nch;       // scan chunks
+  unsigned max_polls;          // as ResArgs
+  int skip_barrier, skip_cta;
   size_t smem;   // dynamic shared memory
   int grid;      // CTAs (all resident: cooperative launch); 0: no plan
 };

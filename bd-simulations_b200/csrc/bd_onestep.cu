@@ -69,7 +69,12 @@ __global__ void __launch_bounds__(256, 2) k_one_step(const __grid_constant__ Run
   const bool rec = ts && b == 0 && threadIdx.x == 0;
   int ph = 0;
   if (rec) ts[0] = global_ns();
-  auto barrier = [&]() -> bool { return grid_barrier(bar, ++ep * (unsigned)G, BAR_MAX_POLLS, &D.err, &s_ok); };
+  // after a barrier that failed in an earlier launch the words still hold its
+  // poison: this launch ends at its first barrier, before anything moves
+  auto barrier = [&]() -> bool {
+    if (P.skip_barrier == (int)ep + 1 && b == P.skip_cta) return false;
+    return grid_barrier(bar, ++ep * (unsigned)G, P.max_polls ? P.max_polls : BAR_MAX_POLLS, &D.err, &s_ok);
+  };
 #define BD_BARRIER()      \
   if (!barrier()) return; \
   if (rec) ts[++ph] = global_ns()

@@ -889,6 +889,9 @@ __global__ void __launch_bounds__(res_threads(KIND), KIND == RES_CLUSTERS ? 2 : 
   const bool alias = (const void*)R.dacc == (const void*)R.spec2;
   const bool adaptive = (R.flags & F_ADAPTIVE) != 0;
   const long long budget = ((volatile RunDyn*)D)->steps_left;
+  // a run that failed takes no step (run_failed). One thread looks: a slow
+  // CTA may start while a failure of this launch is being marked
+  if (threadIdx.x == 0) s_ok = !(((volatile RunDyn*)D)->err & E_BARRIER_TIMEOUT);
   unsigned long long step = ((volatile RunDyn*)D)->step;
   if constexpr (SINGLE) {
     // what the phases read first is requested into L2 ahead of them
@@ -909,6 +912,7 @@ __global__ void __launch_bounds__(res_threads(KIND), KIND == RES_CLUSTERS ? 2 : 
     }
   const int nst = (int)min((long long)A.nsteps, budget);
   __syncthreads();
+  if (!s_ok) return;
   const int nch = (R.C * R.C + SCAN_CHUNK - 1) / SCAN_CHUNK;
   // an equal contiguous share of the particles per CTA, the first pcap of
   // them in shared memory
@@ -918,13 +922,14 @@ __global__ void __launch_bounds__(res_threads(KIND), KIND == RES_CLUSTERS ? 2 : 
   // particle of the run goes through it
   float2* noise = per <= A.pcap && !(R.flags & F_NOWCA) ? reinterpret_cast<float2*>(R.recB) : nullptr;
   unsigned ep = 0;
-  const unsigned maxp = A.max_polls ? A.max_polls : BAR_MAX_POLLS;
+  const bool test = A.skip_barrier > 0 && (!GROUPS || J.a == A.skip_group);
+  const unsigned maxp = test ? A.max_polls : BAR_MAX_POLLS;
   auto barrier = [&]() -> bool {
     if (!grid) {
       cluster_barrier();
       return true;
     }
-    if (A.skip_barrier == (int)ep + 1 && b == A.skip_cta) return false;
+    if (test && A.skip_barrier == (int)ep + 1 && b == A.skip_cta) return false;
     return grid_barrier(bar, ++ep * (unsigned)G, maxp, &D->err, &s_ok);
   };
   const bool rec = SINGLE && A.ts && b == 0 && threadIdx.x == 0;

@@ -447,6 +447,17 @@ int bd_batch_phase_times(bd_batch* b, int nsteps, double* ms, int nphases);
  * bits of a run that never failed. BD_ERR_STATE when the context does not
  * use the fused step; BD_ERR_ARG for barrier outside 1..3 or max_polls 0. */
 int bd_inject_barrier_timeout(bd_ctx* c, int barrier, unsigned max_polls);
+/* The same for every step whose kernels hold grid barriers, whatever its mesh
+ * and dt (barriers counted from the launch's start: per step of the resident
+ * kernel 4, with an adaptive dt 5): a single run; one run of a batch that
+ * steps in groups of CTAs of one cooperative grid (the other runs step on); a
+ * batch in step form 1 (barrier 1 of the cooperative launch: every run's step
+ * fails). Until a synchronising call (bd_zeitschritte, bd_sync,
+ * bd_batch_sync, an adaptive bd_zeitschritt) has returned BD_ERR_TIMEOUT, no
+ * form of stepping or sorting touches a failed run. BD_ERR_STATE when the
+ * steps wait on no grid barrier. */
+int bd_inject_wait_timeout(bd_ctx* c, int barrier, unsigned max_polls);
+int bd_batch_inject_wait_timeout(bd_batch* b, int run, int barrier, unsigned max_polls);
 
 /* ---- serving: continuous batching of run requests ----------------------- */
 typedef struct bd_serve_opts {
