@@ -162,3 +162,32 @@ def test_wait_hook_refused_without_grid_barriers(gpu):
         with pytest.raises(gpu.BdError) as e:
             r._call("bd_inject_wait_timeout", *args)
         assert e.value.status == status
+
+
+# a group barrier behind each phase of an adaptive step, the dt bound's
+# (2) among them; a mesh of each class, 2^k and 3 * 2^k and other factors of 3
+@pytest.mark.parametrize("barrier", [1, 2, 3, 4])
+@pytest.mark.parametrize("n1,n2,mesh", [(400, 301, 64), (900, 800, 144), (2000, 1501, 384)])
+def test_adaptive_step_reports_its_failed_wait(gpu, n1, n2, mesh, barrier):
+    p = _params(gpu, n1, n2, mesh, True, obs_dt=0.01)
+    start = _lattice(p, 9)
+    a, b = gpu.Run(p, seed=4), gpu.Run(p, seed=4)
+    for r in (a, b):
+        r.set_positions_all(start)
+    # the run's first step: no step length to repeat
+    a._call("bd_inject_wait_timeout", barrier, 20000)
+    _timeout(gpu, a.zeitschritte_bis_obs)
+    assert a.step_count() == 0 and a.time() == 0.0
+    _same(a.get_positions(), b.get_positions())
+    assert a.zeitschritt() == b.zeitschritt()
+    a._call("bd_inject_wait_timeout", barrier, 20000)
+    _timeout(gpu, a.zeitschritt)
+    assert a.step_count() == 1 and a.time() == b.time()
+    _same(a.get_positions(), b.get_positions())
+    # the failed steps added nothing to the time since the observation
+    assert a.zeitschritte_bis_obs() == b.zeitschritte_bis_obs()
+    _same(a.get_positions(), b.get_positions())
+    fa, fb = a.get_forces(), b.get_forces()
+    for k in fa:
+        assert np.array_equal(fa[k], fb[k])
+    assert a.time() == b.time()
