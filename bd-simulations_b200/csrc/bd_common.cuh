@@ -208,6 +208,10 @@ __device__ __forceinline__ void mesh_axis(const RunDesc& R, int ic, float off, i
   // the position lies in (-B, L + B]: k in (-Z, 2Z), one conditional wrap
   if (k < 0) k += R.Z;
   else if (k >= R.Z) k -= R.Z;
+  // a position out of the box (not finite, or thrown further than re-binning
+  // reaches) is still one mesh point: the move's deposit uses it in the step
+  // that makes it, before any error is read
+  k = (int)min((unsigned)k, (unsigned)(R.Z - 1));
 }
 
 // weights as the reference's grid routines (gridRoutinen.cpp): NGP puts all
