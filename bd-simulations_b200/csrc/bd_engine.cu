@@ -1794,14 +1794,15 @@ int Engine::sync_check(RunDyn* dd) {
   }
   RK(fetch_dyn(0, runs.size()));
   if (dd && !runs.empty()) *dd = h_dyn[0];
-  for (size_t k = 0; k < runs.size(); k++) {
-    if (h_dyn[k].err & E_NONFINITE) return BD_ERR_NONFINITE;
-    if (h_dyn[k].err & E_BARRIER_TIMEOUT) {
-      RK(recover_fused());
-      return BD_ERR_TIMEOUT;
-    }
+  // a wait that gave up is mended and reported ahead of any other run's error
+  // (which stays for the next call): its run takes no step until then
+  int err = 0;
+  for (size_t k = 0; k < runs.size(); k++) err |= h_dyn[k].err;
+  if (err & E_BARRIER_TIMEOUT) {
+    RK(recover_fused());
+    return BD_ERR_TIMEOUT;
   }
-  return BD_OK;
+  return err & E_NONFINITE ? BD_ERR_NONFINITE : BD_OK;
 }
 
 // A resident step whose grid barrier failed ran no phase past that barrier (the

@@ -66,3 +66,27 @@ def test_thrown_run_of_a_batch(gpu, meshes):
         r.set_positions_all(_lattice(runs[k], 20 + k))
         r.stage_times(5)
         _same(b.get_positions(k), r.get_positions())
+
+
+def test_thrown_run_does_not_hide_another_runs_failed_wait(gpu):
+    """Both errors in one batch: the run whose wait gave up is put back and
+    reported, the thrown one's error stays."""
+    meshes = (96, 384, 64)
+    runs = [_params(gpu, 900, 601, m, k == 1) for k, m in enumerate(meshes)]
+    runs[0] = _thrown(gpu, 900, 601, meshes[0], 1e30)
+    b = gpu.Batch(runs, [1, 2, 3])
+    for k, p in enumerate(runs):
+        b.set_positions(k, _lattice(p, 30 + k))
+    assert gpu.lib().bd_batch_inject_wait_timeout(b.h, 1, 3, 20000) == 0
+    b.step(2)
+    assert _status(gpu, b.sync) == BD_ERR_TIMEOUT
+    assert _status(gpu, b.sync) == BD_ERR_NONFINITE
+    assert b.time(1) == 0.0
+    b.step(4)
+    assert _status(gpu, b.sync) == BD_ERR_NONFINITE
+    for k, n in ((1, 4), (2, 6)):
+        r = gpu.Run(runs[k], seed=k + 1)
+        r.set_positions_all(_lattice(runs[k], 30 + k))
+        r.stage_times(n)
+        _same(b.get_positions(k), r.get_positions())
+        assert b.time(k) == r.time()
