@@ -11,6 +11,7 @@
 #include <tuple>
 
 #include "bd_fft2.cuh"
+#include "bd_forms.h"
 #include "bd_host.h"
 
 namespace bd {
@@ -523,103 +524,53 @@ void Engine::resident_items(std::vector<Item>& all) {
     resident = true;
     return;
   }
+  std::vector<FormRun> fr(runs.size());
+  for (size_t k = 0; k < runs.size(); k++) fr[k] = {runs[k]->N, runs[k]->Z, runs[k]->idgas};
+  auto held = [&](size_t k, int cs) {
+    size_t smem = 0;
+    resident_item(*runs[k], (int)k, cs, res_threads(RES_CLUSTERS) / 2, &smem);
+    if (smem + (size_t)res_pcap(RES_CLUSTERS) * 32 > res_max_smem(RES_CLUSTERS)) return 0;
+    return resident_fit(resident_lz(*runs[k]), RES_CLUSTERS, cs, device);
+  };
+  // groups have a pair of barrier words each and one CTA per SM
+  int nsm = 0, slots = 0;
+  if (cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) nsm = 0;
+  if (runs.size() <= (size_t)std::min(nsm, (int)BAR_GROUPS)) slots = std::min(nsm, resident_fit(-1, RES_GROUPS, 0, device));
+  const BatchForm form = choose_batch_form(fr, held, slots, piped);
+  if (form.step == BATCH_LAUNCHES) return;
+  if (form.step == BATCH_GROUPS) {
+    off_share = (int)all.size();
+    res_share = form.ctas;
+    res_share_smem = 0;
+    int grid = 0;
+    for (size_t k = 0; k < runs.size(); k++) {
+      size_t sm = 0;
+      const Item I = resident_item(*runs[k], (int)k, res_share[k], res_threads(RES_GROUPS) / 2, &sm);
+      res_share_smem = std::max(res_share_smem, sm);
+      for (int c = 0; c < res_share[k]; c++) {
+        all.push_back(I);
+        all.push_back({resident_lz(*runs[k]), (int)k, c, res_share[k]});
+        grid++;
+      }
+    }
+    if (res_share_smem + (size_t)res_pcap(RES_GROUPS) * 32 > res_max_smem(RES_GROUPS)) return;
+    res_share_grid = grid;
+    resident = true;
+    return;
+  }
   struct Ent {
     Item I;
     int lz, cs;
     size_t smem;
-    double load, share;
+    double load;
   };
-  std::vector<Ent> v;
-  // load: particles and a quarter of the mesh points per CTA
-  auto weight = [&](const RunHost& r) { return r.N + (r.idgas ? 0.0 : 0.25 * r.Z * r.Z); };
-  long long particles = 0;
-  for (auto* r : runs) particles += r->N;
-  // every run on clusters of one size, the largest at which the whole batch
-  // is resident at once; then larger clusters for runs that would hold the
-  // others up, while there is room to spare. share: the part of the GPU one
-  // cluster takes (the device is asked: clusters of 16 pack badly into GPCs)
-  auto entry = [&](size_t k, int cs) {
-    const RunHost& r = *runs[k];
-    Ent e{};
-    e.lz = resident_lz(r);
-    e.cs = cs;
-    e.I = resident_item(r, (int)k, cs, res_threads(RES_CLUSTERS) / 2, &e.smem);
-    e.load = weight(r) / cs;
-    const int n = e.smem + (size_t)res_pcap(RES_CLUSTERS) * 32 <= res_max_smem(RES_CLUSTERS) ? resident_fit(e.lz, RES_CLUSTERS, cs, device) : 0;
-    e.share = n > 0 ? 1.0 / n : 1e9;
-    return e;
-  };
-  // a batch that takes a mix of cluster sizes fills the GPU less well (0.8)
-  double most = 1e30;
-  for (int base = 16; base >= 1; base /= 2) {
-    std::vector<Ent> w;
-    double used = 0.0;
-    for (size_t k = 0; k < runs.size() && used <= 1.0; k++) {
-      w.push_back(entry(k, base));
-      used += w.back().share;
-    }
-    if (used > 1.0) continue;
-    size_t top = 0;
-    for (;;) {
-      for (size_t k = 0; k < w.size(); k++)
-        if (w[k].load > w[top].load) top = k;
-      if (w[top].cs >= 16) break;
-      const Ent e = entry(top, w[top].cs * 2);
-      if (used + e.share - w[top].share > 0.8) break;
-      used += e.share - w[top].share;
-      w[top] = e;
-    }
-    if (w[top].load < 0.95 * most) {
-      most = w[top].load;
-      v.swap(w);
-    }
-  }
-  // the same for groups of CTAs of one cooperative grid, a CTA at a time to
-  // the run with the largest load
-  int nsm = 0;
-  if (cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) nsm = 0;
-  const int fit = (int)runs.size() <= std::min(nsm, (int)BAR_GROUPS) ? resident_fit(-1, RES_GROUPS, 0, device) : 0;
-  const int slots = std::min(nsm, fit);
-  std::vector<int>& share = res_share;
-  share.assign(runs.size(), 1);
-  double most_g = 1e30;
-  if (slots >= (int)runs.size()) {
-    auto top = [&]() {
-      size_t t = 0;
-      for (size_t k = 1; k < runs.size(); k++)
-        if (weight(*runs[k]) / share[k] > weight(*runs[t]) / share[t]) t = k;
-      return t;
-    };
-    for (int left = slots - (int)runs.size(); left > 0; left--) share[top()]++;
-    const size_t t = top();
-    most_g = weight(*runs[t]) / share[t];
-  }
-  // Which form: estimates of a step in us, fitted to measurements of 1 to 128
-  // runs of 1000 to 250 000 particles (clusters 12-60, groups 14-45, the
-  // pipelined step 20-110; the stage kernels, 45-900, were never the fastest)
-  const double t_clusters = v.empty() ? 1e30 : 8.0 + 0.025 * most;
-  const double t_groups = 14.0 + 0.016 * most_g;
-  const double t_piped = piped ? 19.0 + 8e-5 * particles : 1e30;
-  if (std::min(t_clusters, t_groups) > t_piped) return;
-  if (t_groups < t_clusters) {
-    off_share = (int)all.size();
-    res_share_smem = 0;
-    for (size_t k = 0; k < runs.size(); k++) {
-      size_t sm = 0;
-      const Item I = resident_item(*runs[k], (int)k, share[k], res_threads(RES_GROUPS) / 2, &sm);
-      res_share_smem = std::max(res_share_smem, sm);
-      for (int c = 0; c < share[k]; c++) {
-        all.push_back(I);
-        all.push_back({resident_lz(*runs[k]), (int)k, c, share[k]});
-        res_share_grid++;
-      }
-    }
-    if (res_share_smem + (size_t)res_pcap(RES_GROUPS) * 32 > res_max_smem(RES_GROUPS)) {
-      res_share_grid = 0;
-      return;
-    }
-    resident = true;
-    return;
+  std::vector<Ent> v(runs.size());
+  for (size_t k = 0; k < runs.size(); k++) {
+    Ent& e = v[k];
+    e.cs = form.ctas[k];
+    e.lz = resident_lz(*runs[k]);
+    e.I = resident_item(*runs[k], (int)k, e.cs, res_threads(RES_CLUSTERS) / 2, &e.smem);
+    e.load = fr[k].weight() / e.cs;
   }
   std::stable_sort(v.begin(), v.end(), [](const Ent& a, const Ent& b) {
     return a.lz != b.lz ? a.lz < b.lz : a.cs != b.cs ? a.cs > b.cs : a.load > b.load;
@@ -648,6 +599,7 @@ int Engine::plan_resident() {
     CK(cudaMemsetAsync(d_bar, 0, 2 * BAR_GROUPS * sizeof(unsigned), stream));
   }
   if (runs.size() > 1) {
+    if (res_share_grid > 0 ? res_share_grid > resident_fit(-1, RES_GROUPS, 0, device) : res_groups.empty()) return BD_OK;
     for (const ResGroup& g : res_groups)
       if (resident_fit(g.lz, RES_CLUSTERS, g.cs, device) <= 0) return BD_OK;
     while (res_streams.size() + 1 < res_groups.size()) {
