@@ -346,12 +346,16 @@ __global__ void __launch_bounds__(FFT_THREADS) k_fft_rows_inv(const RunDesc* __r
   }
 }
 
-// The three passes as kernels (meshes of 2048 and more: four CTAs per SM, 64
-// registers; columns 55 -> 47 us at 2048^2), one item per CTA (an item loop around the
+// The three passes as kernels, one item per CTA (an item loop around the
 // transform with twiddles from global memory makes the compiler hoist the
-// twiddle loads of every pass and spill).
+// twiddle loads of every pass and spill). Meshes of 2048 and more: bounded for
+// four CTAs per SM, 64 registers (columns 55 -> 47 us at 2048^2). Smaller ones
+// name no number of CTAs: told that one is enough, the compiler took 128, 94
+// and 55 registers for columns, inverse and forward rows of 1024 points
+// instead of 80, 64 and 40 (200 meshes of 1024^2, us per pass 2608, 1863 and 868
+// instead of 2053, 1216 and 704).
 template <int LZ>
-__global__ void __launch_bounds__(FFT2_THREADS, LZ >= 11 ? 4 : 1) k_fft2_rows_fwd(const RunDesc* __restrict__ runs,
+__global__ void __launch_bounds__(FFT2_THREADS, LZ >= 11 ? 4 : 0) k_fft2_rows_fwd(const RunDesc* __restrict__ runs,
                                                          const RunDyn* __restrict__ dyn,
                                                          const Item* __restrict__ items, int nitems,
                                                          int require_active) {
@@ -361,11 +365,11 @@ __global__ void __launch_bounds__(FFT2_THREADS, LZ >= 11 ? 4 : 1) k_fft2_rows_fw
   if (require_active && !run_active(dyn, I.run)) return;
   const RunDesc& R = runs[I.run];
   if constexpr (LZ >= 11) big_rows_fwd_item<LZ, false>(R, I.a, I.c, (float2*)smem, R.tw);
-  else fft2_rows_fwd_item<LZ, false, false>(CtaTeam(), R, I.a, I.c, (float2*)smem, R.tw);
+  else fft2_rows_fwd_item<LZ, false, false>(OnceTeam(), R, I.a, I.c, (float2*)smem, R.tw);
 }
 
 template <int LZ>
-__global__ void __launch_bounds__(FFT2_THREADS, LZ >= 11 ? 4 : 1) k_fft2_cols(const RunDesc* __restrict__ runs,
+__global__ void __launch_bounds__(FFT2_THREADS, LZ >= 11 ? 4 : 0) k_fft2_cols(const RunDesc* __restrict__ runs,
                                                      const RunDyn* __restrict__ dyn,
                                                      const Item* __restrict__ items, int nitems,
                                                      int require_active) {
@@ -375,11 +379,11 @@ __global__ void __launch_bounds__(FFT2_THREADS, LZ >= 11 ? 4 : 1) k_fft2_cols(co
   if (require_active && !run_active(dyn, I.run)) return;
   const RunDesc& R = runs[I.run];
   if constexpr (LZ >= 11) big_cols_item<LZ>(R, I.a, I.c, (float2*)smem, R.tw);
-  else fft2_cols_item<LZ, false>(CtaTeam(), R, I.a, I.c, (float2*)smem, R.tw);
+  else fft2_cols_item<LZ, false>(OnceTeam(), R, I.a, I.c, (float2*)smem, R.tw);
 }
 
 template <int LZ>
-__global__ void __launch_bounds__(FFT2_THREADS, LZ >= 11 ? 4 : 1) k_fft2_rows_inv(const RunDesc* __restrict__ runs,
+__global__ void __launch_bounds__(FFT2_THREADS, LZ >= 11 ? 4 : 0) k_fft2_rows_inv(const RunDesc* __restrict__ runs,
                                                          const RunDyn* __restrict__ dyn,
                                                          const Item* __restrict__ items, int nitems,
                                                          int require_active) {
@@ -389,7 +393,7 @@ __global__ void __launch_bounds__(FFT2_THREADS, LZ >= 11 ? 4 : 1) k_fft2_rows_in
   if (require_active && !run_active(dyn, I.run)) return;
   const RunDesc& R = runs[I.run];
   if constexpr (LZ >= 11) big_rows_inv_item<LZ>(R, I.a, I.c, (float2*)smem, R.tw);
-  else fft2_rows_inv_item<LZ, false>(CtaTeam(), R, I.a, I.c, (float2*)smem, R.tw);
+  else fft2_rows_inv_item<LZ, false>(OnceTeam(), R, I.a, I.c, (float2*)smem, R.tw);
 }
 
 // The step's particle kernel: forces, noise, move, re-binning and counts, one
