@@ -416,7 +416,6 @@ void Engine::drop_graphs() {
   if (g1) cudaGraphExecDestroy(g1);
   if (gK) cudaGraphExecDestroy(gK);
   g1 = gK = nullptr;
-  graphs_ok = false;
 }
 
 // The resident step takes runs on power-of-two meshes from 8 to 1024 and on
@@ -832,6 +831,7 @@ int Engine::build_plan() {
   CK(cudaSetDevice(device));
   CK(cudaStreamSynchronize(stream));  // earlier work may still read the old tables
   drop_graphs();
+  fault_barrier = 0;  // a pending recovery-path test is not captured
   dep_valid = grids_valid = false;  // the next resident or pipelined step starts with the prologue
   descs_ok = false;   // the descriptions depend on the plan (the accumulator of piped runs)
   std::vector<Item> all, dep, part, chunk;
@@ -1031,6 +1031,7 @@ int Engine::build_plan() {
   RK(upload_tables());
   RK(plan_resident());
   RK(plan_tail());
+  RK(plan_graphs());
   planned = true;
   return BD_OK;
 }
@@ -1680,27 +1681,42 @@ int Engine::autotune(int reps, bd_tune_result* out) {
   return BD_OK;
 }
 
-int Engine::make_graphs() {
-  if (runs.empty()) return BD_OK;
-  for (int which = 0; which < 2; which++) {
-    const int nst = which == 0 ? 1 : K;
-    cudaGraph_t g = nullptr;
-    CK(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
-    int st = BD_OK;
-    for (int i = 0; i < nst && st == BD_OK; i++) st = enqueue_step(stream);
-    cudaError_t e = cudaStreamEndCapture(stream, &g);
-    if (st != BD_OK || e != cudaSuccess) {
-      if (g) cudaGraphDestroy(g);
-      cudaGetLastError();
-      return st != BD_OK ? st : status_from_cuda(e);
-    }
-    cudaGraphExec_t ex = nullptr;
-    e = cudaGraphInstantiate(&ex, g, 0);
-    cudaGraphDestroy(g);
-    CK(e);
-    (which == 0 ? g1 : gK) = ex;
+// A graph of nst launch-per-step steps.
+int Engine::make_graph(int nst, cudaGraphExec_t* out) {
+  cudaGraph_t g = nullptr;
+  CK(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
+  int st = BD_OK;
+  for (int i = 0; i < nst && st == BD_OK; i++) st = enqueue_step(stream);
+  cudaError_t e = cudaStreamEndCapture(stream, &g);
+  if (st != BD_OK || e != cudaSuccess) {
+    if (g) cudaGraphDestroy(g);
+    cudaGetLastError();
+    return st != BD_OK ? st : status_from_cuda(e);
   }
-  graphs_ok = true;
+  e = cudaGraphInstantiate(out, g, 0);
+  cudaGraphDestroy(g);
+  CK(e);
+  return BD_OK;
+}
+
+// Whether a call of nsteps steps takes the resident step. Several runs: a call
+// of one step takes the launch-per-step form; one run that has the pipelined
+// form too: from 8 steps on, which pay for the force grids it starts from.
+bool Engine::steps_resident(long long nsteps) const {
+  if (!resident) return false;
+  if (runs.size() == 1) return !(piped && nsteps >= 8 && fault_barrier == 0);
+  return nsteps > 1 && !(piped && pipe_form == PIPE_TWO);
+}
+
+// The graphs the coming calls launch, captured with the plan: a first call of
+// steps does not wait for them. A plan whose calls of several steps are
+// resident needs the one of a single step at most, and only where its owner
+// may ask for one.
+int Engine::plan_graphs() {
+  if (runs.empty()) return BD_OK;
+  const bool many = !steps_resident(K);
+  if (many || (one_step_calls && !steps_resident(1))) RK(make_graph(1, &g1));
+  if (many) RK(make_graph(K, &gK));
   return BD_OK;
 }
 
@@ -1713,11 +1729,7 @@ int Engine::step(long long nsteps) {
   if (!planned) RK(build_plan());
   if (runs.empty()) return BD_OK;
   if (nsteps == 0) return BD_OK;
-  // several runs: a call of one step takes the launch-per-step form; one run
-  // that has the pipelined form too: from 8 steps on, which pay for the force
-  // grids it starts from
-  const bool single = runs.size() == 1 && !(piped && nsteps >= 8 && fault_barrier == 0);
-  if (resident && (single || (runs.size() > 1 && nsteps > 1 && !(piped && pipe_form == PIPE_TWO)))) {
+  if (steps_resident(nsteps)) {
     RK(fused_prologue(false));
     grids_valid = false;
     return step_resident(nsteps);
@@ -1728,7 +1740,8 @@ int Engine::step(long long nsteps) {
     RK(enqueue_pipe2(stream));
     nsteps--;
   }
-  if (!graphs_ok) RK(make_graphs());
+  if (nsteps >= K && !gK) RK(make_graph(K, &gK));
+  if (nsteps % K && !g1) RK(make_graph(1, &g1));
   while (nsteps >= K) {
     CK(cudaGraphLaunch(gK, stream));
     nsteps -= K;

@@ -131,6 +131,9 @@ class Engine {
   enum { PIPE_SIX = 0, PIPE_TWO = 1 };
   int pipe_form = PIPE_SIX;  // the faster on every mix measured on a B200
   int tail_minb = 4;  // CTAs per SM of the cooperative launch (2, 3 or 4)
+  // calls of one step are expected (off: a plan that steps several at a time
+  // resident is built without the graph of one)
+  bool one_step_calls = true;
   int set_step_form(int form, int ctas);  // rebuilds the plan and graphs
   int autotune(int reps, bd_tune_result* out);
   int fused_phase_times(int nsteps, double* ms, int nphases);  // fused or pipelined step
@@ -281,8 +284,9 @@ class Engine {
   int time_particles(int shape, int reps, cudaEvent_t e0, cudaEvent_t e1, double* ms);
   int tune_particles(int reps, cudaEvent_t e0, cudaEvent_t e1, bd_tune_result* out);
   int plan_tail();
-  int make_graphs();
-  bool graphs_ok = false;
+  int make_graph(int nst, cudaGraphExec_t* out);
+  int plan_graphs();
+  bool steps_resident(long long nsteps) const;
   void drop_graphs();
   Item* it(int off) { return d_items + off; }
 };

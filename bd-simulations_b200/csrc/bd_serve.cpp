@@ -269,6 +269,7 @@ int bd_serve_create(const bd_serve_opts* o, bd_server** out) {
   if (s->o.steps_per_tick <= 0) s->o.steps_per_tick = 100;
   if (o->snapshot_dir) s->snapdir = o->snapshot_dir;
   s->o.snapshot_dir = nullptr;
+  s->e.one_step_calls = s->o.steps_per_tick == 1;
   int st = s->e.init(o->device);
   if (st != BD_OK) {
     delete s;

@@ -1,0 +1,46 @@
+"""What a program waits for the first time it makes a call: nothing that the
+run's or the batch's creation could have done."""
+import time
+
+import pytest
+
+from test_gpu_resident import _lattice, _params
+
+pytestmark = pytest.mark.gpu
+
+
+def _seconds(fn):
+    t = time.perf_counter()
+    fn()
+    return time.perf_counter() - t
+
+
+def _steps(x, n):
+    x.step(n)
+    x.sync()
+
+
+# 24 pipelined runs; 24 runs whose calls of several steps are resident, asked
+# for single steps; a large run that steps pipelined when asked for many
+@pytest.mark.parametrize("kind", ["pipelined", "one_step", "large_run"])
+def test_first_steps_do_not_wait_for_graphs(gpu, kind):
+    """The launch-per-step graphs are captured with the plan (0.4 to 1.5 ms for
+    these): a first call costs its uploads and cold caches more than a later
+    one (0.05 to 0.35 ms)."""
+    extra = []
+    for rep in range(4):
+        if kind == "large_run":
+            p = _params(gpu, 150000, 150000, 512, False)
+            x = gpu.Run(p, seed=3)
+            call = lambda: x.zeitschritte(20)  # noqa: E731
+        else:
+            p = _params(gpu, 1600, 1500, 128 if kind == "pipelined" else 96, False)
+            x = gpu.Batch([p] * 24, list(range(24)))
+            call = (lambda: _steps(x, 20)) if kind == "pipelined" else (lambda: _steps(x, 1))  # noqa: E731
+        x.sync()
+        first = _seconds(call)
+        later = min(_seconds(call) for _ in range(3))
+        extra.append(first - later)
+        x.close()
+    bound = 0.2e-3 if kind == "one_step" else 0.7e-3
+    assert min(extra) < bound, "first call %s ms longer" % ", ".join("%.2f" % (e * 1e3) for e in extra)
