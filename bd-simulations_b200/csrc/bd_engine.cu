@@ -177,7 +177,6 @@ Engine::~Engine() {
     delete r;
   }
   if (stream) cudaStreamSynchronize(stream);
-  if (h_stage) cudaFreeHost(h_stage);
   if (h_dyn) cudaFreeHost(h_dyn);
   if (ev_stage) cudaEventDestroy(ev_stage);
   for (auto& e : ev_piece)
@@ -789,31 +788,39 @@ int Engine::upload_tables() {
   return BD_OK;
 }
 
-// The pinned staging buffer, at least `bytes` long, once the last copy that
-// used it has ended (the host may write it).
+// The pinned host memory: room for `states` run states, then a staging buffer
+// of at least `bytes`. One allocation: the driver takes 1.3 to 2.9 ms for one
+// that needs fresh pages, and the states' would fall into a run's first
+// synchronising call.
+int Engine::pinned(size_t states, size_t bytes) {
+  if (states <= h_dyn_cap && bytes <= h_stage_cap) return BD_OK;
+  CK(cudaEventSynchronize(ev_stage));  // the last copy that used the buffer has ended
+  if (h_dyn) CK(cudaFreeHost(h_dyn));
+  h_dyn = nullptr;
+  h_stage = nullptr;
+  const size_t ns = std::max(std::max<size_t>(h_dyn_cap, 256), states > h_dyn_cap ? states + states / 2 : 0);
+  const size_t nb = std::max(h_stage_cap, std::max<size_t>(bytes + bytes / 4, 4096));
+  h_dyn_cap = h_stage_cap = 0;
+  void* q = nullptr;
+  CK(cudaHostAlloc(&q, r256(ns * sizeof(RunDyn)) + nb, cudaHostAllocDefault));
+  h_dyn = static_cast<RunDyn*>(q);
+  h_stage = static_cast<char*>(q) + r256(ns * sizeof(RunDyn));
+  h_dyn_cap = ns;
+  h_stage_cap = nb;
+  return BD_OK;
+}
+
+// The staging buffer, at least `bytes` long, once the last copy that used it
+// has ended (the host may write it).
 int Engine::stage_buffer(size_t bytes, void** out) {
   CK(cudaEventSynchronize(ev_stage));
-  if (bytes > h_stage_cap) {
-    if (h_stage) CK(cudaFreeHost(h_stage));
-    h_stage = nullptr;
-    h_stage_cap = 0;
-    const size_t cap = std::max<size_t>(bytes + bytes / 4, 4096);
-    CK(cudaHostAlloc(&h_stage, cap, cudaHostAllocDefault));
-    h_stage_cap = cap;
-  }
+  RK(pinned(runs.size(), bytes));
   *out = h_stage;
   return BD_OK;
 }
 
 int Engine::fetch_dyn(size_t first, size_t n) {
-  if (n > h_dyn_cap) {
-    if (h_dyn) CK(cudaFreeHost(h_dyn));
-    h_dyn = nullptr;
-    h_dyn_cap = 0;
-    const size_t cap = n + n / 2 + 4;
-    CK(cudaHostAlloc((void**)&h_dyn, cap * sizeof(RunDyn), cudaHostAllocDefault));
-    h_dyn_cap = cap;
-  }
+  RK(pinned(n, 0));
   if (n) CK(cudaMemcpyAsync(h_dyn, d_dyn + first, n * sizeof(RunDyn), cudaMemcpyDeviceToHost, stream));
   CK(cudaStreamSynchronize(stream));
   return BD_OK;

@@ -180,17 +180,18 @@ class Engine {
   bool tables_ok = false;  // d_runs / d_dyn hold the current runs (device state authoritative)
   bool descs_ok = false;   // d_runs holds the current runs' descriptions (cleared when they change)
   int upload_tables();
-  // pinned host buffer of the position copies (records in and out): copies
+  // pinned host memory, one allocation. h_dyn: the run states (RunDyn), read
+  // back after most calls (a copy into pageable memory is staged by the driver
+  // and waits twice). h_stage: buffer of the position and force copies: copies
   // from it run asynchronously at full link speed; ev_stage marks the end of
   // the last copy that uses it, waited on before the host writes it again
+  RunDyn* h_dyn = nullptr;
+  size_t h_dyn_cap = 0;
   void* h_stage = nullptr;
   size_t h_stage_cap = 0;
   cudaEvent_t ev_stage = nullptr;
+  int pinned(size_t states, size_t bytes);
   int stage_buffer(size_t bytes, void** out);
-  // pinned copies of the run states (RunDyn), read back after most calls: a
-  // copy into pageable memory is staged by the driver and waits twice
-  RunDyn* h_dyn = nullptr;
-  size_t h_dyn_cap = 0;
   int fetch_dyn(size_t first, size_t n);  // states [first, first + n) into h_dyn, after everything queued
   // the device -> host copies of a run's records go in up to this many
   // pieces, each with its event, converted as they arrive
