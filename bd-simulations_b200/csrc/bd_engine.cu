@@ -1172,7 +1172,7 @@ int Engine::enqueue_fft(int require_active, cudaStream_t s, cudaEvent_t* ev, int
 }
 
 int Engine::launches_per_step() const {
-  if (resident && runs.size() == 1) return 1;
+  if (runs.size() == 1 && steps_resident(1)) return 1;
   if (piped && pipe_form == PIPE_TWO && tail_ok) return 2;  // particles, cooperative tail
   if (piped) return 6;  // particles, then scan and scatter beside three transform passes
   int n = 0;
@@ -1711,7 +1711,11 @@ int Engine::make_graph(int nst, cudaGraphExec_t* out) {
 // form too: from 8 steps on, which pay for the force grids it starts from.
 bool Engine::steps_resident(long long nsteps) const {
   if (!resident) return false;
-  if (runs.size() == 1) return !(piped && nsteps >= 8 && fault_barrier == 0);
+  if (runs.size() == 1) {
+    if (fault_barrier > 0) return true;  // the recovery-path test's barriers
+    if (runs[0]->idgas) return !idgas_stage_kernels(runs[0]->N, nsteps);
+    return !(piped && nsteps >= 8);
+  }
   return nsteps > 1 && !(piped && pipe_form == PIPE_TWO);
 }
 

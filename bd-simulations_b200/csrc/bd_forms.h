@@ -15,6 +15,16 @@ struct FormRun {
   double weight() const { return N + (idgas ? 0.0 : 0.25 * Z * Z); }
 };
 
+// Whether a call of nsteps steps of a single ideal-gas run (no mesh: sort and
+// particle kernels only) takes the stage kernels from a graph. Measured, us per
+// step (resident | stage kernels), particles, calls of many steps: 5000 11.0 |
+// 12.8; 35 000 13.3 | 13.1; 60 000 12.9 | 13.5; 131 072 16.8 | 15.1; 500 000 32.1 |
+// 29.5; adaptive dt: 60 000 16.7 | 18.0; 131 072 22.5 | 21.2; 500 000 48.0 | 45.5. A
+// call per step, which pays the resident launch's start each time: 3000 12.4 |
+// 14.4; 5000 14.4 | 14.7; 8000 15.9 | 14.4; 60 000 18.5 | 14.4; adaptive dt: 5000
+// 31.5 | 36.8; 8000 37.6 | 35.3
+inline bool idgas_stage_kernels(int N, long long nsteps) { return N > 65536 || (nsteps == 1 && N > 6000); }
+
 // A batch's calls of several steps: launches per step (the pipelined or the
 // stage kernels), one cluster of CTAs per run, or a group of CTAs of one
 // cooperative grid per run.
