@@ -485,11 +485,21 @@ static Item resident_item(const RunHost& r, int run, int G, int nt, size_t* smem
   return I;
 }
 
-// Whether a resident kernel can run: its attributes set, the CTAs (cs 0) or
-// clusters of cs CTAs that the device holds at once at the kernels' largest
-// shared memory (0: none). Asked once per process, device and kernel: the
-// queries take a few hundred microseconds, a served mix plans every tick.
-static int resident_fit(int lz, int kind, int cs, int device) {
+// Whether a resident kernel can run: the CTAs (cs 0) or clusters of cs CTAs that
+// the device holds at once at the kernels' largest shared memory (0: none).
+// Asked once per process, device and kernel: the queries take a few hundred
+// microseconds, a served mix plans every tick. The kernel's attributes are set
+// once per engine (a microsecond or two): they live in the device's context,
+// and a program that resets the device between engines loses them.
+int Engine::resident_fit(int lz, int kind, int cs) {
+  const auto kernel = std::make_pair(lz, kind);
+  auto a = res_attr.find(kernel);
+  if (a == res_attr.end()) {
+    const int e = resident_attributes(lz, kind);
+    if (e) cudaGetLastError();
+    a = res_attr.emplace(kernel, e == 0).first;
+  }
+  if (!a->second) return 0;
   static std::mutex mu;
   static std::map<std::tuple<int, int, int, int>, int> known;  // a few hundred entries at most
   std::lock_guard<std::mutex> g(mu);
@@ -497,9 +507,9 @@ static int resident_fit(int lz, int kind, int cs, int device) {
   const auto f = known.find(key);
   if (f != known.end()) return f->second;
   int n = 0;
-  if (resident_configure(lz, kind, res_max_smem(kind), cs, device, &n) || n < 0) {
+  if (resident_held(lz, kind, res_max_smem(kind), cs, device, &n) || n < 0) {
     cudaGetLastError();
-    n = 0;
+    return 0;
   }
   return known[key] = n;
 }
@@ -528,12 +538,12 @@ void Engine::resident_items(std::vector<Item>& all) {
     size_t smem = 0;
     resident_item(*runs[k], (int)k, cs, res_threads(RES_CLUSTERS) / 2, &smem);
     if (smem + (size_t)res_pcap(RES_CLUSTERS) * 32 > res_max_smem(RES_CLUSTERS)) return 0;
-    return resident_fit(resident_lz(*runs[k]), RES_CLUSTERS, cs, device);
+    return resident_fit(resident_lz(*runs[k]), RES_CLUSTERS, cs);
   };
   // groups have a pair of barrier words each and one CTA per SM
   int nsm = 0, slots = 0;
   if (cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) nsm = 0;
-  if (runs.size() <= (size_t)std::min(nsm, (int)BAR_GROUPS)) slots = std::min(nsm, resident_fit(-1, RES_GROUPS, 0, device));
+  if (runs.size() <= (size_t)std::min(nsm, (int)BAR_GROUPS)) slots = std::min(nsm, resident_fit(-1, RES_GROUPS, 0));
   const BatchForm form = choose_batch_form(fr, held, slots, piped);
   if (form.step == BATCH_LAUNCHES) return;
   if (form.step == BATCH_GROUPS) {
@@ -597,9 +607,9 @@ int Engine::plan_resident() {
     CK(cudaMemsetAsync(d_bar, 0, 2 * BAR_GROUPS * sizeof(unsigned), stream));
   }
   if (runs.size() > 1) {
-    if (res_share_grid > 0 ? res_share_grid > resident_fit(-1, RES_GROUPS, 0, device) : res_groups.empty()) return BD_OK;
+    if (res_share_grid > 0 ? res_share_grid > resident_fit(-1, RES_GROUPS, 0) : res_groups.empty()) return BD_OK;
     for (const ResGroup& g : res_groups)
-      if (resident_fit(g.lz, RES_CLUSTERS, g.cs, device) <= 0) return BD_OK;
+      if (resident_fit(g.lz, RES_CLUSTERS, g.cs) <= 0) return BD_OK;
     while (res_streams.size() + 1 < res_groups.size()) {
       cudaStream_t s = nullptr;
       CK(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
@@ -627,8 +637,8 @@ int Engine::plan_resident() {
   const size_t work = std::max(sm_c, sm_g);
   rone_smem = work + (size_t)res_pcap(RES_SINGLE) * 32;
   if (rone_smem > res_max_smem(RES_SINGLE)) return BD_OK;
-  if (res_cs && resident_fit(rone_lz, RES_SINGLE, res_cs, device) <= 0) res_cs = 0;
-  const int n = resident_fit(rone_lz, RES_SINGLE, 0, device);
+  if (res_cs && resident_fit(rone_lz, RES_SINGLE, res_cs) <= 0) res_cs = 0;
+  const int n = resident_fit(rone_lz, RES_SINGLE, 0);
   if (n <= 0) return BD_OK;
   res_grid = std::min(n, want);
   rone = ResArgs{};

@@ -5,11 +5,13 @@
 #include <condition_variable>
 #include <cstdint>
 #include <functional>
+#include <map>
 #include <memory>
 #include <mutex>
 #include <random>
 #include <string>
 #include <thread>
+#include <utility>
 #include <vector>
 
 #include <cuda_runtime.h>
@@ -229,6 +231,8 @@ class Engine {
   size_t res_share_smem = 0;
   std::vector<int> res_share;  // CTAs of every run's group
   int res_chunk = 1;  // steps per launch
+  std::map<std::pair<int, int>, bool> res_attr;  // kernels whose attributes are set (false: refused)
+  int resident_fit(int lz, int kind, int cs);
   void resident_items(std::vector<Item>& all);
   int plan_resident();
   int launch_one(int nsteps, bool fault, unsigned long long* ts);

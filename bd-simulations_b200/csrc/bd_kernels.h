@@ -149,9 +149,10 @@ struct ResArgs {
 // kind: one run, one cluster per run, or groups of CTAs of one cooperative grid.
 // lz: the mesh side: 2^lz (3..10), 3 * 2^(lz - 16) (20..24: 48 to 768), 0:
 // other meshes with a factor 3 and ideal-gas runs, -1: any (groups). cs: CTAs per cluster, 0: cooperative grid (single run).
-// resident_configure: attributes for smem bytes of dynamic shared memory;
-// *n: resident CTAs (cs 0) or clusters the device can hold at once
-int resident_configure(int lz, int kind, size_t smem, int cs, int device, int* n);
+// resident_held, once resident_attributes has set the kernel's: *n: resident
+// CTAs (cs 0) or clusters the device can hold at once
+int resident_attributes(int lz, int kind);
+int resident_held(int lz, int kind, size_t smem, int cs, int device, int* n);
 int launch_resident(int lz, int kind, const ResArgs& A, int nclusters, int cs, int grid, size_t smem,
                     cudaStream_t s);
 // One step of one run on a power-of-two mesh up to 1024^2 with a fixed dt in

@@ -4,24 +4,39 @@
 namespace bd {
 
 template <int LZ, int KIND>
-int resident_configure_t(size_t smem, int cs, int nsm, int* grid);
+int resident_attributes_t();
+template <int LZ, int KIND>
+int resident_held_t(size_t smem, int cs, int nsm, int* n);
 template <int LZ, int KIND>
 int launch_resident_t(const ResArgs& A, int nclusters, int cs, int grid, size_t smem, cudaStream_t s);
 
 #define BD_RES_SIZES(X) \
   X(0) X(3) X(4) X(5) X(6) X(7) X(8) X(9) X(10) X(20) X(21) X(22) X(23) X(24)
 
-int resident_configure(int lz, int kind, size_t smem, int cs, int device, int* n) {
+int resident_attributes(int lz, int kind) {
+  if (kind == RES_GROUPS) return resident_attributes_t<-1, RES_GROUPS>();
+  switch (lz) {
+#define BD_CASE(L)                                                                                      \
+  case L:                                                                                               \
+    return kind == RES_SINGLE ? resident_attributes_t<L, RES_SINGLE>() : resident_attributes_t<L, RES_CLUSTERS>();
+    BD_RES_SIZES(BD_CASE)
+#undef BD_CASE
+    default:
+      return (int)cudaErrorInvalidValue;
+  }
+}
+
+int resident_held(int lz, int kind, size_t smem, int cs, int device, int* n) {
   *n = 0;
   int nsm = 0;
   cudaError_t e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, device);
   if (e != cudaSuccess) return (int)e;
-  if (kind == RES_GROUPS) return resident_configure_t<-1, RES_GROUPS>(smem, 0, nsm, n);
+  if (kind == RES_GROUPS) return resident_held_t<-1, RES_GROUPS>(smem, 0, nsm, n);
   switch (lz) {
 #define BD_CASE(L)                                                       \
   case L:                                                                \
-    return kind == RES_SINGLE ? resident_configure_t<L, RES_SINGLE>(smem, cs, nsm, n)      \
-                              : resident_configure_t<L, RES_CLUSTERS>(smem, cs, nsm, n);
+    return kind == RES_SINGLE ? resident_held_t<L, RES_SINGLE>(smem, cs, nsm, n)      \
+                              : resident_held_t<L, RES_CLUSTERS>(smem, cs, nsm, n);
     BD_RES_SIZES(BD_CASE)
 #undef BD_CASE
     default:

@@ -968,23 +968,28 @@ __global__ void __launch_bounds__(res_threads(KIND), KIND == RES_CLUSTERS ? 2 : 
   if (grid) grid_exit(bar, (unsigned)G);
 }
 
-// sets the kernel's attributes for `smem` bytes; grid mode: fills *grid with
-// the CTAs that can be resident; cluster mode: *grid > 0 when clusters of
-// `cs` CTAs can be scheduled. Returns 0 or a cudaError_t.
+// the kernel's attributes: its largest shared memory, clusters beyond eight CTAs
 template <int LZ, int KIND>
-int resident_configure_t(size_t smem, int cs, int nsm, int* grid) {
+int resident_attributes_t() {
+  auto* f = k_resident<LZ, KIND>;
+  cudaError_t e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)res_max_smem(KIND));
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(f, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+  return (int)e;
+}
+
+// with the attributes set: grid mode (cs 0): fills *n with the CTAs that can
+// be resident; cluster mode: with the clusters of cs CTAs. Returns 0 or a
+// cudaError_t.
+template <int LZ, int KIND>
+int resident_held_t(size_t smem, int cs, int nsm, int* n) {
   auto* f = k_resident<LZ, KIND>;
   if (smem > res_max_smem(KIND)) return (int)cudaErrorInvalidValue;
-  cudaError_t e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)res_max_smem(KIND));
-  if (e != cudaSuccess) return (int)e;
   if (cs == 0) {
     int per = 0;
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, f, res_threads(KIND), smem);
-    *grid = per * nsm;
+    const cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, f, res_threads(KIND), smem);
+    *n = per * nsm;
     return (int)e;
   }
-  e = cudaFuncSetAttribute(f, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-  if (e != cudaSuccess) return (int)e;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(cs);
   cfg.blockDim = dim3(res_threads(KIND));
@@ -995,7 +1000,7 @@ int resident_configure_t(size_t smem, int cs, int nsm, int* grid) {
   attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  return (int)cudaOccupancyMaxActiveClusters(grid, f, &cfg);
+  return (int)cudaOccupancyMaxActiveClusters(n, f, &cfg);
 }
 
 template <int LZ, int KIND>
@@ -1020,7 +1025,8 @@ int launch_resident_t(const ResArgs& A, int nclusters, int cs, int grid, size_t 
 }
 
 #define BD_RES_INSTANTIATE_KIND(L, K)                           \
-  template int resident_configure_t<L, K>(size_t, int, int, int*); \
+  template int resident_attributes_t<L, K>();                     \
+  template int resident_held_t<L, K>(size_t, int, int, int*);     \
   template int launch_resident_t<L, K>(const ResArgs&, int, int, int, size_t, cudaStream_t);
 #define BD_RES_INSTANTIATE(L)            \
   BD_RES_INSTANTIATE_KIND(L, RES_CLUSTERS) \
