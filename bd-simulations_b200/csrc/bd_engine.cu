@@ -533,7 +533,7 @@ void Engine::resident_items(std::vector<Item>& all) {
     return;
   }
   std::vector<FormRun> fr(runs.size());
-  for (size_t k = 0; k < runs.size(); k++) fr[k] = {runs[k]->N, runs[k]->Z, runs[k]->idgas};
+  for (size_t k = 0; k < runs.size(); k++) fr[k] = {runs[k]->N, runs[k]->Z, runs[k]->idgas, runs[k]->adaptive};
   auto held = [&](size_t k, int cs) {
     size_t smem = 0;
     resident_item(*runs[k], (int)k, cs, res_threads(RES_CLUSTERS) / 2, &smem);
@@ -544,7 +544,7 @@ void Engine::resident_items(std::vector<Item>& all) {
   int nsm = 0, slots = 0;
   if (cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) nsm = 0;
   if (runs.size() <= (size_t)std::min(nsm, (int)BAR_GROUPS)) slots = std::min(nsm, resident_fit(-1, RES_GROUPS, 0));
-  const BatchForm form = choose_batch_form(fr, held, slots, piped);
+  const BatchForm form = choose_batch_form(fr, held, slots, piped, std::max(nsm, 1));
   if (form.step == BATCH_LAUNCHES) return;
   if (form.step == BATCH_GROUPS) {
     off_share = (int)all.size();

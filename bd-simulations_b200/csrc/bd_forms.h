@@ -3,6 +3,7 @@
 #pragma once
 
 #include <algorithm>
+#include <set>
 #include <vector>
 
 namespace bd {
@@ -11,9 +12,64 @@ namespace bd {
 struct FormRun {
   int N, Z;
   bool idgas;
+  bool adaptive = false;
   // work per CTA counts particles and a quarter of the mesh points
   double weight() const { return N + (idgas ? 0.0 : 0.25 * Z * Z); }
+  double points() const { return idgas ? 0.0 : (double)Z * Z; }
+  bool pow2() const { return (Z & (Z - 1)) == 0; }
+  // a power of two, or 3 * 2^k with transforms of its own in the resident step
+  bool compiled() const { return pow2() || (Z >= 48 && Z % 3 == 0 && ((Z / 3) & (Z / 3 - 1)) == 0); }
 };
+
+// us per step of a batch in the stage kernels' launches, which wait for one set
+// of transforms after another (a set for every power of two, one for all meshes
+// with a factor 3) and for the deposit tile of most particles.
+inline double estimate_launches(const std::vector<FormRun>& runs) {
+  double n = 0.0, m2 = 0.0, m3 = 0.0, tile = 0.0;
+  std::set<int> sides;
+  bool adaptive = false, factor3 = false;
+  for (const FormRun& r : runs) {
+    n += r.N;
+    adaptive = adaptive || r.adaptive;
+    if (r.idgas) continue;
+    (r.pow2() ? m2 : m3) += r.points();
+    if (r.pow2()) sides.insert(r.Z);
+    else factor3 = true;
+    int mt = 4;
+    for (int c : {64, 48, 32, 24, 16, 12, 8, 6})
+      if (r.Z % c == 0) {
+        mt = c;
+        break;
+      }
+    const double side = std::max(1, r.Z / mt);
+    tile = std::max(tile, r.N / (side * side));
+  }
+  if (m2 + m3 == 0.0) return 12.0 + (adaptive ? 6.0 : 0.0) + 3.7e-5 * n;
+  return 10.0 + (adaptive ? 6.0 : 0.0) + 18.0 * (double)sides.size() + (factor3 ? 34.0 : 0.0) +
+         (adaptive ? 1.4e-4 : 1.3e-4) * n + 2.3e-5 * m2 + 5.7e-5 * m3 + 1.9e-3 * tile;
+}
+
+// us per step of a batch without the pipelined step whose run k has ctas[k] CTAs,
+// that of the run that takes longest: clusters (two CTAs per SM once there are
+// more than SMs, which slow each other down) or groups (a CTA per SM, up to
+// 2048 particles in its shared memory).
+inline double estimate_resident(const std::vector<FormRun>& runs, const std::vector<int>& ctas, bool clusters, int sms) {
+  double most = 0.0, all = 0.0;
+  bool adaptive = false, mesh = false;
+  for (size_t k = 0; k < runs.size(); k++) {
+    const FormRun& r = runs[k];
+    const double n = (double)r.N / ctas[k], m = r.points() / ctas[k];
+    adaptive = adaptive || r.adaptive;
+    mesh = mesh || !r.idgas;
+    all += ctas[k];
+    const double per_point = clusters ? (r.compiled() ? 0.0055 : 0.0171) : (r.compiled() ? 0.0056 : 0.0129);
+    const double per_n = clusters ? (r.adaptive ? 0.0176 : 0.0089) : (r.adaptive ? 0.0144 : 0.0061);
+    most = std::max(most, per_n * n + per_point * m + (clusters ? 0.0 : 0.0011 * std::max(0.0, n - 2048.0)));
+  }
+  if (!clusters) return (mesh ? 16.8 : 10.4) + (adaptive ? 1.4 : 0.0) + most;
+  const double full = std::min(1.0, std::max(0.0, all / sms - 1.0));
+  return (mesh ? 12.9 : 7.8) + (adaptive ? 1.2 : 0.0) + most * (1.0 + 0.56 * full);
+}
 
 // Whether a call of nsteps steps of a single ideal-gas run (no mesh: sort and
 // particle kernels only) takes the stage kernels from a graph. Measured, us per
@@ -32,17 +88,17 @@ enum BatchStep { BATCH_LAUNCHES, BATCH_CLUSTERS, BATCH_GROUPS };
 struct BatchForm {
   BatchStep step = BATCH_LAUNCHES;
   std::vector<int> ctas;  // per run: CTAs of its cluster or group
+  double us = 0.0;        // estimate of a step
 };
 
 // held(k, cs): clusters of cs CTAs for run k that the device holds at once (0:
 // none). slots: CTAs to share out among groups (0: no groups). piped: the batch
-// has the pipelined step.
+// has the pipelined step. sms: SMs of the device.
 template <class Held>
-BatchForm choose_batch_form(const std::vector<FormRun>& runs, const Held& held, int slots, bool piped) {
+BatchForm choose_batch_form(const std::vector<FormRun>& runs, const Held& held, int slots, bool piped, int sms = 148) {
   BatchForm out;
   const size_t n = runs.size();
   double particles = 0.0;
-  for (const FormRun& r : runs) particles += r.N;
   // Clusters: every run on clusters of one size, the largest at which the
   // whole batch is resident at once; then larger clusters for runs that would
   // hold the others up, while there is room to spare (a batch that takes a mix
@@ -92,22 +148,41 @@ BatchForm choose_batch_form(const std::vector<FormRun>& runs, const Held& held, 
     const size_t t = top();
     most_g = runs[t].weight() / share[t];
   }
-  // Estimates of a step in us, fitted to measurements of 1 to 128 runs of 1000
-  // to 250 000 particles (clusters 12-60, groups 14-45, the pipelined step
-  // 20-110; the stage kernels, 45-900, were never the fastest). A form that
-  // does not fit is not compared.
-  const double t_clusters = 8.0 + 0.025 * most_c, t_groups = 14.0 + 0.016 * most_g;
-  double best = 19.0 + 8e-5 * particles;  // pipelined
-  bool have = piped;
-  auto consider = [&](BatchStep s, const std::vector<int>& ctas, double t) {
-    if (ctas.empty() || (have && t > best)) return;
-    have = true;
-    best = t;
+  double most;  // a resident form has to take less than this
+  bool mesh = false;
+  for (const FormRun& r : runs) {
+    particles += r.N;
+    mesh = mesh || !r.idgas;
+  }
+  if (piped) {
+    // Estimates fitted to 1 to 128 runs of 1000 to 250 000 particles (clusters
+    // 12-60 us, groups 14-45, the pipelined step 20-110). Of 171 batches of 2 to
+    // 320 runs timed in every form, 5 took longer in the chosen one than in
+    // launches (1.15 times at most).
+    most = out.us = 19.0 + 8e-5 * particles;
+  } else {
+    // Estimates fitted to 864 batches of 2 to 320 runs of 300 to 100 000
+    // particles on meshes of 32 to 1024 points a side, timed in every form (rms
+    // errors of launches, groups and clusters 11, 12 and 23 %, hence the 0.9).
+    // In the chosen form 7 of them take longer than in launches (by more than
+    // 4 %; 1.44 times at most), and a step is 1.6 times as fast on average. The
+    // piped batches' estimates, used for these too before, did not look at the
+    // stage kernels: 157 took longer (256 adaptive runs on meshes of 32 to 1024
+    // points: 6580 us a step on clusters of one CTA, 1464 in launches), 1.49
+    // times as fast.
+    out.us = estimate_launches(runs);
+    most = (mesh ? 0.9 : 1.0) * out.us;
+  }
+  auto consider = [&](BatchStep s, const std::vector<int>& ctas, double t_piped) {
+    if (ctas.empty()) return;
+    const double t = piped ? t_piped : estimate_resident(runs, ctas, s == BATCH_CLUSTERS, sms);
+    if (t >= most) return;
+    most = out.us = t;
     out.step = s;
     out.ctas = ctas;
   };
-  consider(BATCH_CLUSTERS, clusters, t_clusters);
-  consider(BATCH_GROUPS, share, t_groups);
+  consider(BATCH_CLUSTERS, clusters, 8.0 + 0.025 * most_c);
+  consider(BATCH_GROUPS, share, 14.0 + 0.016 * most_g);
   return out;
 }
 
