@@ -524,16 +524,13 @@ void Engine::resident_items(std::vector<Item>& all) {
   if (runs.empty()) return;
   for (auto* r : runs)
     if (!resident_run(*r)) return;
-  long long total = 0;
-  for (auto* r : runs) total += r->N;
-  // steps per launch: about 50 ms of device time at most
-  res_chunk = (int)std::max<long long>(8, std::min<long long>(1024, 400000000ll / std::max<long long>(total, 1)));
+  std::vector<FormRun> fr(runs.size());
+  for (size_t k = 0; k < runs.size(); k++) fr[k] = {runs[k]->N, runs[k]->Z, runs[k]->idgas, runs[k]->adaptive};
   if (runs.size() == 1) {
+    res_chunk = steps_per_launch(estimate_single(fr[0]));
     resident = true;
     return;
   }
-  std::vector<FormRun> fr(runs.size());
-  for (size_t k = 0; k < runs.size(); k++) fr[k] = {runs[k]->N, runs[k]->Z, runs[k]->idgas, runs[k]->adaptive};
   auto held = [&](size_t k, int cs) {
     size_t smem = 0;
     resident_item(*runs[k], (int)k, cs, res_threads(RES_CLUSTERS) / 2, &smem);
@@ -546,6 +543,7 @@ void Engine::resident_items(std::vector<Item>& all) {
   if (runs.size() <= (size_t)std::min(nsm, (int)BAR_GROUPS)) slots = std::min(nsm, resident_fit(-1, RES_GROUPS, 0));
   const BatchForm form = choose_batch_form(fr, held, slots, piped, std::max(nsm, 1));
   if (form.step == BATCH_LAUNCHES) return;
+  res_chunk = steps_per_launch(form.us);
   if (form.step == BATCH_GROUPS) {
     off_share = (int)all.size();
     res_share = form.ctas;

@@ -81,6 +81,16 @@ inline double estimate_resident(const std::vector<FormRun>& runs, const std::vec
 // 31.5 | 36.8; 8000 37.6 | 35.3
 inline bool idgas_stage_kernels(int N, long long nsteps) { return N > 65536 || (nsteps == 1 && N > 6000); }
 
+// us per step of a single resident run, about (to a factor of two: 64 000
+// particles on 768^2 47, 262 144 on 1024^2 83, 3 000 000 on 1024^2 591).
+inline double estimate_single(const FormRun& r) {
+  return r.idgas ? 10.0 + 1e-4 * r.N : 15.0 + 1.9e-4 * r.N + (r.compiled() ? 5e-5 : 1.5e-4) * r.points();
+}
+
+// Steps of one resident launch: about 50 ms of the device's time, whatever the
+// runs are (other work waits for a whole launch).
+inline int steps_per_launch(double us) { return (int)std::max(1.0, std::min(1024.0, 5e4 / std::max(us, 1.0))); }
+
 // A batch's calls of several steps: launches per step (the pipelined or the
 // stage kernels), one cluster of CTAs per run, or a group of CTAs of one
 // cooperative grid per run.

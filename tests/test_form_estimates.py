@@ -24,7 +24,8 @@ int main(int argc, char** argv) {
   for (int k = 0; k < n; k++) runs.push_back(kinds[k % kinds.size()]);
   auto held = [&](size_t k, int cs) { return runs[k].Z > 1024 ? 0 : cs == 16 ? 8 : 296 / cs; };
   const BatchForm f = choose_batch_form(runs, held, n <= 148 ? 148 : 0, std::atoi(argv[1]) != 0, 148);
-  std::printf("%d %.3f %d\n", (int)f.step, f.us, idgas_stage_kernels(kinds[0].N, kinds[0].Z));
+  std::printf("%d %.3f %d %d %d\n", (int)f.step, f.us, idgas_stage_kernels(kinds[0].N, kinds[0].Z),
+              steps_per_launch(f.us), steps_per_launch(estimate_single(kinds[0])));
   return 0;
 }
 """
@@ -44,7 +45,7 @@ def harness(tmp_path_factory):
 def _form(harness, piped, runs, kinds):
     o = subprocess.run([harness, str(piped), str(runs)] + [str(v) for k in kinds for v in k], check=True,
                        capture_output=True, text=True).stdout.split()
-    return int(o[0]), float(o[1]), int(o[2])
+    return int(o[0]), float(o[1]), int(o[2]), int(o[3]), int(o[4])
 
 
 # us per step measured in launches, on clusters, in groups (None: do not fit)
@@ -65,7 +66,7 @@ def _form(harness, piped, runs, kinds):
     (0, 256, [(305, 32, 1, 0)], (16.2, 11.5, None)),
 ])
 def test_the_fastest_form(harness, piped, runs, kinds, us):
-    form, estimate, _ = _form(harness, piped, runs, kinds)
+    form, estimate = _form(harness, piped, runs, kinds)[:2]
     best = min((t, k) for k, t in enumerate(us) if t is not None)[1]
     assert form == best or us[form] < 1.1 * us[best]
     if not piped:  # the pipelined step's estimate counts particles only
@@ -75,3 +76,16 @@ def test_the_fastest_form(harness, piped, runs, kinds, us):
 @pytest.mark.parametrize("n,steps,launches", [(6000, 1, 0), (6001, 1, 1), (6001, 2, 0), (65536, 400, 0), (65537, 400, 1)])
 def test_single_ideal_gas_runs(harness, n, steps, launches):
     assert _form(harness, 0, 1, [(n, steps, 1, 0)])[2] == launches
+
+
+# us per step measured: batches, single runs
+@pytest.mark.parametrize("runs,kind,us", [(256, (1000, 768, 0, 1), 5368), (148, (1000, 768, 0, 0), 3326),
+                                          (256, (16000, 192, 0, 1), 830), (290, (479, 32, 0, 1), 32),
+                                          (1, (2000, 128, 0, 0), 15), (1, (64000, 648, 0, 1), 78),
+                                          (1, (262144, 1024, 0, 1), 83), (1, (3000000, 1024, 0, 1), 591)])
+def test_a_launch_takes_about_50_ms_at_most(harness, runs, kind, us):
+    f = _form(harness, 0, runs, [kind])
+    steps = f[4] if runs == 1 else f[3]
+    assert runs == 1 or f[0] != LAUNCHES
+    assert 1 <= steps <= 1024 and steps * us <= 100e3
+    assert steps == 1024 or steps * us >= 25e3
