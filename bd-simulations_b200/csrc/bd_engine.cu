@@ -1573,8 +1573,8 @@ int Engine::time_mesh_passes(int reps, cudaEvent_t e0, cudaEvent_t e1, double* m
   return BD_OK;
 }
 
-// reps launches of the step's particle kernel in the given shape (MODE_STEP
-// with the deposit of a pipelined plan; MODE_FORCES for adaptive-dt plans),
+// reps launches of the step's particle kernel in the given shape (launch_step,
+// with the deposit of a pipelined plan; the forces alone for adaptive-dt plans),
 // the first untimed. What they leave (cell counts, chunk totals, the step's
 // records in recB, density accumulators, forces, the per-run counters) is
 // put back by tune_particles.

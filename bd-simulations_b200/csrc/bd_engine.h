@@ -245,8 +245,7 @@ class Engine {
   unsigned* d_bar = nullptr;  // barrier words, two per group of CTAs (BAR_GROUPS of them)
   static constexpr int BAR_GROUPS = 256;
   // pipelined stage step (power-of-two meshes, fixed dt, two or more runs or one
-  // on a mesh of 2048 or 4096):
-  // six launches per step, the density deposited in the move, its transform
+  // large one, pipelined_single): six launches per step, the density deposited in the move, its transform
   // beside the cell sort. Its transform items of every mesh size (log2 Z in
   // Item.b) and their shared memory:
   bool piped = false;

@@ -754,8 +754,7 @@ __device__ __forceinline__ void wca_row(const RunDesc& R, const WcaP& W, const R
   }
 }
 
-// Forces and (MODE_STEP) the move of the particle at sorted index gi; DEP:
-// the move also deposits the new position into R.dacc.
+// Forces of the particle at sorted index gi in the mode asked for.
 template <bool NC>
 __device__ __forceinline__ void particle_item(const RunDesc& R, RunDyn& D, const unsigned long long& step, int gi, int mode,
                                               int mask) {
@@ -782,9 +781,8 @@ __device__ __forceinline__ void count_into_cell(const RunDesc& R, int key, unsig
   if ((threadIdx.x & 31) == __ffs(grp) - 1) red_add(&R.chunk_sum[ch], __popc(grp));
 }
 
-// Everything after the WCA sum: store it (MODE_SET/ADD), or add the mesh
-// force and the noise and store the forces (MODE_FORCES) or move and re-bin
-// (MODE_STEP).
+// Everything after the WCA sum: store it (MODE_SET, MODE_ADD), or store it with
+// the mesh force and the noise and take the dt bound (MODE_FORCES).
 template <bool NC>
 __device__ inline void finish_particle(const RunDesc& R, RunDyn& D, const unsigned long long& step, int mode, int mask,
                                        const Rec& p, int ic, int jc, int gi, float2 Fw) {
@@ -803,15 +801,12 @@ __device__ inline void finish_particle(const RunDesc& R, RunDyn& D, const unsign
   const float2 Fk = (R.flags & F_IDGAS) ? make_float2(0.f, 0.f) : mesh_force<NC>(R, p, ic, jc, R.scheme);
   float2 xi = make_float2(0.f, 0.f);
   if (!(R.flags & F_NOWCA)) xi = particle_noise(R.noise, R.seed, step, (uint32_t)p.pid);
-  if (mode == MODE_FORCES) {
-    R.Fw[p.pid] = Fw;
-    R.Fk[p.pid] = Fk;
-    R.Fn[p.pid] = xi;
-    float bnd = fminf(dt_bound(Fw.x + Fk.x, xi.x, R.mrd, R.T), dt_bound(Fw.y + Fk.y, xi.y, R.mrd, R.T));
-    if (!(bnd >= 0.f)) bnd = 3.0e38f;  // NaN never wins the minimum (std::min semantics)
-    if (bnd < R.dt_max) atomicMin(&D.dt_bits, __float_as_uint(bnd));
-    return;
-  }
+  R.Fw[p.pid] = Fw;
+  R.Fk[p.pid] = Fk;
+  R.Fn[p.pid] = xi;
+  float bnd = fminf(dt_bound(Fw.x + Fk.x, xi.x, R.mrd, R.T), dt_bound(Fw.y + Fk.y, xi.y, R.mrd, R.T));
+  if (!(bnd >= 0.f)) bnd = 3.0e38f;  // NaN never wins the minimum (std::min semantics)
+  if (bnd < R.dt_max) atomicMin(&D.dt_bits, __float_as_uint(bnd));
 }
 
 // Forces, noise and move of the particle at sorted index gi, its counts and

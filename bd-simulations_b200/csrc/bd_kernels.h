@@ -14,7 +14,7 @@ struct Item {
   int run, a, b, c;
 };
 
-enum CellblockMode { MODE_STEP = 0, MODE_SET = 1, MODE_ADD = 2, MODE_FORCES = 3 };
+enum CellblockMode { MODE_SET = 1, MODE_ADD = 2, MODE_FORCES = 3 };
 
 constexpr int SCAN_CHUNK = 2048;
 constexpr int FFT_THREADS = 512;
@@ -127,6 +127,9 @@ constexpr size_t RES_DESC_BYTES = 1024;   // the run's description
 __host__ __device__ constexpr size_t RES_TW_BYTES(int Z) {  // twiddles and sine tables
   return ((size_t)8 * Z + 4 * (Z + Z / 2 + 1) + 255) & ~(size_t)255;
 }
+// mesh classes with kernels of their own (res_side); 0: the rest, ideal gas
+#define BD_RES_SIZES(X) \
+  X(0) X(3) X(4) X(5) X(6) X(7) X(8) X(9) X(10) X(20) X(21) X(22) X(23) X(24)
 struct ResArgs {
   RunDesc one;             // the single run (its dacc set)
   Item one_item;           // its item: run 0, a/b/c = log2 rows forward, columns, rows inverse per item

@@ -10,9 +10,6 @@ int resident_held_t(size_t smem, int cs, int nsm, int* n);
 template <int LZ, int KIND>
 int launch_resident_t(const ResArgs& A, int nclusters, int cs, int grid, size_t smem, cudaStream_t s);
 
-#define BD_RES_SIZES(X) \
-  X(0) X(3) X(4) X(5) X(6) X(7) X(8) X(9) X(10) X(20) X(21) X(22) X(23) X(24)
-
 int resident_attributes(int lz, int kind) {
   if (kind == RES_GROUPS) return resident_attributes_t<-1, RES_GROUPS>();
   switch (lz) {

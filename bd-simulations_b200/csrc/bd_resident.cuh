@@ -823,8 +823,6 @@ __device__ __noinline__ void res_place(RunDyn* D, int b, int g0, int g1, int nc,
 }
 
 // The transform phases with the mesh class known at run time (RES_GROUPS).
-#define BD_RES_SIZES(X) \
-  X(0) X(3) X(4) X(5) X(6) X(7) X(8) X(9) X(10) X(20) X(21) X(22) X(23) X(24)
 template <int LZ, int NT>
 __device__ __forceinline__ void res_inv_of(int lz, int b, int G, int lri, bool alias) {
   if constexpr (LZ >= 0) res_inv<LZ, NT>(b, G, lri, alias);
