@@ -93,14 +93,15 @@ struct RunDesc {
 };
 
 // Mutable per-run state on the device.
-struct RunDyn {
-  unsigned long long step;  // Philox step counter
+struct alignas(16) RunDyn {
+  // what every block of a launch-per-step form looks at first, one 16-byte read
   long long steps_left;     // batched stepping stops a run at zero
-  double t;                 // simulated time
-  float dt;                 // time step used by the current step
-  unsigned int dt_bits;     // min-reduction of the adaptive bound (float bits)
   int err;
   int sorting;  // set by the step's chunk scan: the run takes part in this sort
+  unsigned long long step;  // Philox step counter
+  float dt;                 // time step used by the current step
+  unsigned int dt_bits;     // min-reduction of the adaptive bound (float bits)
+  double t;                 // simulated time
   int pad;
   int moved[2];       // particles of species 1, 2 that left their cell in this step
   int moved_last[2];  // the same for the last completed step
