@@ -744,10 +744,14 @@ def reference_arm(args):
         "cpu_baseline": {"value": value, "unit": "particle-steps/s", "cores": procs, "kind": kind,
                          "cpu": host_cpu(),
                          "sample": "%d steps (+%d warm-up) of the single-run workload in each of %d "
-                                   "processes; reference built with g++ -O3 and the project FFT shim "
-                                   "(FFTW unavailable)" % (steps, args.warmup, procs)},
+                                   "processes; %s" % (steps, args.warmup, procs, CPU_BUILD[kind])},
         "e2e": {"value": value, "unit": "particle-steps/s", "h2d_bytes_per_step": 0, "d2h_bytes_per_step": 0},
     }
+
+
+# what the CPU arm timed (cpu_reference's kind)
+CPU_BUILD = {"reference": "the reference's sources built with g++ -O3 and the project FFT shim (FFTW unavailable)",
+             "port": "this repository's FP64 restatement in C (oracle), the reference's sources not being present"}
 
 
 def main():
