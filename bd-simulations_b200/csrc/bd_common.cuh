@@ -206,13 +206,13 @@ __device__ __forceinline__ void mesh_axis(const RunDesc& R, int ic, float off, i
   t = f - fl;
   if (t >= 1.0f) t = 0.0f, k = q + (int)fl + 1;
   else k = q + (int)fl;
-  // the position lies in (-B, L + B]: k in (-Z, 2Z), one conditional wrap
-  if (k < 0) k += R.Z;
-  else if (k >= R.Z) k -= R.Z;
-  // a position out of the box (not finite, or thrown further than re-binning
-  // reaches) is still one mesh point: the move's deposit uses it in the step
-  // that makes it, before any error is read
-  k = (int)min((unsigned)k, (unsigned)(R.Z - 1));
+  // the position lies in (-B, L + B]: k in (-Z, 2Z), wrapped by the smallest of
+  // k, k + Z and k - Z as unsigned numbers. A position out of the box (not
+  // finite, or thrown further than re-binning reaches) is still one mesh point,
+  // by the fourth: the move's deposit uses it in the step that makes it, before
+  // any error is read
+  const unsigned u = (unsigned)k, Z = (unsigned)R.Z;
+  k = (int)min(min(u, u + Z), min(u - Z, Z - 1u));
 }
 
 // weights as the reference's grid routines (gridRoutinen.cpp): NGP puts all
