@@ -13,7 +13,9 @@
 // Measured, us per call of one step, L2 flushed before it (resident kernel |
 // this one): 2000 particles, 128^2 34.0 | 25.4; 16 384, 256^2 34.8 | 28.6; 65 536,
 // 512^2 42.4 | 31.5; 262 144, 1024^2 97.8 | 76.0; not flushed 23.2 | 25.2, 29.0 |
-// 27.6, 37.4 | 31.2, 86.0 | 67.9: every size takes this kernel.
+// 27.6, 37.4 | 31.2, 86.0 | 67.9. Every size takes this kernel: for the smallest
+// the resident launch is 2 us ahead where calls follow each other directly and
+// 8.6 behind where other work has used the L2 in between.
 #include <algorithm>
 
 #include "bd_items.cuh"

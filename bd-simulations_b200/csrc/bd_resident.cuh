@@ -20,10 +20,11 @@
 // chains (L2 round trips, one thread's instructions, the barriers: storing,
 // meeting and loading again takes 1400 cycles in a cluster of 16 and 3400 on
 // the grid), not bandwidth; about 30 % of the issue slots of its SMs are used.
-// Measured, us per step, one launch per step or eight before | here: 2000
-// particles, 128^2 20.2 | 14.9; 65 536, 512^2 27.7 | 26.1; 4000, 384^2
-// adaptive 79 | 23; 2204, 96^2 adaptive 48 | 17; 70 002, 768^2 88 | 45; a batch
-// of 16 adaptive runs 179 | 51.
+// Measured, us per step of whole calls of many steps with the positions read
+// behind them, one launch per step or eight before | here: 2000 particles, 128^2
+// 20.4 | 15.2; 65 536, 512^2 27.8 | 27.6 (one launch per step already: no gain);
+// 2204, 96^2 adaptive 48 | 18; 70 002, 768^2 88 | 47; a batch of 16 adaptive runs
+// 179 | 57. The steps alone: 14.5, 25.2, 16.8 and 44.2; 4000, 384^2 adaptive 21.9.
 //
 // State between launches, as the prologue (deposit, forward rows, columns)
 // leaves it: spec2 holds the column-transformed spectrum of the current

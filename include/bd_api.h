@@ -454,8 +454,8 @@ int bd_inject_barrier_timeout(bd_ctx* c, int barrier, unsigned max_polls);
  * batch in step form 1 (barrier 1 of the cooperative launch: every run's step
  * fails). Until a synchronising call (bd_zeitschritte, bd_sync,
  * bd_batch_sync, an adaptive bd_zeitschritt) has returned BD_ERR_TIMEOUT, no
- * form of stepping or sorting touches a failed run. BD_ERR_STATE when the
- * steps wait on no grid barrier. */
+ * form of stepping or sorting touches a failed run: positions set in between
+ * are not taken. BD_ERR_STATE when the steps wait on no grid barrier. */
 int bd_inject_wait_timeout(bd_ctx* c, int barrier, unsigned max_polls);
 int bd_batch_inject_wait_timeout(bd_batch* b, int run, int barrier, unsigned max_polls);
 
