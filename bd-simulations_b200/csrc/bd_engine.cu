@@ -427,16 +427,6 @@ static bool resident_run(const RunHost& r) {
   return pow2(r.Z) ? r.Z >= 8 && r.Z <= 1024 : r.Z <= 648 || r.Z == 768;
 }
 
-// A single run that steps pipelined when asked for several steps (on a mesh
-// beyond the resident step's, always). Measured, us per step, 128 steps a call
-// (resident | pipelined | a launch per step), particles, mesh side:
-// 131 072, 256 27.5 | 29.3 | 31.0; 131 072, 512 32.5 | 31.6 | 35.4; 262 144, 512
-// 45.1 | 41.0 | 51.4; 524 288, 512 64.2 | 57.4 | 71.9; 131 072, 1024 60.5 | 49.3 |
-// 51.6; 262 144, 1024 72.9 | 59.9 | 64.1; 900 000, 1024 122 | 105 | 116
-static bool pipelined_single(const RunHost& r) {
-  return r.Z > 1024 || (r.N >= 131072 && r.Z >= 512) || r.N >= 262144;
-}
-
 static int resident_lz(const RunHost& r) {
   if (r.idgas) return 0;
   if (pow2(r.Z)) return ilog2(r.Z);
@@ -701,10 +691,7 @@ int Engine::step_resident(long long nsteps) {
       RK(launch_one(k, true, nullptr));
       nsteps -= k;
     }
-    // 1024^2: four elements per thread of half the CTAs' threads are short of
-    // the transforms' work, the launches cost less (65 536 particles, us per
-    // step: 55.6 resident, 43.9 a launch each)
-    const bool each = one_step.grid > 0 && (piped || runs[0]->Z == 1024);
+    const bool each = one_step.grid > 0 && (piped || launch_per_step_single(runs[0]->N, runs[0]->Z));
     while (nsteps > 0) {
       const int k = each ? 1 : (int)std::min<long long>(nsteps, res_chunk);
       RK(launch_one(k, false, nullptr));
@@ -864,7 +851,7 @@ int Engine::build_plan() {
   // take as many sequences per item as FFT2_THREADS threads transform at
   // once (Z/16 threads per length-Z sequence).
   const size_t nr = runs.size();
-  bool pipe_runs = nr >= 2 || (nr == 1 && pipelined_single(*runs[0]));
+  bool pipe_runs = nr >= 2 || (nr == 1 && pipelined_single(runs[0]->N, runs[0]->Z));
   for (auto* r : runs) pipe_runs = pipe_runs && r->d.dacc != nullptr;
   std::vector<int> lrf(nr), lri(nr), lw(nr);
   for (size_t k = 0; k < nr; k++) {
@@ -973,13 +960,12 @@ int Engine::build_plan() {
   put(chunk, off_chunk, n_chunk);
   off_part_all = off_part;
   n_part_all = n_part;
-  // the particle kernel's form: for runs of 131 072 particles and more on
-  // average, whose arrays do not stay in L2 from one kernel to the next.
-  // Measured, us per step (that form | the other), runs x particles, mesh:
-  // 2 x 100 000, 256^2 36.7 | 35.6; 4 x 100 000 50.8 | 52.3; 2 x 250 000, 512^2
-  // 59.9 | 64.2; 8 x 250 000 200 | 258; 4 x 600 000 206 | 280; 1 x 2 000 000,
-  // 2048^2 247 | 351; the 256-run ensemble (24 000 on average) 562 | 537
-  part_large = n_part >= (int)nr * 512 ? 1 : 0;
+  double particles = 0.0, points = 0.0;
+  for (const auto* r : runs) {
+    particles += r->N;
+    points += r->idgas ? 0.0 : (double)r->Z * r->Z;
+  }
+  part_large = step_kernel_prefetches(n_part, (int)nr, particles, points) ? 1 : 0;
   // pipelined stage step: several runs, every one depositing in the move, or
   // one large run (pipelined_single): 2.1 M particles on 2048^2, 335 us per step
   // with the stage kernels, 252 pipelined

@@ -71,6 +71,55 @@ inline double estimate_resident(const std::vector<FormRun>& runs, const std::vec
   return (mesh ? 12.9 : 7.8) + (adaptive ? 1.2 : 0.0) + most * (1.0 + 0.56 * full);
 }
 
+// more than k particles to a mesh point
+inline bool many_per_point(double n, double points, double k) { return n > k * points; }
+
+// A single run that steps pipelined when asked for several steps (on a mesh
+// beyond the resident step's, always). Measured, us per step, 128 steps a call
+// (resident | pipelined | a launch per step), particles, mesh side:
+// 131 072, 256 27.5 | 29.3 | 31.0; 131 072, 512 32.5 | 31.6 | 35.4; 262 144, 512
+// 45.1 | 41.0 | 51.4; 524 288, 512 64.2 | 57.4 | 71.9; 131 072, 1024 60.5 | 49.3 |
+// 51.6; 262 144, 1024 72.9 | 59.9 | 64.1; 900 000, 1024 122 | 105 | 116.
+// Not with many particles to a mesh point: the blocks under way hold
+// neighbouring cells, and the deposits of all of them meet on a few points; in
+// a launch per step every CTA has a share of its own. 1 000 000, 128 (61 a point)
+// 122 | 127 | 115; 3 000 000, 256 (46) 364 | 324 | 346; 3 000 000, 128 352 | 628 |
+// 340; 1 000 000, 64 167 | 299 | 159 to 200; 3 000 000, 64 588 | 2202 | 532.
+// 4096: the accumulator does not stay in L2 between the move and the rows, and
+// from 262 144 particles on the stage kernels (second) are ahead of what they
+// were before their transforms went through registers (third) where the
+// pipelined step (first) is not: 64 000 444 | 411 | 461; 300 000 501 | 443 | 497;
+// 1 000 000 600 | 489 | 572; 4 000 000 792 | 732 | 857.
+inline bool pipelined_single(int N, int Z) {
+  if (Z > 1024) return Z < 4096 || N < 262144;
+  if (many_per_point(N, (double)Z * Z, 48)) return false;
+  return (N >= 131072 && Z >= 512) || N >= 262144;
+}
+
+// A single run with the one-step kernel that takes it, a launch per step, for
+// calls of several steps too (where they are not pipelined). 1024^2: four
+// elements per thread of half the CTAs' threads are short of the transforms'
+// work, the launches cost less (65 536 particles, us per step: 55.6 resident,
+// 43.9 a launch each). Many particles to a mesh point: as above (64 000 particles,
+// 16^2 76.9 | 68.2; 131 072, 64^2 33.0 | 31.4; 500 000, 64^2 93 | 78).
+inline bool launch_per_step_single(int N, int Z) {
+  return Z == 1024 || (N >= 50000 && many_per_point(N, (double)Z * Z, 24));
+}
+
+// The particle kernel's form (k_step, AHEAD): for runs of 131 072 particles and
+// more on average, whose arrays do not stay in L2 from one kernel to the next.
+// Measured, us per step (that form | the other), runs x particles, mesh:
+// 2 x 100 000, 256^2 36.7 | 35.6; 4 x 100 000 50.8 | 52.3; 2 x 250 000, 512^2
+// 59.9 | 64.2; 8 x 250 000 200 | 258; 4 x 600 000 206 | 280; 1 x 2 000 000,
+// 2048^2 247 | 351; the 256-run ensemble (24 000 on average) 562 | 537. But not
+// with many particles to a mesh point: the blocks that it keeps under way are
+// neighbours and deposit on the same few points (500 000, 64^2 106 | 87;
+// 1 000 000, 128^2 127 | 112; 3 000 000, 64^2 2202 | 789).
+// blocks: of 256 particles, all runs together.
+inline bool step_kernel_prefetches(int blocks, int runs, double particles, double points) {
+  return blocks >= runs * 512 && (points == 0.0 || !many_per_point(particles, points, 24));
+}
+
 // Whether a call of nsteps steps of a single ideal-gas run (no mesh: sort and
 // particle kernels only) takes the stage kernels from a graph. Measured, us per
 // step (resident | stage kernels), particles, calls of many steps: 5000 11.0 |
