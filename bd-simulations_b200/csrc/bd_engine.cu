@@ -970,7 +970,10 @@ int Engine::build_plan() {
   // one large run (pipelined_single): 2.1 M particles on 2048^2, 335 us per step
   // with the stage kernels, 252 pipelined
   piped = pipe_runs;
-  if (piped) {
+  // its work lists also for a run on 4096^2 that steps with the stage kernels:
+  // bd_fused_phase_times times the pipelined step of any large mesh
+  pipe_lists = piped || (nr == 1 && runs[0]->Z > 1024 && runs[0]->d.dacc != nullptr);
+  if (pipe_lists) {
     std::vector<Item> pl[3];
     size_t psm[3] = {0, 0, 0};
     for (int P = 1; P < 14; P++)
@@ -1408,7 +1411,7 @@ int Engine::fused_phase_times(int nsteps, double* ms, int nphases) {
     if (!r->has_pos) return BD_ERR_STATE;
   CK(cudaSetDevice(device));
   if (!planned) RK(build_plan());
-  if (piped && !fused) return pipe_phase_times(nsteps, ms, nphases);
+  if (pipe_lists && !fused) return pipe_phase_times(nsteps, ms, nphases);
   if (!fused) return BD_ERR_STATE;
   RK(fused_prologue(false));
   unsigned long long* d_ts = nullptr;

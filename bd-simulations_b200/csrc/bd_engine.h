@@ -249,6 +249,7 @@ class Engine {
   // beside the cell sort. Its transform items of every mesh size (log2 Z in
   // Item.b) and their shared memory:
   bool piped = false;
+  bool pipe_lists = false;  // the lists are there (phase times)
   // its second stream (the transform kernels beside the sort) and the events
   // that fork and join it
   cudaStream_t stream2 = nullptr;

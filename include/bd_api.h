@@ -418,7 +418,8 @@ int bd_batch_set_step_form(bd_batch* b, int form, int ctas_per_sm);
  * launch, or for large runs the pipelined step below); bd_launches_per_step then reports 1 and
  * bd_stage_times times the stage kernels instead. Runs on
  * power-of-two meshes with a fixed dt otherwise (a batch of two or more of
- * them, one on a larger mesh) step in six launches per step (the pipelined stage step;
+ * them, one on 2048^2 or, below 262 144 particles, on 4096^2) step in six
+ * launches per step (the pipelined stage step;
  * bd_launches_per_step reports 6): the particle kernel, then the cell sort
  * beside the transform of the new density on a second stream. This runs
  * nsteps steps and returns the mean time per step of each phase in ms (the

@@ -57,3 +57,24 @@ def test_first_sync_allocates_no_pinned_pages(gpu):
         took.append(_seconds(r.sync))
         r.close()
     assert min(took) < 0.7e-3, "first sync %s ms" % ", ".join("%.2f" % (e * 1e3) for e in took)
+
+
+def test_phase_times_of_a_run_that_steps_with_the_stage_kernels(gpu):
+    """300 000 particles on 4096^2: steps in the stage kernels' launches; the
+    pipelined step's phases can still be timed, and the steps around them have
+    the bits of stage kernels throughout."""
+    p = _params(gpu, 200000, 100000, 4096, False, rho=0.1)
+    start = _lattice(p, 3)
+    a, b = gpu.Run(p, seed=6), gpu.Run(p, seed=6)
+    for r in (a, b):
+        r.set_positions_all(start)
+    assert a.launches_per_step() > 6
+    a.zeitschritte(2)
+    ms = a.fused_phase_times(3)
+    assert ms is not None and sum(ms.values()) > 0.0
+    a.zeitschritte(2)
+    b.stage_times(7)
+    x, y = a.get_positions(), b.get_positions()
+    for s in (0, 1):
+        assert (x[s][0] == y[s][0]).all() and (x[s][1] == y[s][1]).all()
+    assert a.step_count() == b.step_count() == 7
